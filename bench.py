@@ -697,14 +697,13 @@ def measure(args, workload, steps, e2e_steps, dist, world, rank, local, cpu_seco
             "bound": "int_mad", "achieved": achieved, "peak": peak / 1e12, "unit": "Tmad/s",
             "frac": achieved / (peak / 1e12) if peak else None,
             "traffic": tpk * step_keys if tpk else None,
-            "peak_source": "measured live: rows of mad.lo.cc/madc.hi.cc carry chains shaped like the field "
+            "peak_source": "measured live: rows of mad.lo.cc/madc.hi.cc pairs (wide products) shaped like the field "
                            "multiply, independent accumulators, full occupancy (mk_measure_mad_peaks)",
             "peak_mad_lo": peak_lo / 1e12,
             "frac_of_mad_lo": achieved / (peak_lo / 1e12) if peak_lo else None,
             "work_per_key": {"field_muls": field_muls, "int_mads": mads_per_key,
-                             "mul_form": ("schoolbook: 144 MADs a multiplication" if source == 2 else
-                                          "Karatsuba: 112 MADs a multiplication (comb, batch, back-sweep); "
-                                          "pooled inversions schoolbook (144), squarings 88")},
+                             "mul_form": "schoolbook in even/odd accumulators: 144 MADs (72 wide products) a "
+                                         "multiplication, squarings 88"},
             # the peak's pieces, each on independent chains or carry-linked rows (Tmad/s)
             "imad_pieces": {k: v / 1e12 for k, v in pieces.items()} if pieces else None,
             "kernel_ms_per_launch": ms_local / (steps * launches),

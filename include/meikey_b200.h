@@ -430,8 +430,8 @@ MK_API int mk_measure_field_mul(mk_ctx* ctx, double* radix32_per_s, double* radi
 
 /* Field multiplications per second of the two radix-2^32 forms, measured like
  * mk_measure_field_mul: the schoolbook product (64 mad.lo + 64 mad.hi) and one level of
- * Karatsuba on the 128-bit halves (48 + 48, plus about 60 adds and logic operations), which
- * the secure path's comb additions and batches use.  Both forms run the same chains;
+ * Karatsuba on the 128-bit halves (48 + 48, plus about 60 adds and logic operations).  The
+ * kernels multiply in the schoolbook form, the faster one.  Both forms run the same chains;
  * MK_ERR_SELF_CHECK if any result differs. */
 MK_API int mk_measure_field_mul_forms(mk_ctx* ctx, double* schoolbook_per_s, double* karatsuba_per_s);
 
@@ -451,7 +451,7 @@ MK_API int mk_table_entry(mk_ctx* ctx, uint32_t row, uint64_t col, uint32_t out[
 
 /* Field products on the device, for tests: for i < n (at most 2^20), a[8i..8i+8) times
  * b[8i..8i+8) mod 2^255 - 19, little-endian 32-bit words of any value below 2^256, in the
- * schoolbook form into schoolbook[8i..] and in the Karatsuba form the secure path uses into
+ * schoolbook form the kernels use into schoolbook[8i..] and in the Karatsuba form into
  * karatsuba[8i..].  The results are the kernels' own words: below 2^256, congruent to the
  * product, not reduced to canonical.  Allocates device memory and waits for the context's
  * stream. */
@@ -470,13 +470,13 @@ MK_API int mk_ctx_work_per_key(const mk_ctx* ctx, int seed_source, double* field
 /* Measured peaks of 32-bit integer multiply-adds on the context's device, in MADs/s, each
  * the best of three bounded runs of 10-30 ms at full occupancy with no memory traffic:
  *   *chain_per_s  rows of a schoolbook product as the field multiply issues them
- *                 (mad.lo.cc/madc.lo.cc then madc.hi.cc carry chains, 8 lo + 8 hi per row);
+ *                 (mad.lo.cc/madc.hi.cc pairs on aligned words, four products per chain);
  *                 the denominator of the int-MAD roofline;
  *   *lo_per_s     plain mad.lo.u32 on independent registers (the low-half multiply rate).
  * The reference reports no roofline. */
 MK_API int mk_measure_mad_peaks(mk_ctx* ctx, double* chain_per_s, double* lo_per_s);
 
-/* The pieces of that instruction shape, each on 8 independent chains per thread at full
+/* Low and high halves and wide products apart, each on 8 independent chains per thread at full
  * occupancy (multiply-adds per second): independent mad.hi.u32, independent mad.wide.u32
  * (a full 64-bit product into a 64-bit sum), and rows of 8 madc.lo.cc or 8 madc.hi.cc linked
  * through the carry flag.  Together with mk_measure_mad_peaks they separate the issue cost of

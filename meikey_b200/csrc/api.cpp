@@ -981,11 +981,8 @@ int mk_ctx_work_per_key(const mk_ctx* c, int seed_source, double* field_muls, do
     if (!c || !field_muls || !int_mads || seed_source < MK_SEED_CHACHA20 || seed_source > MK_SEED_INCREMENTAL)
         return MK_ERR_BAD_ARG;
     // radix-2^32 costs: a schoolbook multiplication is 64 mad.lo + 64 mad.hi (8x8 limbs) + 16
-    // (fold by 38), the Karatsuba form 48 + 48 + 16, a squaring 28 cross products + 8 diagonal
-    // ones (72) + 16.  The secure path's comb, batch and back-sweep multiply in the Karatsuba
-    // form; the incremental path and the pooled inversions in the schoolbook one.
+    // (fold by 38), a squaring 28 cross products + 8 diagonal ones (72) + 16.
     const double MUL = mkb::MADS_MUL_SCHOOLBOOK, SQ = mkb::MADS_SQUARE;
-    const double PATH_MUL = seed_source == MK_SEED_INCREMENTAL ? MUL : mkb::MADS_MUL_KARATSUBA;
     const double kpt = c->kpt, rows = c->geom.rows;
     const double ct = mkb::search_threads(c->block, c->layout);
     // comb: row 0 is free, full additions cost 7 multiplications, the last one 3
@@ -1005,7 +1002,7 @@ int mk_ctx_work_per_key(const mk_ctx* c, int seed_source, double* field_muls, do
     double pool_mul = pools * (3.0 * (groups - 1) + 11.0) / (ct * kpt);
     double pool_sq = pools * 254.0 / (ct * kpt);
     *field_muls = comb + batch + pool_mul + pool_sq;
-    *int_mads = (comb + batch) * PATH_MUL + pool_mul * MUL + pool_sq * SQ;
+    *int_mads = (comb + batch + pool_mul) * MUL + pool_sq * SQ;
     return MK_OK;
 }
 

@@ -97,36 +97,181 @@ __device__ __forceinline__ fe fe_sub(const fe& a, const fe& b) {
     return r;
 }
 
-// Fold a 512-bit product t[0..15] to 8 words: t_lo + 38·t_hi, then the top word again.
+// ---- products in even/odd accumulators ----
+//
+// A product of two limbs a_i·b_j is added at words i+j, i+j+1.  The integer pipe adds a full
+// 64-bit product to an aligned register pair in one instruction (with the carry in and out), so
+// the products at even words go to one accumulator e (pairs e[2k], e[2k+1]) and those at odd
+// words to a second one o, one word up (o[k] stands for word k+1): every pair is aligned, and
+// the two are added once at the end.  Rows that add all products into one array put every other
+// chain on misaligned pairs, which splits its products into low and high halves (three issue
+// slots instead of two).  On B200, one chain per thread and 16 warps per SM: 111 G
+// multiplications/s against 102 G for the one-array rows and 100 G for Karatsuba on them
+// (117 against 91 and 103 with four chains); Karatsuba on even/odd accumulators runs at 106 G:
+// its 25 % fewer products do not pay for about 60 more adds.  The search kernel gains 3 % on hashed
+// seeds (2^29 candidates: 696 -> 675 ms; it multiplied in the Karatsuba form) and 12 % on the
+// incremental source (2^30: 128.0 -> 114.0 ms).
+
+// w[0..1] = x·y
+__device__ __forceinline__ void wide(u32* w, u32 x, u32 y) {
+    asm("mul.lo.u32 %0, %2, %3;\n\t"
+        "mul.hi.u32 %1, %2, %3;"
+        : "=&r"(w[0]), "=r"(w[1])
+        : "r"(x), "r"(y));
+}
+
+// One chain of n products by the same limb y on consecutive pairs, w[2i..2i+1] += x_i·y:
+//   rown_carry  every pair holds a sum already; the carry starts the next pair, w[2n] = carry;
+//   rown_top    the last pair is new but for a carry `top` (0 or 1) of an earlier row; it cannot
+//               overflow (x·y + 2 < 2^64).
+__device__ __forceinline__ void row1_carry(u32* w, u32 x0, u32 y) {
+    asm("mad.lo.cc.u32 %0, %3, %4, %0;\n\t"
+        "madc.hi.cc.u32 %1, %3, %4, %1;\n\t"
+        "addc.u32 %2, 0, 0;"
+        : "+r"(w[0]), "+r"(w[1]), "=r"(w[2])
+        : "r"(x0), "r"(y));
+}
+
+__device__ __forceinline__ void row1_top(u32* w, u32 x0, u32 y, u32 top) {
+    asm("mad.lo.cc.u32 %0, %2, %3, %4;\n\t"
+        "madc.hi.u32 %1, %2, %3, 0;"
+        : "=&r"(w[0]), "=r"(w[1])
+        : "r"(x0), "r"(y), "r"(top));
+}
+
+__device__ __forceinline__ void row2_carry(u32* w, u32 x0, u32 x1, u32 y) {
+    asm("mad.lo.cc.u32 %0, %5, %7, %0;\n\t"
+        "madc.hi.cc.u32 %1, %5, %7, %1;\n\t"
+        "madc.lo.cc.u32 %2, %6, %7, %2;\n\t"
+        "madc.hi.cc.u32 %3, %6, %7, %3;\n\t"
+        "addc.u32 %4, 0, 0;"
+        : "+r"(w[0]), "+r"(w[1]), "+r"(w[2]), "+r"(w[3]), "=r"(w[4])
+        : "r"(x0), "r"(x1), "r"(y));
+}
+
+__device__ __forceinline__ void row2_top(u32* w, u32 x0, u32 x1, u32 y, u32 top) {
+    asm("mad.lo.cc.u32 %0, %4, %6, %0;\n\t"
+        "madc.hi.cc.u32 %1, %4, %6, %1;\n\t"
+        "madc.lo.cc.u32 %2, %5, %6, %7;\n\t"
+        "madc.hi.u32 %3, %5, %6, 0;"
+        : "+r"(w[0]), "+r"(w[1]), "=&r"(w[2]), "=r"(w[3])
+        : "r"(x0), "r"(x1), "r"(y), "r"(top));
+}
+
+__device__ __forceinline__ void row3_carry(u32* w, u32 x0, u32 x1, u32 x2, u32 y) {
+    asm("mad.lo.cc.u32 %0, %7, %10, %0;\n\t"
+        "madc.hi.cc.u32 %1, %7, %10, %1;\n\t"
+        "madc.lo.cc.u32 %2, %8, %10, %2;\n\t"
+        "madc.hi.cc.u32 %3, %8, %10, %3;\n\t"
+        "madc.lo.cc.u32 %4, %9, %10, %4;\n\t"
+        "madc.hi.cc.u32 %5, %9, %10, %5;\n\t"
+        "addc.u32 %6, 0, 0;"
+        : "+r"(w[0]), "+r"(w[1]), "+r"(w[2]), "+r"(w[3]), "+r"(w[4]), "+r"(w[5]), "=r"(w[6])
+        : "r"(x0), "r"(x1), "r"(x2), "r"(y));
+}
+
+__device__ __forceinline__ void row3_top(u32* w, u32 x0, u32 x1, u32 x2, u32 y, u32 top) {
+    asm("mad.lo.cc.u32 %0, %6, %9, %0;\n\t"
+        "madc.hi.cc.u32 %1, %6, %9, %1;\n\t"
+        "madc.lo.cc.u32 %2, %7, %9, %2;\n\t"
+        "madc.hi.cc.u32 %3, %7, %9, %3;\n\t"
+        "madc.lo.cc.u32 %4, %8, %9, %10;\n\t"
+        "madc.hi.u32 %5, %8, %9, 0;"
+        : "+r"(w[0]), "+r"(w[1]), "+r"(w[2]), "+r"(w[3]), "=&r"(w[4]), "=r"(w[5])
+        : "r"(x0), "r"(x1), "r"(x2), "r"(y), "r"(top));
+}
+
+__device__ __forceinline__ void row4_carry(u32* w, u32 x0, u32 x1, u32 x2, u32 x3, u32 y) {
+    asm("mad.lo.cc.u32 %0, %9, %13, %0;\n\t"
+        "madc.hi.cc.u32 %1, %9, %13, %1;\n\t"
+        "madc.lo.cc.u32 %2, %10, %13, %2;\n\t"
+        "madc.hi.cc.u32 %3, %10, %13, %3;\n\t"
+        "madc.lo.cc.u32 %4, %11, %13, %4;\n\t"
+        "madc.hi.cc.u32 %5, %11, %13, %5;\n\t"
+        "madc.lo.cc.u32 %6, %12, %13, %6;\n\t"
+        "madc.hi.cc.u32 %7, %12, %13, %7;\n\t"
+        "addc.u32 %8, 0, 0;"
+        : "+r"(w[0]), "+r"(w[1]), "+r"(w[2]), "+r"(w[3]), "+r"(w[4]), "+r"(w[5]), "+r"(w[6]), "+r"(w[7]),
+          "=r"(w[8])
+        : "r"(x0), "r"(x1), "r"(x2), "r"(x3), "r"(y));
+}
+
+__device__ __forceinline__ void row4_top(u32* w, u32 x0, u32 x1, u32 x2, u32 x3, u32 y, u32 top) {
+    asm("mad.lo.cc.u32 %0, %8, %12, %0;\n\t"
+        "madc.hi.cc.u32 %1, %8, %12, %1;\n\t"
+        "madc.lo.cc.u32 %2, %9, %12, %2;\n\t"
+        "madc.hi.cc.u32 %3, %9, %12, %3;\n\t"
+        "madc.lo.cc.u32 %4, %10, %12, %4;\n\t"
+        "madc.hi.cc.u32 %5, %10, %12, %5;\n\t"
+        "madc.lo.cc.u32 %6, %11, %12, %13;\n\t"
+        "madc.hi.u32 %7, %11, %12, 0;"
+        : "+r"(w[0]), "+r"(w[1]), "+r"(w[2]), "+r"(w[3]), "+r"(w[4]), "+r"(w[5]), "=&r"(w[6]), "=r"(w[7])
+        : "r"(x0), "r"(x1), "r"(x2), "r"(x3), "r"(y), "r"(top));
+}
+
+// t = e + o·2^32 over n+1 words (t[0] = e[0]); the sum fits
+__device__ __forceinline__ void merge7(const u32* e, const u32* o, u32* t) {
+    t[0] = e[0];
+    asm("add.cc.u32 %0, %7, %14;\n\t"
+        "addc.cc.u32 %1, %8, %15;\n\t"
+        "addc.cc.u32 %2, %9, %16;\n\t"
+        "addc.cc.u32 %3, %10, %17;\n\t"
+        "addc.cc.u32 %4, %11, %18;\n\t"
+        "addc.cc.u32 %5, %12, %19;\n\t"
+        "addc.u32 %6, %13, %20;"
+        : "=r"(t[1]), "=r"(t[2]), "=r"(t[3]), "=r"(t[4]), "=r"(t[5]), "=r"(t[6]), "=r"(t[7])
+        : "r"(e[1]), "r"(e[2]), "r"(e[3]), "r"(e[4]), "r"(e[5]), "r"(e[6]), "r"(e[7]),
+          "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]), "r"(o[4]), "r"(o[5]), "r"(o[6]));
+}
+
+__device__ __forceinline__ void merge15(const u32* e, const u32* o, u32* t) {
+    t[0] = e[0];
+    asm("add.cc.u32 %0, %15, %30;\n\t"
+        "addc.cc.u32 %1, %16, %31;\n\t"
+        "addc.cc.u32 %2, %17, %32;\n\t"
+        "addc.cc.u32 %3, %18, %33;\n\t"
+        "addc.cc.u32 %4, %19, %34;\n\t"
+        "addc.cc.u32 %5, %20, %35;\n\t"
+        "addc.cc.u32 %6, %21, %36;\n\t"
+        "addc.cc.u32 %7, %22, %37;\n\t"
+        "addc.cc.u32 %8, %23, %38;\n\t"
+        "addc.cc.u32 %9, %24, %39;\n\t"
+        "addc.cc.u32 %10, %25, %40;\n\t"
+        "addc.cc.u32 %11, %26, %41;\n\t"
+        "addc.cc.u32 %12, %27, %42;\n\t"
+        "addc.cc.u32 %13, %28, %43;\n\t"
+        "addc.u32 %14, %29, %44;"
+        : "=r"(t[1]), "=r"(t[2]), "=r"(t[3]), "=r"(t[4]), "=r"(t[5]), "=r"(t[6]), "=r"(t[7]), "=r"(t[8]),
+          "=r"(t[9]), "=r"(t[10]), "=r"(t[11]), "=r"(t[12]), "=r"(t[13]), "=r"(t[14]), "=r"(t[15])
+        : "r"(e[1]), "r"(e[2]), "r"(e[3]), "r"(e[4]), "r"(e[5]), "r"(e[6]), "r"(e[7]), "r"(e[8]),
+          "r"(e[9]), "r"(e[10]), "r"(e[11]), "r"(e[12]), "r"(e[13]), "r"(e[14]), "r"(e[15]),
+          "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]),
+          "r"(o[8]), "r"(o[9]), "r"(o[10]), "r"(o[11]), "r"(o[12]), "r"(o[13]), "r"(o[14]));
+}
+
+// Fold a 512-bit product t[0..15] to 8 words: t_lo + 38·t_hi, then the top word again.  The
+// products 38·t[8+j] of even j extend the pairs of t_lo, those of odd j go one word up.
 __device__ __forceinline__ fe fe_reduce512(const u32 t[16]) {
+    u32 s[8], w[9];
+#pragma unroll
+    for (int k = 0; k < 4; k++) wide(s + 2 * k, t[9 + 2 * k], 38u);
+#pragma unroll
+    for (int i = 0; i < 8; i++) w[i] = t[i];
+    row4_carry(w, t[8], t[10], t[12], t[14], 38u);
     fe r;
-    u32 top;
-    // lo parts of 38·t[8+j] into words j, carries through
-    asm("mad.lo.cc.u32 %0, %9, 38, %17;\n\t"
-        "madc.lo.cc.u32 %1, %10, 38, %18;\n\t"
-        "madc.lo.cc.u32 %2, %11, 38, %19;\n\t"
-        "madc.lo.cc.u32 %3, %12, 38, %20;\n\t"
-        "madc.lo.cc.u32 %4, %13, 38, %21;\n\t"
-        "madc.lo.cc.u32 %5, %14, 38, %22;\n\t"
-        "madc.lo.cc.u32 %6, %15, 38, %23;\n\t"
-        "madc.lo.cc.u32 %7, %16, 38, %24;\n\t"
-        "addc.u32 %8, 0, 0;\n\t"
-        : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]), "=r"(r.v[6]),
-          "=r"(r.v[7]), "=r"(top)
-        : "r"(t[8]), "r"(t[9]), "r"(t[10]), "r"(t[11]), "r"(t[12]), "r"(t[13]), "r"(t[14]), "r"(t[15]),
-          "r"(t[0]), "r"(t[1]), "r"(t[2]), "r"(t[3]), "r"(t[4]), "r"(t[5]), "r"(t[6]), "r"(t[7]));
-    // hi parts of 38·t[8+j] into words j+1
-    asm("mad.hi.cc.u32 %1, %9, 38, %1;\n\t"
-        "madc.hi.cc.u32 %2, %10, 38, %2;\n\t"
-        "madc.hi.cc.u32 %3, %11, 38, %3;\n\t"
-        "madc.hi.cc.u32 %4, %12, 38, %4;\n\t"
-        "madc.hi.cc.u32 %5, %13, 38, %5;\n\t"
-        "madc.hi.cc.u32 %6, %14, 38, %6;\n\t"
-        "madc.hi.cc.u32 %7, %15, 38, %7;\n\t"
-        "madc.hi.u32 %8, %16, 38, %8;\n\t"
-        : "+r"(r.v[0]), "+r"(r.v[1]), "+r"(r.v[2]), "+r"(r.v[3]), "+r"(r.v[4]), "+r"(r.v[5]), "+r"(r.v[6]),
-          "+r"(r.v[7]), "+r"(top)
-        : "r"(t[8]), "r"(t[9]), "r"(t[10]), "r"(t[11]), "r"(t[12]), "r"(t[13]), "r"(t[14]), "r"(t[15]));
+    u32 top = w[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) r.v[i] = w[i];
+    asm("add.cc.u32 %0, %0, %8;\n\t"
+        "addc.cc.u32 %1, %1, %9;\n\t"
+        "addc.cc.u32 %2, %2, %10;\n\t"
+        "addc.cc.u32 %3, %3, %11;\n\t"
+        "addc.cc.u32 %4, %4, %12;\n\t"
+        "addc.cc.u32 %5, %5, %13;\n\t"
+        "addc.cc.u32 %6, %6, %14;\n\t"
+        "addc.u32 %7, %7, %15;"
+        : "+r"(r.v[1]), "+r"(r.v[2]), "+r"(r.v[3]), "+r"(r.v[4]), "+r"(r.v[5]), "+r"(r.v[6]), "+r"(r.v[7]), "+r"(top)
+        : "r"(s[0]), "r"(s[1]), "r"(s[2]), "r"(s[3]), "r"(s[4]), "r"(s[5]), "r"(s[6]), "r"(s[7]));
     // top < 40: fold 38·top; one more carry is possible and is folded as 38 without further carry
     u32 add = 38u * top, c2;
     asm("add.cc.u32 %0, %0, %9;\n\t"
@@ -145,66 +290,39 @@ __device__ __forceinline__ fe fe_reduce512(const u32 t[16]) {
     return r;
 }
 
-// One row of the operand-scanning product: t[i..i+8] += a · b_i.
-// Even-indexed a_j go in one carry chain (their lo/hi pairs tile words i..i+7),
-// odd-indexed a_j in a second chain (words i+1..i+8).
-#define MK32_ROW(I)                                                                                  \
-    asm("mad.lo.cc.u32 %0, %9, %13, %0;\n\t"                                                        \
-        "madc.hi.cc.u32 %1, %9, %13, %1;\n\t"                                                       \
-        "madc.lo.cc.u32 %2, %10, %13, %2;\n\t"                                                      \
-        "madc.hi.cc.u32 %3, %10, %13, %3;\n\t"                                                      \
-        "madc.lo.cc.u32 %4, %11, %13, %4;\n\t"                                                      \
-        "madc.hi.cc.u32 %5, %11, %13, %5;\n\t"                                                      \
-        "madc.lo.cc.u32 %6, %12, %13, %6;\n\t"                                                      \
-        "madc.hi.cc.u32 %7, %12, %13, %7;\n\t"                                                      \
-        "addc.u32 %8, %8, 0;\n\t"                                                                   \
-        : "+r"(t[I]), "+r"(t[I + 1]), "+r"(t[I + 2]), "+r"(t[I + 3]), "+r"(t[I + 4]), "+r"(t[I + 5]), \
-          "+r"(t[I + 6]), "+r"(t[I + 7]), "+r"(t[I + 8])                                            \
-        : "r"(a.v[0]), "r"(a.v[2]), "r"(a.v[4]), "r"(a.v[6]), "r"(b.v[I]));                         \
-    asm("mad.lo.cc.u32 %0, %8, %12, %0;\n\t"                                                        \
-        "madc.hi.cc.u32 %1, %8, %12, %1;\n\t"                                                       \
-        "madc.lo.cc.u32 %2, %9, %12, %2;\n\t"                                                       \
-        "madc.hi.cc.u32 %3, %9, %12, %3;\n\t"                                                       \
-        "madc.lo.cc.u32 %4, %10, %12, %4;\n\t"                                                      \
-        "madc.hi.cc.u32 %5, %10, %12, %5;\n\t"                                                      \
-        "madc.lo.cc.u32 %6, %11, %12, %6;\n\t"                                                      \
-        "madc.hi.u32 %7, %11, %12, %7;\n\t"                                                         \
-        : "+r"(t[I + 1]), "+r"(t[I + 2]), "+r"(t[I + 3]), "+r"(t[I + 4]), "+r"(t[I + 5]),             \
-          "+r"(t[I + 6]), "+r"(t[I + 7]), "+r"(t[I + 8])                                            \
-        : "r"(a.v[1]), "r"(a.v[3]), "r"(a.v[5]), "r"(a.v[7]), "r"(b.v[I]));
-
-// r = a·b mod p (as a value below 2^256), schoolbook: 64 lo + 64 hi products
+// r = a·b mod p (as a value below 2^256), schoolbook: 64 products.  Limb b_i meets the limbs
+// a_j of its own parity on the even words and the others on the odd ones; each row's chain either
+// opens a new top pair or leaves its carry there for the next row.
 __device__ __forceinline__ fe fe_mul_schoolbook(const fe& a, const fe& b) {
-    u32 t[16];
+    u32 e[16], o[16], t[16];
+    const u32 a0 = a.v[0], a1 = a.v[1], a2 = a.v[2], a3 = a.v[3], a4 = a.v[4], a5 = a.v[5], a6 = a.v[6], a7 = a.v[7];
+    wide(e, a0, b.v[0]); wide(e + 2, a2, b.v[0]); wide(e + 4, a4, b.v[0]); wide(e + 6, a6, b.v[0]);
+    wide(o, a1, b.v[0]); wide(o + 2, a3, b.v[0]); wide(o + 4, a5, b.v[0]); wide(o + 6, a7, b.v[0]);
+    row4_top(e + 2, a1, a3, a5, a7, b.v[1], 0u);
+    row4_carry(o, a0, a2, a4, a6, b.v[1]);
 #pragma unroll
-    for (int i = 0; i < 16; i++) t[i] = 0;
-    // after row I the partial sum is below 2^(32(I+9)), so word I+8 absorbs the final carry
-    MK32_ROW(0) MK32_ROW(1) MK32_ROW(2) MK32_ROW(3) MK32_ROW(4) MK32_ROW(5) MK32_ROW(6) MK32_ROW(7)
+    for (int i = 2; i < 8; i += 2) {
+        row4_carry(e + i, a0, a2, a4, a6, b.v[i]);
+        row4_top(o + i, a1, a3, a5, a7, b.v[i], o[i + 6]);
+        row4_top(e + i + 2, a1, a3, a5, a7, b.v[i + 1], e[i + 8]);
+        row4_carry(o + i, a0, a2, a4, a6, b.v[i + 1]);
+    }
+    merge15(e, o, t);
     return fe_reduce512(t);
 }
 
-// One row of a 128 x 128-bit product: T[I..I+4] += X · Y_I, the even X limbs in one carry
-// chain and the odd ones in a second; after row I the sum is below 2^(32(I+5)).
-#define MK32_ROW4(T, X, Y, I)                                                                        \
-    asm("mad.lo.cc.u32 %0, %5, %7, %0;\n\t"                                                          \
-        "madc.hi.cc.u32 %1, %5, %7, %1;\n\t"                                                         \
-        "madc.lo.cc.u32 %2, %6, %7, %2;\n\t"                                                         \
-        "madc.hi.cc.u32 %3, %6, %7, %3;\n\t"                                                         \
-        "addc.u32 %4, %4, 0;\n\t"                                                                    \
-        : "+r"(T[I]), "+r"(T[I + 1]), "+r"(T[I + 2]), "+r"(T[I + 3]), "+r"(T[I + 4])                 \
-        : "r"(X[0]), "r"(X[2]), "r"(Y[I]));                                                          \
-    asm("mad.lo.cc.u32 %0, %4, %6, %0;\n\t"                                                          \
-        "madc.hi.cc.u32 %1, %4, %6, %1;\n\t"                                                         \
-        "madc.lo.cc.u32 %2, %5, %6, %2;\n\t"                                                         \
-        "madc.hi.u32 %3, %5, %6, %3;\n\t"                                                            \
-        : "+r"(T[I + 1]), "+r"(T[I + 2]), "+r"(T[I + 3]), "+r"(T[I + 4])                             \
-        : "r"(X[1]), "r"(X[3]), "r"(Y[I]));
-
-// t[0..7] = x · y for 128-bit x, y (four limbs each): 16 lo + 16 hi products
+// t[0..7] = x · y for 128-bit x, y (four limbs each): 16 products
 __device__ __forceinline__ void mul128(const u32 x[4], const u32 y[4], u32 t[8]) {
-#pragma unroll
-    for (int i = 0; i < 8; i++) t[i] = 0;
-    MK32_ROW4(t, x, y, 0) MK32_ROW4(t, x, y, 1) MK32_ROW4(t, x, y, 2) MK32_ROW4(t, x, y, 3)
+    u32 e[8], o[8];
+    wide(e, x[0], y[0]); wide(e + 2, x[2], y[0]);
+    wide(o, x[1], y[0]); wide(o + 2, x[3], y[0]);
+    row2_top(e + 2, x[1], x[3], y[1], 0u);
+    row2_carry(o, x[0], x[2], y[1]);
+    row2_carry(e + 2, x[0], x[2], y[2]);
+    row2_top(o + 2, x[1], x[3], y[2], o[4]);
+    row2_top(e + 4, x[1], x[3], y[3], e[6]);
+    row2_carry(o + 2, x[0], x[2], y[3]);
+    merge7(e, o, t);
 }
 
 // d = |x - y| for 128-bit x, y; returns all ones when x < y, else 0
@@ -308,111 +426,28 @@ __device__ __forceinline__ fe fe_mul_karatsuba(const fe& a, const fe& b) {
 // r = a·b mod p (as a value below 2^256)
 __device__ __forceinline__ fe fe_mul(const fe& a, const fe& b) { return fe_mul_schoolbook(a, b); }
 
-// r = a·b mod p in the form a kernel picks at compile time: Karatsuba when K.  Both forms
-// return the same words for the same inputs.
-template <bool K>
-__device__ __forceinline__ fe fe_mul_as(const fe& a, const fe& b) {
-    if constexpr (K) return fe_mul_karatsuba(a, b);
-    else return fe_mul_schoolbook(a, b);
-}
-
-// r = a^2 mod p: the 28 cross products a_i·a_j (i < j) in per-row carry chains (row i
-// adds a_i·a_(i+1..7) into t[2i+1 .. i+8]; the row's partial sum stays below 2^(32(i+9)),
-// so word i+8 absorbs its carry), then doubled with funnel shifts, plus the 8 diagonal
-// squares in one chain: 72 multiply-adds before the fold instead of 128.
+// r = a^2 mod p: the 28 cross products a_i·a_j (i < j) in even/odd accumulators, doubled with
+// funnel shifts, plus the 8 diagonal squares (even words) in one chain: 36 products before the
+// fold instead of 64.
 __device__ __forceinline__ fe fe_sq(const fe& a) {
-    u32 t[16];
-#pragma unroll
-    for (int i = 0; i < 16; i++) t[i] = 0;
-    asm("mad.lo.cc.u32 %0, %7, %8, %0;\n\t"
-        "madc.hi.cc.u32 %1, %7, %8, %1;\n\t"
-        "madc.lo.cc.u32 %2, %7, %9, %2;\n\t"
-        "madc.hi.cc.u32 %3, %7, %9, %3;\n\t"
-        "madc.lo.cc.u32 %4, %7, %10, %4;\n\t"
-        "madc.hi.cc.u32 %5, %7, %10, %5;\n\t"
-        "addc.u32 %6, %6, 0;\n\t"
-        : "+r"(t[2]), "+r"(t[3]), "+r"(t[4]), "+r"(t[5]), "+r"(t[6]), "+r"(t[7]), "+r"(t[8])
-        : "r"(a.v[0]), "r"(a.v[2]), "r"(a.v[4]), "r"(a.v[6]));
-    asm("mad.lo.cc.u32 %0, %8, %9, %0;\n\t"
-        "madc.hi.cc.u32 %1, %8, %9, %1;\n\t"
-        "madc.lo.cc.u32 %2, %8, %10, %2;\n\t"
-        "madc.hi.cc.u32 %3, %8, %10, %3;\n\t"
-        "madc.lo.cc.u32 %4, %8, %11, %4;\n\t"
-        "madc.hi.cc.u32 %5, %8, %11, %5;\n\t"
-        "madc.lo.cc.u32 %6, %8, %12, %6;\n\t"
-        "madc.hi.u32 %7, %8, %12, %7;\n\t"
-        : "+r"(t[1]), "+r"(t[2]), "+r"(t[3]), "+r"(t[4]), "+r"(t[5]), "+r"(t[6]), "+r"(t[7]), "+r"(t[8])
-        : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[3]), "r"(a.v[5]), "r"(a.v[7]));
-    asm("mad.lo.cc.u32 %0, %7, %8, %0;\n\t"
-        "madc.hi.cc.u32 %1, %7, %8, %1;\n\t"
-        "madc.lo.cc.u32 %2, %7, %9, %2;\n\t"
-        "madc.hi.cc.u32 %3, %7, %9, %3;\n\t"
-        "madc.lo.cc.u32 %4, %7, %10, %4;\n\t"
-        "madc.hi.cc.u32 %5, %7, %10, %5;\n\t"
-        "addc.u32 %6, %6, 0;\n\t"
-        : "+r"(t[3]), "+r"(t[4]), "+r"(t[5]), "+r"(t[6]), "+r"(t[7]), "+r"(t[8]), "+r"(t[9])
-        : "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[4]), "r"(a.v[6]));
-    asm("mad.lo.cc.u32 %0, %6, %7, %0;\n\t"
-        "madc.hi.cc.u32 %1, %6, %7, %1;\n\t"
-        "madc.lo.cc.u32 %2, %6, %8, %2;\n\t"
-        "madc.hi.cc.u32 %3, %6, %8, %3;\n\t"
-        "madc.lo.cc.u32 %4, %6, %9, %4;\n\t"
-        "madc.hi.u32 %5, %6, %9, %5;\n\t"
-        : "+r"(t[4]), "+r"(t[5]), "+r"(t[6]), "+r"(t[7]), "+r"(t[8]), "+r"(t[9])
-        : "r"(a.v[1]), "r"(a.v[3]), "r"(a.v[5]), "r"(a.v[7]));
-    asm("mad.lo.cc.u32 %0, %5, %6, %0;\n\t"
-        "madc.hi.cc.u32 %1, %5, %6, %1;\n\t"
-        "madc.lo.cc.u32 %2, %5, %7, %2;\n\t"
-        "madc.hi.cc.u32 %3, %5, %7, %3;\n\t"
-        "addc.u32 %4, %4, 0;\n\t"
-        : "+r"(t[6]), "+r"(t[7]), "+r"(t[8]), "+r"(t[9]), "+r"(t[10])
-        : "r"(a.v[2]), "r"(a.v[4]), "r"(a.v[6]));
-    asm("mad.lo.cc.u32 %0, %6, %7, %0;\n\t"
-        "madc.hi.cc.u32 %1, %6, %7, %1;\n\t"
-        "madc.lo.cc.u32 %2, %6, %8, %2;\n\t"
-        "madc.hi.cc.u32 %3, %6, %8, %3;\n\t"
-        "madc.lo.cc.u32 %4, %6, %9, %4;\n\t"
-        "madc.hi.u32 %5, %6, %9, %5;\n\t"
-        : "+r"(t[5]), "+r"(t[6]), "+r"(t[7]), "+r"(t[8]), "+r"(t[9]), "+r"(t[10])
-        : "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[5]), "r"(a.v[7]));
-    asm("mad.lo.cc.u32 %0, %5, %6, %0;\n\t"
-        "madc.hi.cc.u32 %1, %5, %6, %1;\n\t"
-        "madc.lo.cc.u32 %2, %5, %7, %2;\n\t"
-        "madc.hi.cc.u32 %3, %5, %7, %3;\n\t"
-        "addc.u32 %4, %4, 0;\n\t"
-        : "+r"(t[7]), "+r"(t[8]), "+r"(t[9]), "+r"(t[10]), "+r"(t[11])
-        : "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[6]));
-    asm("mad.lo.cc.u32 %0, %4, %5, %0;\n\t"
-        "madc.hi.cc.u32 %1, %4, %5, %1;\n\t"
-        "madc.lo.cc.u32 %2, %4, %6, %2;\n\t"
-        "madc.hi.u32 %3, %4, %6, %3;\n\t"
-        : "+r"(t[8]), "+r"(t[9]), "+r"(t[10]), "+r"(t[11])
-        : "r"(a.v[3]), "r"(a.v[5]), "r"(a.v[7]));
-    asm("mad.lo.cc.u32 %0, %3, %4, %0;\n\t"
-        "madc.hi.cc.u32 %1, %3, %4, %1;\n\t"
-        "addc.u32 %2, %2, 0;\n\t"
-        : "+r"(t[10]), "+r"(t[11]), "+r"(t[12])
-        : "r"(a.v[4]), "r"(a.v[6]));
-    asm("mad.lo.cc.u32 %0, %4, %5, %0;\n\t"
-        "madc.hi.cc.u32 %1, %4, %5, %1;\n\t"
-        "madc.lo.cc.u32 %2, %4, %6, %2;\n\t"
-        "madc.hi.u32 %3, %4, %6, %3;\n\t"
-        : "+r"(t[9]), "+r"(t[10]), "+r"(t[11]), "+r"(t[12])
-        : "r"(a.v[4]), "r"(a.v[5]), "r"(a.v[7]));
-    asm("mad.lo.cc.u32 %0, %3, %4, %0;\n\t"
-        "madc.hi.cc.u32 %1, %3, %4, %1;\n\t"
-        "addc.u32 %2, %2, 0;\n\t"
-        : "+r"(t[11]), "+r"(t[12]), "+r"(t[13])
-        : "r"(a.v[5]), "r"(a.v[6]));
-    asm("mad.lo.cc.u32 %0, %2, %3, %0;\n\t"
-        "madc.hi.u32 %1, %2, %3, %1;\n\t"
-        : "+r"(t[12]), "+r"(t[13])
-        : "r"(a.v[5]), "r"(a.v[7]));
-    asm("mad.lo.cc.u32 %0, %2, %3, %0;\n\t"
-        "madc.hi.u32 %1, %2, %3, %1;\n\t"
-        : "+r"(t[13]), "+r"(t[14])
-        : "r"(a.v[6]), "r"(a.v[7]));
-
+    u32 e[16], o[16], t[16];
+    const u32 a0 = a.v[0], a1 = a.v[1], a2 = a.v[2], a3 = a.v[3], a4 = a.v[4], a5 = a.v[5], a6 = a.v[6], a7 = a.v[7];
+    e[0] = e[1] = e[14] = e[15] = 0;
+    wide(e + 2, a2, a0); wide(e + 4, a4, a0); wide(e + 6, a6, a0);
+    wide(o, a1, a0); wide(o + 2, a3, a0); wide(o + 4, a5, a0); wide(o + 6, a7, a0);
+    row3_top(e + 4, a3, a5, a7, a1, 0u);
+    row3_carry(o + 2, a2, a4, a6, a1);
+    row2_carry(e + 6, a4, a6, a2);
+    row3_top(o + 4, a3, a5, a7, a2, o[8]);
+    row2_top(e + 8, a5, a7, a3, e[10]);
+    row2_carry(o + 6, a4, a6, a3);
+    row1_carry(e + 10, a6, a4);
+    row2_top(o + 8, a5, a7, a4, o[10]);
+    row1_top(e + 12, a7, a5, e[12]);
+    row1_carry(o + 10, a6, a5);
+    row1_top(o + 12, a7, a6, o[12]);
+    o[14] = 0;  // the cross sum is below 2^511
+    merge15(e, o, t);
     // t = 2·t (the cross sum is below 2^511)
 #pragma unroll
     for (int k = 15; k > 0; k--) t[k] = __funnelshift_l(t[k - 1], t[k], 1);

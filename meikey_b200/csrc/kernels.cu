@@ -28,12 +28,6 @@ using mk32::niels;
 using mk32::u32;
 using mk32::u64;
 
-// Field-multiply form of the secure path (comb additions, thread batches and back-sweep): one
-// level of Karatsuba, 48 lo + 48 hi products a multiplication instead of 64 + 64, with the same
-// results.  On B200 it is the faster form there; the incremental path, with few multiplies
-// between its other work, runs faster with the schoolbook form and keeps it.
-constexpr bool SECURE_KARATSUBA = true;
-
 // ---------------------------------------------------------------------------
 // shared helpers
 // ---------------------------------------------------------------------------
@@ -207,11 +201,11 @@ __device__ __forceinline__ void comb_mul(const uint4* __restrict__ table, const 
         fetch_entry(slot, (row + 1) & 1, table, entry_index(g, row + 1, dn));
         wait_entries<1>();
         niels n = read_entry(slot, row & 1);
-        P = mk32::ge_add_niels<SECURE_KARATSUBA>(P, n, d < 0);
+        P = mk32::ge_add_niels(P, n, d < 0);
     }
     wait_entries<0>();
     niels n = read_entry(slot, (rows - 1) & 1);
-    mk32::ge_add_niels_frac<SECURE_KARATSUBA>(P, n, yn, yd, xn, xd);
+    mk32::ge_add_niels_frac(P, n, yn, yd, xn, xd);
 }
 
 // comb_mul with one 8-round step of the SHA-512 `run` (the next iteration's seed) in every
@@ -245,11 +239,11 @@ __device__ __forceinline__ void comb_mul_sha(const uint4* __restrict__ table, co
         wait_entries<1>();
         niels n = read_entry(slot, row & 1);
         mkh::sha_run_step(run, 8u * (row - 1));
-        P = mk32::ge_add_niels<SECURE_KARATSUBA>(P, n, d < 0);
+        P = mk32::ge_add_niels(P, n, d < 0);
     }
     wait_entries<0>();
     niels n = read_entry(slot, (rows - 1) & 1);
-    mk32::ge_add_niels_frac<SECURE_KARATSUBA>(P, n, yn, yd, nullptr, nullptr);
+    mk32::ge_add_niels_frac(P, n, yn, yd, nullptr, nullptr);
 }
 
 // 6-bit values of the 44-character base64 tail of the key blob (0x20 then the key),
@@ -453,11 +447,11 @@ __device__ __forceinline__ void comb_mul_smem(const uint4* stab, const CombGeom&
 #pragma unroll 1
     for (u32 row = 1; row + 1 < rows; row++) {
         d = next_digit(g, m, row, carry);
-        P = mk32::ge_add_niels<SECURE_KARATSUBA>(P, smem_niels(stab + entry_index(g, row, d) * 6), d < 0);
+        P = mk32::ge_add_niels(P, smem_niels(stab + entry_index(g, row, d) * 6), d < 0);
     }
     // the top row's digit is unsigned: the carry lands in it unchanged
     d = (int)bits_at(m, g.offset[rows - 1], g.width[rows - 1]) + carry;
-    mk32::ge_add_niels_frac<SECURE_KARATSUBA>(P, smem_niels(stab + entry_index(g, rows - 1, d) * 6), yn, yd, nullptr, nullptr);
+    mk32::ge_add_niels_frac(P, smem_niels(stab + entry_index(g, rows - 1, d) * 6), yn, yd, nullptr, nullptr);
 }
 
 // Comb multiplies of the KPT scalars (IMAD work) into the batch; STAB: from the table in
@@ -475,8 +469,8 @@ __device__ __forceinline__ void combs(const KeyLaunch& L, const CombGeom& g, con
             b.a[0] = num;
             run = b.den[0];
         } else {
-            b.a[j] = mk32::fe_mul_as<SECURE_KARATSUBA>(num, run);
-            run = mk32::fe_mul_as<SECURE_KARATSUBA>(run, b.den[j]);
+            b.a[j] = mk32::fe_mul(num, run);
+            run = mk32::fe_mul(run, b.den[j]);
         }
     }
     b.prod = run;
@@ -526,24 +520,23 @@ __device__ __forceinline__ void combs_sha(const KeyLaunch& L, const CombGeom& g,
             b.a[0] = num;
             run = b.den[0];
         } else {
-            b.a[j] = mk32::fe_mul_as<SECURE_KARATSUBA>(num, run);
-            run = mk32::fe_mul_as<SECURE_KARATSUBA>(run, b.den[j]);
+            b.a[j] = mk32::fe_mul(num, run);
+            run = mk32::fe_mul(run, b.den[j]);
         }
     }
     b.prod = run;
 }
 
 // Backward pass: `inv` is 1/(product of the batch's denominators); yields each key's
-// canonical y (sign bit 0), tests the needles and reports candidate hits.  K: Karatsuba
-// multiplies.
-template <int KPT, bool K = false>
+// canonical y (sign bit 0), tests the needles and reports candidate hits.
+template <int KPT>
 __device__ __forceinline__ void backward(const KeyLaunch& L, const MatchSet& ms, const u32* lane_masks, u64 first,
                                          const Batch<KPT>& b, fe inv, u32& sink) {
 #pragma unroll 1
     for (int j = KPT - 1; j >= 0; j--) {
         u32 pk[8];
-        mk32::fe_to_words(mk32::fe_mul_as<K>(b.a[j], inv), pk);
-        if (j > 0) inv = mk32::fe_mul_as<K>(inv, b.den[j]);
+        mk32::fe_to_words(mk32::fe_mul(b.a[j], inv), pk);
+        if (j > 0) inv = mk32::fe_mul(inv, b.den[j]);
         sink ^= pk[7];
         u64 hw[2];
         match_key(ms, lane_masks, pk, hw);
@@ -819,7 +812,7 @@ __global__ void __launch_bounds__(BLOCK, 512 / BLOCK) k_search(const KeyLaunch L
         const int b = it & 1;
         if (it + 1 < iters && it + 1 < stop_iter) produce(it + 1);
         if (!inverts(it)) bar_sync(3 + b, BLOCK);
-        backward<KPT, !INCR && SECURE_KARATSUBA>(L, ms, ms.narrow ? lane_masks : nullptr, first_of(it), batch[b],
+        backward<KPT>(L, ms, ms.narrow ? lane_masks : nullptr, first_of(it), batch[b],
                                                  prod[b][tid], sink);
         if (it + 1 >= iters || it + 1 >= stop_iter) break;
     }
@@ -980,8 +973,8 @@ __global__ void __launch_bounds__(BLOCK, 1) k_search_hw(const KeyLaunch L) {
                 bt.a[0] = num;
                 run = bt.den[0];
             } else {
-                bt.a[j] = mk32::fe_mul_as<SECURE_KARATSUBA>(num, run);
-                run = mk32::fe_mul_as<SECURE_KARATSUBA>(run, bt.den[j]);
+                bt.a[j] = mk32::fe_mul(num, run);
+                run = mk32::fe_mul(run, bt.den[j]);
             }
         }
         bt.prod = run;
@@ -993,7 +986,7 @@ __global__ void __launch_bounds__(BLOCK, 1) k_search_hw(const KeyLaunch L) {
         const int b = it & 1;
         if (it + 1 < iters && it + 1 < stop_iter) produce(it + 1);
         bar_sync(3 + b, B_PIPE);
-        backward<KPT, SECURE_KARATSUBA>(L, ms, ms.narrow ? lane_masks : nullptr, first_of(it, gid), batch[b],
+        backward<KPT>(L, ms, ms.narrow ? lane_masks : nullptr, first_of(it, gid), batch[b],
                                         prod[b][tid], sink);
         if (it + 1 >= iters || it + 1 >= stop_iter) break;
     }
@@ -1216,46 +1209,39 @@ __global__ void __launch_bounds__(256) k_mad_lo_peak(uint32_t iters, uint32_t x,
     out[(uint64_t)blockIdx.x * blockDim.x + threadIdx.x] = s;
 }
 
-// Peak of the field multiply's own instruction shape: one row of a schoolbook product,
-// acc[0..8] += a·b[0..7] as a mad.lo.cc/madc.lo.cc chain followed by the madc.hi.cc chain
-// one word up (16 multiply-adds and one addc), on four independent accumulators per thread.
-// The multiplier a is the accumulator's top word plus the iteration, so no product can be
-// hoisted out of the loop.
+// Peak of the field multiply's own instruction shape: four products a·b_i accumulated on four
+// aligned pairs as one mad.lo.cc/madc.hi.cc chain (rows of even/odd accumulators, fe32.cuh), on
+// four independent accumulators per thread.  The multiplier a is the accumulator's top word plus
+// the iteration, so no product can be hoisted out of the loop.
 __global__ void __launch_bounds__(256) k_mad_chain_peak(uint32_t iters, uint32_t seed, uint32_t* out) {
-    uint32_t acc[4][9], b[8];
+    uint32_t acc[4][9], b[4];
 #pragma unroll
-    for (int i = 0; i < 8; i++) b[i] = seed * (2 * i + 1) + threadIdx.x;
+    for (int i = 0; i < 4; i++) b[i] = seed * (2 * i + 1) + threadIdx.x;
 #pragma unroll
     for (int q = 0; q < 4; q++)
 #pragma unroll
         for (int i = 0; i < 9; i++) acc[q][i] = threadIdx.x ^ (q * 9 + i);
     for (uint32_t it = 0; it < iters; it++) {
 #pragma unroll
-        for (int q = 0; q < 4; q++) {
-            uint32_t* t = acc[q];
-            const uint32_t a = t[8] + it;
-            asm volatile(
-                "mad.lo.cc.u32 %0, %9, %10, %0;\n\t"
-                "madc.lo.cc.u32 %1, %9, %11, %1;\n\t"
-                "madc.lo.cc.u32 %2, %9, %12, %2;\n\t"
-                "madc.lo.cc.u32 %3, %9, %13, %3;\n\t"
-                "madc.lo.cc.u32 %4, %9, %14, %4;\n\t"
-                "madc.lo.cc.u32 %5, %9, %15, %5;\n\t"
-                "madc.lo.cc.u32 %6, %9, %16, %6;\n\t"
-                "madc.lo.cc.u32 %7, %9, %17, %7;\n\t"
-                "addc.u32 %8, %8, 0;\n\t"
-                "mad.hi.cc.u32 %1, %9, %10, %1;\n\t"
-                "madc.hi.cc.u32 %2, %9, %11, %2;\n\t"
-                "madc.hi.cc.u32 %3, %9, %12, %3;\n\t"
-                "madc.hi.cc.u32 %4, %9, %13, %4;\n\t"
-                "madc.hi.cc.u32 %5, %9, %14, %5;\n\t"
-                "madc.hi.cc.u32 %6, %9, %15, %6;\n\t"
-                "madc.hi.cc.u32 %7, %9, %16, %7;\n\t"
-                "madc.hi.u32 %8, %9, %17, %8;\n\t"
-                : "+r"(t[0]), "+r"(t[1]), "+r"(t[2]), "+r"(t[3]), "+r"(t[4]), "+r"(t[5]), "+r"(t[6]), "+r"(t[7]),
-                  "+r"(t[8])
-                : "r"(a), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]), "r"(b[4]), "r"(b[5]), "r"(b[6]), "r"(b[7]));
-        }
+        for (int r = 0; r < 2; r++)
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                uint32_t* t = acc[q];
+                const uint32_t a = t[8] + it;
+                asm volatile(
+                    "mad.lo.cc.u32 %0, %9, %10, %0;\n\t"
+                    "madc.hi.cc.u32 %1, %9, %10, %1;\n\t"
+                    "madc.lo.cc.u32 %2, %9, %11, %2;\n\t"
+                    "madc.hi.cc.u32 %3, %9, %11, %3;\n\t"
+                    "madc.lo.cc.u32 %4, %9, %12, %4;\n\t"
+                    "madc.hi.cc.u32 %5, %9, %12, %5;\n\t"
+                    "madc.lo.cc.u32 %6, %9, %13, %6;\n\t"
+                    "madc.hi.cc.u32 %7, %9, %13, %7;\n\t"
+                    "addc.u32 %8, %8, 0;\n\t"
+                    : "+r"(t[0]), "+r"(t[1]), "+r"(t[2]), "+r"(t[3]), "+r"(t[4]), "+r"(t[5]), "+r"(t[6]), "+r"(t[7]),
+                      "+r"(t[8])
+                    : "r"(a), "r"(b[0]), "r"(b[1]), "r"(b[2]), "r"(b[3]));
+            }
     }
     uint32_t s = 0;
 #pragma unroll
@@ -1430,7 +1416,7 @@ __global__ void __launch_bounds__(256) k_fe_mul_rate(uint32_t iters, uint32_t se
         for (int q = 0; q < 4; q++) a[q] = mk32::fe_from_words(wa[q]);
         for (uint32_t it = 0; it < iters; it++)
 #pragma unroll
-            for (int q = 0; q < 4; q++) a[q] = mk32::fe_mul_as<RADIX == 33>(a[q], b);
+            for (int q = 0; q < 4; q++) a[q] = RADIX == 33 ? mk32::fe_mul_karatsuba(a[q], b) : mk32::fe_mul(a[q], b);
 #pragma unroll
         for (int q = 0; q < 4; q++) {
             uint32_t w[8];

@@ -87,10 +87,9 @@ cudaError_t measure_field_mul_forms(int sms, cudaStream_t st, double* schoolbook
 // synchronizes `st`.
 cudaError_t field_mul_pairs(const uint32_t* a, const uint32_t* b, uint32_t n, uint32_t* out_s, uint32_t* out_k,
                             cudaStream_t st);
-// Integer multiply-adds of one radix-2^32 field multiplication in each form (products and the
-// fold by 38) and of a squaring; the secure path multiplies in the Karatsuba form.
+// Integer multiply-adds (32-bit halves) of one radix-2^32 field multiplication (products and the
+// fold by 38) and of a squaring.
 constexpr double MADS_MUL_SCHOOLBOOK = 64 + 64 + 16;
-constexpr double MADS_MUL_KARATSUBA = 48 + 48 + 16;
 constexpr double MADS_SQUARE = 72 + 16;
 // The kernel of a variant and its dynamic shared memory (for graph nodes); sets the
 // kernel's shared-memory limit like launch_keys does.
