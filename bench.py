@@ -703,7 +703,7 @@ def measure(args, workload, steps, e2e_steps, dist, world, rank, local, cpu_seco
             "frac_of_mad_lo": achieved / (peak_lo / 1e12) if peak_lo else None,
             "work_per_key": {"field_muls": field_muls, "int_mads": mads_per_key,
                              "mul_form": "schoolbook in even/odd accumulators: 144 MADs (72 wide products) a "
-                                         "multiplication, squarings 88"},
+                                         "multiplication; inversions by division steps"},
             # the peak's pieces, each on independent chains or carry-linked rows (Tmad/s)
             "imad_pieces": {k: v / 1e12 for k, v in pieces.items()} if pieces else None,
             "kernel_ms_per_launch": ms_local / (steps * launches),

@@ -981,8 +981,8 @@ int mk_ctx_work_per_key(const mk_ctx* c, int seed_source, double* field_muls, do
     if (!c || !field_muls || !int_mads || seed_source < MK_SEED_CHACHA20 || seed_source > MK_SEED_INCREMENTAL)
         return MK_ERR_BAD_ARG;
     // radix-2^32 costs: a schoolbook multiplication is 64 mad.lo + 64 mad.hi (8x8 limbs) + 16
-    // (fold by 38), a squaring 28 cross products + 8 diagonal ones (72) + 16.
-    const double MUL = mkb::MADS_MUL_SCHOOLBOOK, SQ = mkb::MADS_SQUARE;
+    // (fold by 38).
+    const double MUL = mkb::MADS_MUL_SCHOOLBOOK;
     const double kpt = c->kpt, rows = c->geom.rows;
     const double ct = mkb::search_threads(c->block, c->layout);
     // comb: row 0 is free, full additions cost 7 multiplications, the last one 3
@@ -997,12 +997,11 @@ int mk_ctx_work_per_key(const mk_ctx* c, int seed_source, double* field_muls, do
         comb = (3.0 * (kpt - 1) + 7.0) / kpt;
     }
     // pooled inversion by the CTA's inverting warp: `pools` lanes, each over `groups` thread
-    // products, 3(groups-1) multiplications and one inversion (254 squarings + 11 multiplications)
+    // products, 3(groups-1) multiplications and one inversion by division steps
     const double pools = c->inv_pools, groups = ct / pools;
-    double pool_mul = pools * (3.0 * (groups - 1) + 11.0) / (ct * kpt);
-    double pool_sq = pools * 254.0 / (ct * kpt);
-    *field_muls = comb + batch + pool_mul + pool_sq;
-    *int_mads = (comb + batch + pool_mul) * MUL + pool_sq * SQ;
+    double pool_mul = pools * 3.0 * (groups - 1) / (ct * kpt);
+    *field_muls = comb + batch + pool_mul;
+    *int_mads = *field_muls * MUL + pools * mkb::MADS_INVERT / (ct * kpt);
     return MK_OK;
 }
 

@@ -124,21 +124,6 @@ __device__ __forceinline__ void wide(u32* w, u32 x, u32 y) {
 //   rown_carry  every pair holds a sum already; the carry starts the next pair, w[2n] = carry;
 //   rown_top    the last pair is new but for a carry `top` (0 or 1) of an earlier row; it cannot
 //               overflow (x·y + 2 < 2^64).
-__device__ __forceinline__ void row1_carry(u32* w, u32 x0, u32 y) {
-    asm("mad.lo.cc.u32 %0, %3, %4, %0;\n\t"
-        "madc.hi.cc.u32 %1, %3, %4, %1;\n\t"
-        "addc.u32 %2, 0, 0;"
-        : "+r"(w[0]), "+r"(w[1]), "=r"(w[2])
-        : "r"(x0), "r"(y));
-}
-
-__device__ __forceinline__ void row1_top(u32* w, u32 x0, u32 y, u32 top) {
-    asm("mad.lo.cc.u32 %0, %2, %3, %4;\n\t"
-        "madc.hi.u32 %1, %2, %3, 0;"
-        : "=&r"(w[0]), "=r"(w[1])
-        : "r"(x0), "r"(y), "r"(top));
-}
-
 __device__ __forceinline__ void row2_carry(u32* w, u32 x0, u32 x1, u32 y) {
     asm("mad.lo.cc.u32 %0, %5, %7, %0;\n\t"
         "madc.hi.cc.u32 %1, %5, %7, %1;\n\t"
@@ -156,29 +141,6 @@ __device__ __forceinline__ void row2_top(u32* w, u32 x0, u32 x1, u32 y, u32 top)
         "madc.hi.u32 %3, %5, %6, 0;"
         : "+r"(w[0]), "+r"(w[1]), "=&r"(w[2]), "=r"(w[3])
         : "r"(x0), "r"(x1), "r"(y), "r"(top));
-}
-
-__device__ __forceinline__ void row3_carry(u32* w, u32 x0, u32 x1, u32 x2, u32 y) {
-    asm("mad.lo.cc.u32 %0, %7, %10, %0;\n\t"
-        "madc.hi.cc.u32 %1, %7, %10, %1;\n\t"
-        "madc.lo.cc.u32 %2, %8, %10, %2;\n\t"
-        "madc.hi.cc.u32 %3, %8, %10, %3;\n\t"
-        "madc.lo.cc.u32 %4, %9, %10, %4;\n\t"
-        "madc.hi.cc.u32 %5, %9, %10, %5;\n\t"
-        "addc.u32 %6, 0, 0;"
-        : "+r"(w[0]), "+r"(w[1]), "+r"(w[2]), "+r"(w[3]), "+r"(w[4]), "+r"(w[5]), "=r"(w[6])
-        : "r"(x0), "r"(x1), "r"(x2), "r"(y));
-}
-
-__device__ __forceinline__ void row3_top(u32* w, u32 x0, u32 x1, u32 x2, u32 y, u32 top) {
-    asm("mad.lo.cc.u32 %0, %6, %9, %0;\n\t"
-        "madc.hi.cc.u32 %1, %6, %9, %1;\n\t"
-        "madc.lo.cc.u32 %2, %7, %9, %2;\n\t"
-        "madc.hi.cc.u32 %3, %7, %9, %3;\n\t"
-        "madc.lo.cc.u32 %4, %8, %9, %10;\n\t"
-        "madc.hi.u32 %5, %8, %9, 0;"
-        : "+r"(w[0]), "+r"(w[1]), "+r"(w[2]), "+r"(w[3]), "=&r"(w[4]), "=r"(w[5])
-        : "r"(x0), "r"(x1), "r"(x2), "r"(y), "r"(top));
 }
 
 __device__ __forceinline__ void row4_carry(u32* w, u32 x0, u32 x1, u32 x2, u32 x3, u32 y) {
@@ -425,54 +387,6 @@ __device__ __forceinline__ fe fe_mul_karatsuba(const fe& a, const fe& b) {
 
 // r = a·b mod p (as a value below 2^256)
 __device__ __forceinline__ fe fe_mul(const fe& a, const fe& b) { return fe_mul_schoolbook(a, b); }
-
-// r = a^2 mod p: the 28 cross products a_i·a_j (i < j) in even/odd accumulators, doubled with
-// funnel shifts, plus the 8 diagonal squares (even words) in one chain: 36 products before the
-// fold instead of 64.
-__device__ __forceinline__ fe fe_sq(const fe& a) {
-    u32 e[16], o[16], t[16];
-    const u32 a0 = a.v[0], a1 = a.v[1], a2 = a.v[2], a3 = a.v[3], a4 = a.v[4], a5 = a.v[5], a6 = a.v[6], a7 = a.v[7];
-    e[0] = e[1] = e[14] = e[15] = 0;
-    wide(e + 2, a2, a0); wide(e + 4, a4, a0); wide(e + 6, a6, a0);
-    wide(o, a1, a0); wide(o + 2, a3, a0); wide(o + 4, a5, a0); wide(o + 6, a7, a0);
-    row3_top(e + 4, a3, a5, a7, a1, 0u);
-    row3_carry(o + 2, a2, a4, a6, a1);
-    row2_carry(e + 6, a4, a6, a2);
-    row3_top(o + 4, a3, a5, a7, a2, o[8]);
-    row2_top(e + 8, a5, a7, a3, e[10]);
-    row2_carry(o + 6, a4, a6, a3);
-    row1_carry(e + 10, a6, a4);
-    row2_top(o + 8, a5, a7, a4, o[10]);
-    row1_top(e + 12, a7, a5, e[12]);
-    row1_carry(o + 10, a6, a5);
-    row1_top(o + 12, a7, a6, o[12]);
-    o[14] = 0;  // the cross sum is below 2^511
-    merge15(e, o, t);
-    // t = 2·t (the cross sum is below 2^511)
-#pragma unroll
-    for (int k = 15; k > 0; k--) t[k] = __funnelshift_l(t[k - 1], t[k], 1);
-    t[0] = 0;
-    asm("mad.lo.cc.u32 %0, %16, %16, %0;\n\t"
-        "madc.hi.cc.u32 %1, %16, %16, %1;\n\t"
-        "madc.lo.cc.u32 %2, %17, %17, %2;\n\t"
-        "madc.hi.cc.u32 %3, %17, %17, %3;\n\t"
-        "madc.lo.cc.u32 %4, %18, %18, %4;\n\t"
-        "madc.hi.cc.u32 %5, %18, %18, %5;\n\t"
-        "madc.lo.cc.u32 %6, %19, %19, %6;\n\t"
-        "madc.hi.cc.u32 %7, %19, %19, %7;\n\t"
-        "madc.lo.cc.u32 %8, %20, %20, %8;\n\t"
-        "madc.hi.cc.u32 %9, %20, %20, %9;\n\t"
-        "madc.lo.cc.u32 %10, %21, %21, %10;\n\t"
-        "madc.hi.cc.u32 %11, %21, %21, %11;\n\t"
-        "madc.lo.cc.u32 %12, %22, %22, %12;\n\t"
-        "madc.hi.cc.u32 %13, %22, %22, %13;\n\t"
-        "madc.lo.cc.u32 %14, %23, %23, %14;\n\t"
-        "madc.hi.u32 %15, %23, %23, %15;\n\t"
-        : "+r"(t[0]), "+r"(t[1]), "+r"(t[2]), "+r"(t[3]), "+r"(t[4]), "+r"(t[5]), "+r"(t[6]), "+r"(t[7]),
-          "+r"(t[8]), "+r"(t[9]), "+r"(t[10]), "+r"(t[11]), "+r"(t[12]), "+r"(t[13]), "+r"(t[14]), "+r"(t[15])
-        : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]), "r"(a.v[6]), "r"(a.v[7]));
-    return fe_reduce512(t);
-}
 
 // Canonical value (mod p) as 8 words
 __device__ __forceinline__ void fe_to_words(const fe& a, u32 out[8]) {

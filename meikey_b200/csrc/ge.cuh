@@ -7,6 +7,7 @@
 // sum is wanted (then y = (B+A)/(2Z-C) and x = (B-A)/(2Z+C)).
 #pragma once
 #include "fe32.cuh"
+#include "modinv.cuh"
 
 namespace mk32 {
 
@@ -86,26 +87,11 @@ __device__ __forceinline__ ge ge_identity() {
     return r;
 }
 
-// x^(p-2) by the standard addition chain for 2^255-21 (254 squarings, 11 multiplications)
-__device__ __forceinline__ fe fe_pow2k(fe a, int k) {
-#pragma unroll 1
-    for (int i = 0; i < k; i++) a = fe_sq(a);
-    return a;
-}
-
+// 1/z (0 for z = 0 mod p), not canonical
 __device__ __noinline__ fe fe_invert(const fe z) {
-    fe z2 = fe_sq(z);                               // 2
-    fe z9 = fe_mul(fe_sq(fe_sq(z2)), z);            // 9
-    fe z11 = fe_mul(z9, z2);                        // 11
-    fe z_5_0 = fe_mul(fe_sq(z11), z9);              // 2^5 - 1
-    fe z_10_0 = fe_mul(fe_pow2k(z_5_0, 5), z_5_0);  // 2^10 - 1
-    fe z_20_0 = fe_mul(fe_pow2k(z_10_0, 10), z_10_0);
-    fe z_40_0 = fe_mul(fe_pow2k(z_20_0, 20), z_20_0);
-    fe z_50_0 = fe_mul(fe_pow2k(z_40_0, 10), z_10_0);
-    fe z_100_0 = fe_mul(fe_pow2k(z_50_0, 50), z_50_0);
-    fe z_200_0 = fe_mul(fe_pow2k(z_100_0, 100), z_100_0);
-    fe z_250_0 = fe_mul(fe_pow2k(z_200_0, 50), z_50_0);
-    return fe_mul(fe_pow2k(z_250_0, 5), z11);       // 2^255 - 32 + 11 = p - 2
+    fe r;
+    mkinv::invert(z.v, r.v);
+    return r;
 }
 
 }  // namespace mk32

@@ -63,7 +63,7 @@ __device__ __forceinline__ u32 bits_at(const u64 m[4], u32 off, u32 w) {
 // comb table build
 // ---------------------------------------------------------------------------
 
-__global__ void __launch_bounds__(256) k_build_table(uint4* table, const CombGeom g, const u32* __restrict__ points,
+__global__ void __launch_bounds__(256, 2) k_build_table(uint4* table, const CombGeom g, const u32* __restrict__ points,
                                                      u64 first, u64 count) {
     u64 e = first + (u64)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= first + count || e >= g.entries) return;

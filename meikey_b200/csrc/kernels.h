@@ -88,9 +88,10 @@ cudaError_t measure_field_mul_forms(int sms, cudaStream_t st, double* schoolbook
 cudaError_t field_mul_pairs(const uint32_t* a, const uint32_t* b, uint32_t n, uint32_t* out_s, uint32_t* out_k,
                             cudaStream_t st);
 // Integer multiply-adds (32-bit halves) of one radix-2^32 field multiplication (products and the
-// fold by 38) and of a squaring.
+// fold by 38), and of an inversion by division steps (modinv.cuh; 18 batches on random values,
+// each 6 products a step and 72 wide products on the limbs).
 constexpr double MADS_MUL_SCHOOLBOOK = 64 + 64 + 16;
-constexpr double MADS_SQUARE = 72 + 16;
+constexpr double MADS_INVERT = 18 * (30 * 6 + 2 * 72);
 // The kernel of a variant and its dynamic shared memory (for graph nodes); sets the
 // kernel's shared-memory limit like launch_keys does.
 cudaError_t keys_kernel(bool derive, bool incr, uint32_t kpt, uint32_t block, uint32_t layout, uint32_t dfa_smem,
