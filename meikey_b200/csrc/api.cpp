@@ -991,10 +991,10 @@ int mk_ctx_work_per_key(const mk_ctx* c, int seed_source, double* field_muls, do
     // back-sweep y_j = a_j·inv and inv·den_j
     double batch = (4.0 * (kpt - 1) + 1.0) / kpt;
     if (seed_source == MK_SEED_INCREMENTAL) {
-        // no comb: key j > 0 of a thread's run is the y of Q + j·B (3 multiplications), and Q
-        // advances once per run by a full mixed addition (7); the thread's start point
-        // (at most 8 additions per launch) is left out
-        comb = (3.0 * (kpt - 1) + 7.0) / kpt;
+        // no comb: the keys of a thread's run are the y of Q ± d·B for d up to kpt/2 (3
+        // multiplications per d), and Q advances once per run by a full mixed addition (7); the
+        // thread's start point (at most 8 additions per launch) is left out
+        comb = (3.0 * kpt / 2 + 7.0) / kpt;
     }
     // pooled inversion by the CTA's inverting warp: `pools` lanes, each over `groups` thread
     // products, 3(groups-1) multiplications and one inversion by division steps
