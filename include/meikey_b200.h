@@ -71,7 +71,9 @@ enum mk_mode { MK_MODE_CONTAINS = 0, MK_MODE_SUFFIX = 1, MK_MODE_REGEX = 2 };
 typedef struct mk_options {
     uint32_t table_rows;      /* 10..63; default 12 (rows 10-20 are HBM tables of 26 GB down to 11 MB, 32-63 the
                                  comb windows of 8 down to 4 bits) */
-    uint32_t keys_per_thread; /* keys one thread derives before the pooled inversion (default 16) */
+    uint32_t keys_per_thread; /* keys per counted thread of one iteration's span (default 16), and the incremental
+                                 source's and mk_derive's batch per thread; searches of hashed seeds
+                                 invert in batches of 8 keys per thread, the fastest, whatever the span */
     uint32_t block;           /* threads per CTA (default 512): 256 or 512, keys per thread 4, 8 or 16;
                                  see inverter_rotates for who inverts */
     uint32_t blocks_per_sm;   /* resident CTAs per SM the grid is sized for (0 = occupancy maximum) */
@@ -80,14 +82,16 @@ typedef struct mk_options {
     uint32_t hash_warps;      /* 4: search with hashing warps (block 512, keys per thread 8 or 16): 11 comb
                                  warps, 1 inverter, 4 warps computing the SHA-512 scalars, so that hashing
                                  overlaps the comb multiplies; ChaCha20 and counter seeds only.  0: off */
-    uint32_t inverter_rotates;/* 0: a search CTA's last warp only inverts the CTA's products; 1: every warp
-                                 derives keys and the inversion rotates over four warps, one per SM
-                                 sub-partition (pays with long iterations: many needles).  Not with hash_warps */
+    uint32_t inverter_rotates;/* 0: the span of an iteration counts block - 32 threads of a CTA; 1: all of them.
+                                 Who inverts no longer depends on it: with hashed seeds every warp derives
+                                 keys and the inversion rotates over the warps, with the incremental source
+                                 the last warp only inverts.  Not with hash_warps */
     uint32_t inversion_batch; /* keys sharing one field inversion (the batch of Montgomery's trick, the
                                  reference's MEIKEY_BATCH x 4 pooled threads, kernel.cu:2024-2028):
-                                 keys_per_thread x compute threads / pools, for pools a divisor of the
-                                 compute threads (480; 512 with inverter_rotates; 352 with hash_warps) of
-                                 at most 32, e.g. 256 = 8 x 480 / 15.  0: 32 pools (keys_per_thread x 15,
+                                 keys_per_thread x counted threads / pools, for pools a divisor of the
+                                 counted threads (480; 512 with inverter_rotates; 352 with hash_warps) of
+                                 at most 32, e.g. 256 = 8 x 480 / 15; searches take the pool count that
+                                 comes nearest to it (256 = 8 x 512 / 16).  0: 32 pools (keys_per_thread x 15,
                                  x 16 with inverter_rotates, x 11 with hash_warps); else
                                  MK_ERR_OUT_OF_RANGE when no pool count gives it */
     uint32_t table_in_smem;   /* 1: every search CTA copies the comb table into shared memory and reads its

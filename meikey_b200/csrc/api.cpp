@@ -42,7 +42,7 @@ struct mk_ctx {
     uint32_t kpt = 8, block = 256, grid = 0;
     uint32_t hash_warps = 0;  // 4: search kernel with hashing warps (ChaCha20 / counter seeds)
     uint32_t layout = mkb::LAYOUT_INVERTER_WARP;  // division of work inside a search CTA
-    uint32_t inv_pools = 32;  // field inversions per search CTA and iteration
+    uint32_t inv_batch = 0;   // keys per field inversion asked for (0: 32 inversions per CTA and iteration)
     uint32_t table_smem = 0;  // bytes of the comb table each search CTA keeps in shared memory (0: HBM)
     uint32_t hit_capacity = 1u << 16;
     uint8_t* noalloc = nullptr;  // device address of mk_derive_noalloc's fixed staging array
@@ -303,7 +303,7 @@ int mk_ctx_create(int device, const mk_options* options, mk_ctx** out) try {
     c->block = o.block;
     c->hash_warps = o.hash_warps;
     c->layout = layout;
-    c->inv_pools = pools;
+    c->inv_batch = o.inversion_batch;
     if (o.hit_capacity) c->hit_capacity = o.hit_capacity;
     MK_CUDA(c, cudaSetDevice(device));
     MK_CUDA(c, mkb::noalloc_staging(&c->noalloc));
@@ -370,7 +370,8 @@ int mk_ctx_create(int device, const mk_options* options, mk_ctx** out) try {
             return fail(c, MK_ERR_OUT_OF_MEMORY, "incremental table allocation failed");
         }
         MK_CUDA(c, cudaMemcpy(c->incr, words.data(), words.size() * 4, cudaMemcpyHostToDevice));
-        mkh25519::niels_of_multiple((uint64_t)c->grid * mkb::search_threads(c->block, c->layout) * c->kpt, c->delta);
+        mkh25519::niels_of_multiple((uint64_t)c->grid * mkb::search_kernel_threads(true, c->block, c->layout, 0) * c->kpt,
+                                    c->delta);
     }
     // info
     mk_info& in = c->info;
@@ -384,7 +385,7 @@ int mk_ctx_create(int device, const mk_options* options, mk_ctx** out) try {
     // the threads of a search CTA that derive keys (all but a dedicated inverter warp, unless the
     // inversion rotates; 352 comb threads with hashing warps)
     in.keys_per_iter = (uint64_t)c->grid * mkb::search_threads(c->block, c->layout) * c->kpt;
-    in.inversion_batch = mkb::search_threads(c->block, c->layout) * c->kpt / c->inv_pools;
+    in.inversion_batch = mkb::search_threads(c->block, c->layout) * c->kpt / pools;
     in.table_in_smem = c->table_smem ? 1 : 0;
     snprintf(in.name, sizeof in.name, "%.95s", prop.name);
     if (o.self_check) {
@@ -754,6 +755,15 @@ static uint32_t dfa_smem_bytes(const mk_job* j) {
     return total <= mkb::DFA_SMEM_MAX ? (uint32_t)total : 0;
 }
 
+// Field inversions per CTA and iteration of the kernel that serves a context's searches of a
+// source: the pools whose batches come nearest to the keys per inversion asked for.
+static uint32_t search_pools(const mk_ctx* c, bool incr) {
+    if (!c->inv_batch) return 32;
+    const uint32_t keys = mkb::search_kernel_threads(incr, c->block, c->layout, c->table_smem) *
+                          mkb::search_kernel_keys(incr, c->kpt, c->layout, c->table_smem);
+    return std::min(32u, std::max(1u, (keys + c->inv_batch / 2) / c->inv_batch));
+}
+
 // Kernel parameters of one search launch of a job.
 static mkb::KeyLaunch search_params(const mk_job* j, uint64_t base, uint32_t iters) {
     const mk_ctx* c = j->ctx;
@@ -764,6 +774,8 @@ static mkb::KeyLaunch search_params(const mk_job* j, uint64_t base, uint32_t ite
         L.key[i] = (uint32_t)j->key[4 * i] | (uint32_t)j->key[4 * i + 1] << 8 | (uint32_t)j->key[4 * i + 2] << 16 | (uint32_t)j->key[4 * i + 3] << 24;
     L.seed_src = (uint32_t)j->source;
     L.iters = iters;
+    const bool incr = j->source == MK_SEED_INCREMENTAL;
+    L.chunks = c->info.keys_per_iter / mkb::search_kernel_keys(incr, c->kpt, c->layout, c->table_smem) * iters;
     L.base = base;
     L.match = j->d_match;
     L.hits = j->d_hits;
@@ -771,10 +783,10 @@ static mkb::KeyLaunch search_params(const mk_job* j, uint64_t base, uint32_t ite
     L.stop_on_hit = (uint32_t)j->stop_on_hit;
     L.job = j->d_job;
     L.sink = j->d_sink;
-    if (j->source == MK_SEED_INCREMENTAL) set_incremental(c, j->key, base, L);
+    if (incr) set_incremental(c, j->key, base, L);
     L.dfa_smem = dfa_smem_bytes(j);
     L.layout = c->layout;
-    L.inv_pools = c->inv_pools;
+    L.inv_pools = search_pools(c, incr);
     L.table_smem = c->table_smem;
     return L;
 }
@@ -983,8 +995,9 @@ int mk_ctx_work_per_key(const mk_ctx* c, int seed_source, double* field_muls, do
     // radix-2^32 costs: a schoolbook multiplication is 64 mad.lo + 64 mad.hi (8x8 limbs) + 16
     // (fold by 38).
     const double MUL = mkb::MADS_MUL_SCHOOLBOOK;
-    const double kpt = c->kpt, rows = c->geom.rows;
-    const double ct = mkb::search_threads(c->block, c->layout);
+    const bool incr = seed_source == MK_SEED_INCREMENTAL;
+    const double kpt = mkb::search_kernel_keys(incr, c->kpt, c->layout, c->table_smem), rows = c->geom.rows;
+    const double ct = mkb::search_kernel_threads(incr, c->block, c->layout, c->table_smem);
     // comb: row 0 is free, full additions cost 7 multiplications, the last one 3
     double comb = 7.0 * (rows - 2) + 3.0;
     // Montgomery batch inside a thread: a_j and the running product (2 each for j > 0),
@@ -998,7 +1011,7 @@ int mk_ctx_work_per_key(const mk_ctx* c, int seed_source, double* field_muls, do
     }
     // pooled inversion by the CTA's inverting warp: `pools` lanes, each over `groups` thread
     // products, 3(groups-1) multiplications and one inversion by division steps
-    const double pools = c->inv_pools, groups = ct / pools;
+    const double pools = search_pools(c, incr), groups = ct / pools;
     double pool_mul = pools * 3.0 * (groups - 1) / (ct * kpt);
     *field_muls = comb + batch + pool_mul;
     *int_mads = *field_muls * MUL + pools * mkb::MADS_INVERT / (ct * kpt);

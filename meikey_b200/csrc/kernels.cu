@@ -535,11 +535,11 @@ __device__ __forceinline__ int incr_key(int s) {
 }
 
 // Backward pass: `inv` is 1/(product of the batch's denominators); yields each key's
-// canonical y (sign bit 0), tests the needles and reports candidate hits.  INCR: slot j holds key
-// incr_key(j).
+// canonical y (sign bit 0), tests the needles and reports candidate hits (none when `valid` is
+// false: a run past the launch's last one).  INCR: slot j holds key incr_key(j).
 template <int KPT, bool INCR>
 __device__ __forceinline__ void backward(const KeyLaunch& L, const MatchSet& ms, const u32* lane_masks, u64 first,
-                                         const Batch<KPT>& b, fe inv, u32& sink) {
+                                         bool valid, const Batch<KPT>& b, fe inv, u32& sink) {
 #pragma unroll 1
     for (int j = KPT - 1; j >= 0; j--) {
         u32 pk[8];
@@ -548,6 +548,7 @@ __device__ __forceinline__ void backward(const KeyLaunch& L, const MatchSet& ms,
         sink ^= pk[7];
         u64 hw[2];
         match_key(ms, lane_masks, pk, hw);
+        if (!valid) hw[0] = hw[1] = 0;
         const bool any = (hw[0] | hw[1]) != 0;
         // warp ballot: the (rare) warps with a hit compact their records into the ring
         if (__ballot_sync(0xffffffffu, any)) report_hits(hw, first + (u64)(INCR ? incr_key<KPT>(j) : j), L.hits, L.hit_cap, L.job);
@@ -559,14 +560,15 @@ __device__ __forceinline__ void backward(const KeyLaunch& L, const MatchSet& ms,
 __device__ __forceinline__ void bar_sync(int id, int count) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory"); }
 __device__ __forceinline__ void bar_arrive(int id, int count) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory"); }
 
-// Inverts the `pools`·`groups` products prod[0 .. pools·groups) in place with one field
-// inversion per pool: lane l < pools of the calling warp handles the strided pool l, l+pools,
-// l+2·pools, ... (Montgomery's trick inside each pool); the other lanes idle.  With 32 pools
-// every lane works; fewer pools share each inversion among more keys (the inversion batch of a
-// pool is groups x the keys per thread).
-__device__ __forceinline__ void invert_pools(fe* prod, fe* scratch, int groups, int pools = 32) {
+// Inverts the n products prod[0 .. n) in place with one field inversion per pool: lane l < pools
+// of the calling warp handles the strided pool l, l+pools, l+2·pools, ... (Montgomery's trick
+// inside each pool); the other lanes idle.  With 32 pools every lane works; fewer pools share
+// each inversion among more keys (the inversion batch of a pool is its products x the keys per
+// thread).
+__device__ __forceinline__ void invert_pools(fe* prod, fe* scratch, int n, int pools = 32) {
     const int l = threadIdx.x & 31;
     if (l >= pools) return;
+    const int groups = (n - l + pools - 1) / pools;
     fe acc = prod[l];
     scratch[l] = acc;
 #pragma unroll 1
@@ -679,22 +681,29 @@ __device__ __forceinline__ void incr_fracs(const ge& Q, const uint4* steps, Batc
     b.prod = run;
 }
 
-// Search kernel.  The compute threads each handle KPT consecutive indices per iteration
-// (index = base + (it·nthreads + gid)·KPT + j, where gid and nthreads count the compute
-// threads).  Iterations are pipelined two deep: a compute thread runs the forward pass of
-// iteration it+1 before the backward pass of it, and the CTA's products of iteration it are
-// turned into their inverses in between.  Who inverts:
-//   ROT false: the CTA's last warp, which does nothing else (BLOCK-32 compute threads).  The
-//     inversion's long dependent chain runs beside the other warps' work.  That warp's SM
-//     sub-partition (warp w runs on sub-partition w % 4) then holds three compute warps
-//     against four elsewhere;
-//   ROT true: every thread computes keys, and the inversion of iteration it falls to warp
-//     BLOCK/32 - 4 + it % 4, one warp per sub-partition in turn.  The sub-partitions carry
-//     equal shares, but the inverting warp starts its next iteration only after the chain.
-//     That pays when iterations are long (many needles) and costs when they are short.
+// Search kernel.  The launch's keys are L.chunks runs of KPT consecutive indices.  Each compute
+// thread takes one run per iteration: warp w of CTA c takes runs ((it·warps + w)·CTAs + c)·32 + lane,
+// so a last iteration with fewer runs than threads leaves whole warps out, spread over the SMs
+// (they only take part in the barriers).  Iterations are pipelined two deep: a compute thread runs
+// the forward pass of iteration it before the backward pass of it-1, and the CTA's products of an
+// iteration are turned into their inverses in between.  Who inverts:
+//   ROT true (hashed seeds): every warp computes keys, and the inversion of iteration it falls to
+//     warp it mod the CTA's warps, so that consecutive inversions run on different SM
+//     sub-partitions and every warp carries the same share.  A dedicated inverter leaves its
+//     sub-partition with three compute warps against four (warp w runs on sub-partition w % 4):
+//     on B200, 8 keys per thread, 0.82 G keys/s against 0.89 with the rotating duty;
+//   ROT false (the incremental source, whose iterations are an order shorter): the CTA's last warp,
+//     which does nothing else (BLOCK-32 compute threads), so the inversion's dependent chain runs
+//     beside the other warps' work (11.0 against 8.8 G keys/s with the rotating duty).
 // The CTA's CT products of an iteration are inverted in L.inv_pools pools (default 32: lane l
 // of the inverting warp takes threads l, l+32, ...), one field inversion each, so one
-// inversion serves KPT·CT/pools keys.
+// inversion serves about KPT·CT/pools keys.
+// Hashed seeds run 8 keys per thread whatever the context's keys per thread (which sets the
+// launch's span): the two batches in flight of 16 keys, 155 MB over the chip, do not stay in the
+// L2 cache, and 4 keys share the barriers among too few (0.85 G keys/s at 16, 0.78 at 4, 0.895 at 8).
+// The one call of the forward pass stands inside the loop: a second one for the first iteration
+// makes the compiler keep it out of line, with the batch behind pointers (0.83 against 0.895 G
+// keys/s).
 // Named barriers, all BLOCK threads: products of buffer b ready (1 + b): the inverting warp
 // waits, the others arrive; inverses of buffer b ready (3 + b): the inverting warp arrives,
 // the others wait.  Stop requests (host stop word, or a hit with stop_on_hit) are read by
@@ -721,9 +730,11 @@ __global__ void __launch_bounds__(BLOCK, 512 / BLOCK) k_search(const KeyLaunch L
     __shared__ u32 lane_masks[64 * 32];  // see match_key
     __shared__ u32 key[8];
     __shared__ mkh::CounterMid mid;
-    __shared__ volatile u32 stop_iter;
+    __shared__ volatile u64 stop_iter;
     __shared__ uint4 steps[INCR ? INCR_STEPS * (ENTRY_WORDS / 4) : 1];
     const u32 tid = threadIdx.x;
+    const u64 nthreads = (u64)gridDim.x * CT;
+    const u64 iters = (L.chunks + nthreads - 1) / nthreads;
     if (INCR) load_steps(L, steps, tid, BLOCK);
     {
         const u32* src = (const u32*)&L.geom;
@@ -733,7 +744,7 @@ __global__ void __launch_bounds__(BLOCK, 512 / BLOCK) k_search(const KeyLaunch L
         u32* d2 = (u32*)&ms;
         for (u32 i = tid; i < sizeof(MatchSet) / 4; i += BLOCK) d2[i] = s2[i];
         if (tid < 8) key[tid] = L.key[tid];
-        if (tid == 0) stop_iter = L.iters;
+        if (tid == 0) stop_iter = iters;
     }
     __syncthreads();
     if (STAB)  // entries 128 bytes apart in HBM, 96 here
@@ -769,25 +780,23 @@ __global__ void __launch_bounds__(BLOCK, 512 / BLOCK) k_search(const KeyLaunch L
     if (INCR && tid < (u32)INCR_STEPS) step_to_yx(steps, tid);
     if (tid == 0 && L.seed_src == 1) mid = mkh::counter_mid(key);
     __syncthreads();
-    const u32 iters = L.iters;
     if (iters == 0) return;
-    // inversion pools of the CTA (a divisor of CT, at most 32; the host checks it)
-    const int pools = L.inv_pools ? (int)L.inv_pools : 32;
+    const int pools = (int)L.inv_pools;  // inversion pools of the CTA, 1..32
+    auto read_stop = [&](u64 it) {       // by the inverting warp
+        if ((tid & 31) == 0) {
+            const volatile JobDevice* jd = L.job;
+            if ((jd->stop != 0 || (L.stop_on_hit && jd->hit_count != 0)) && it + 2 < stop_iter) stop_iter = it + 2;
+        }
+        __syncwarp();
+    };
 
     if (!ROT && tid >= (u32)CT) {
         // ---- dedicated inverter warp ----
-        for (u32 it = 0;; it++) {
+        for (u64 it = 0;; it++) {
             const int b = it & 1;
             bar_sync(1 + b, BLOCK);
-            if ((tid & 31) == 0) {
-                const volatile JobDevice* jd = L.job;
-                if (jd->stop != 0 || (L.stop_on_hit && jd->hit_count != 0)) {
-                    u32 s = it + 2;
-                    if (s < stop_iter) stop_iter = s;
-                }
-            }
-            __syncwarp();
-            invert_pools(prod[b], scratch[b], CT / pools, pools);
+            read_stop(it);
+            invert_pools(prod[b], scratch[b], CT, pools);
             __syncwarp();
             bar_arrive(3 + b, BLOCK);
             if (it + 1 >= iters || it + 1 >= stop_iter) break;
@@ -798,58 +807,55 @@ __global__ void __launch_bounds__(BLOCK, 512 / BLOCK) k_search(const KeyLaunch L
 
     // ---- compute warps ----
     const u32 warp = tid >> 5;
-    auto inverts = [&](u32 it) { return ROT && warp == (u32)CW - 4u + (it & 3u); };
-    const u64 gid = (u64)blockIdx.x * CT + tid;
-    const u64 nthreads = (u64)gridDim.x * CT;
+    auto inverts = [&](u64 it) { return ROT && warp == (u32)it % (u32)CW; };
+    auto chunk_of = [&](u64 it) { return ((it * CW + warp) * gridDim.x + blockIdx.x) * 32u + (tid & 31u); };
+    auto first_of = [&](u64 it) { return L.base + chunk_of(it) * KPT; };
     EntrySlot& slot = slots[INCR || STAB ? 0 : tid];
     Batch<KPT> batch[2];
     u64 sc[KPT][4];
     u32 sink = 0;
     ge Q;
-    if (INCR) Q = incr_start(L, gid * KPT + KPT / 2);
-    auto first_of = [&](u32 it) { return L.base + ((u64)it * nthreads + gid) * KPT; };
-    auto produce = [&](u32 it) {
-        const int b = it & 1;
-        if (INCR) {
-            incr_fracs<KPT>(Q, steps, batch[b]);
-            Q = mk32::ge_add_niels(Q, words_niels(L.delta), false);
-        } else if (SHAI) {
-            if (it == 0) scalars<KPT>(L, key, mid, first_of(0), sc);
-            combs_sha<KPT>(L, g, sc, slot, batch[b], key, mid, first_of(it + 1));
-        } else {
-            scalars<KPT>(L, key, mid, first_of(it), sc);
-            combs<KPT, STAB>(L, g, sc, slot, stab, batch[b]);
-        }
-        prod[b][tid] = batch[b].prod;
-        if (inverts(it)) {
-            bar_sync(1 + b, BLOCK);
-            if ((tid & 31) == 0) {
-                const volatile JobDevice* jd = L.job;
-                if (jd->stop != 0 || (L.stop_on_hit && jd->hit_count != 0)) {
-                    u32 s = it + 2;
-                    if (s < stop_iter) stop_iter = s;
-                }
+    if (INCR) Q = incr_start(L, chunk_of(0) * KPT + KPT / 2);
+    for (u64 it = 0;; it++) {
+        if (it == 0 || (it < iters && it < stop_iter)) {
+            // forward pass of iteration it
+            const int b = it & 1;
+            if (chunk_of(it) - (tid & 31u) >= L.chunks) {
+                batch[b].prod = mk32::fe_small(1);  // a warp past the last run
+            } else if (INCR) {
+                incr_fracs<KPT>(Q, steps, batch[b]);
+                Q = mk32::ge_add_niels(Q, words_niels(L.delta), false);
+            } else if (SHAI) {
+                if (it == 0) scalars<KPT>(L, key, mid, first_of(0), sc);
+                combs_sha<KPT>(L, g, sc, slot, batch[b], key, mid, first_of(it + 1));
+            } else {
+                scalars<KPT>(L, key, mid, first_of(it), sc);
+                combs<KPT, STAB>(L, g, sc, slot, stab, batch[b]);
             }
-            __syncwarp();
-            invert_pools(prod[b], scratch[b], CT / pools, pools);
-            __syncwarp();
-            bar_arrive(3 + b, BLOCK);
-        } else {
-            bar_arrive(1 + b, BLOCK);
+            prod[b][tid] = batch[b].prod;
+            if (inverts(it)) {
+                bar_sync(1 + b, BLOCK);
+                read_stop(it);
+                invert_pools(prod[b], scratch[b], CT, pools);
+                __syncwarp();
+                bar_arrive(3 + b, BLOCK);
+            } else {
+                bar_arrive(1 + b, BLOCK);
+            }
         }
-    };
-    produce(0);
-    for (u32 it = 0;; it++) {
-        const int b = it & 1;
-        if (it + 1 < iters && it + 1 < stop_iter) produce(it + 1);
-        if (!inverts(it)) bar_sync(3 + b, BLOCK);
-        backward<KPT, INCR>(L, ms, ms.narrow ? lane_masks : nullptr, first_of(it), batch[b],
-                                                 prod[b][tid], sink);
-        if (it + 1 >= iters || it + 1 >= stop_iter) break;
+        if (it == 0) continue;
+        // backward pass of iteration it - 1
+        const u64 p = it - 1;
+        const int b = p & 1;
+        if (!inverts(p)) bar_sync(3 + b, BLOCK);
+        if (chunk_of(p) - (tid & 31u) < L.chunks)
+            backward<KPT, INCR>(L, ms, ms.narrow ? lane_masks : nullptr, first_of(p), chunk_of(p) < L.chunks, batch[b],
+                                prod[b][tid], sink);
+        if (it >= iters || it >= stop_iter) break;
     }
-    // warp 0 never inverts, so with ROT the last stop decision is visible here
+    // the decision of the iteration that ended the loop is visible here (its inverses were waited for)
     if (ROT && tid == 0 && stop_iter < iters) atomicOr(&L.job->status, 1u);
-    if (L.sink) L.sink[gid] = sink;
+    if (L.sink) L.sink[(u64)blockIdx.x * CT + tid] = sink;
 }
 
 // Search kernel with hashing warps (ChaCha20 / counter seeds).  Warps 0..10 run the comb
@@ -909,7 +915,7 @@ __global__ void __launch_bounds__(BLOCK, 1) k_search_hw(const KeyLaunch L) {
     if (iters == 0) return;
     const u64 nthreads = (u64)gridDim.x * CT;
     auto first_of = [&](u32 it, u64 gid) { return L.base + ((u64)it * nthreads + gid) * KPT; };
-    const int pools = L.inv_pools ? (int)L.inv_pools : 32;  // a divisor of CT, at most 32
+    const int pools = (int)L.inv_pools;  // 1..32
 
     if (warp > (u32)INV_WARP) {
         // ---- hashing warps ----
@@ -966,7 +972,7 @@ __global__ void __launch_bounds__(BLOCK, 1) k_search_hw(const KeyLaunch L) {
             const bool more = it + 1 < iters && it + 1 < stop_iter;
             // the hashing warps wait on this decision only when they will consider iteration it+2
             if (it + 2 < iters && more) bar_arrive(9 + (it & 1), B_STOP);
-            invert_pools(prod[b], scratch[b], CT / pools, pools);
+            invert_pools(prod[b], scratch[b], CT, pools);
             __syncwarp();
             bar_arrive(3 + b, B_PIPE);
             if (!more) break;
@@ -1017,7 +1023,7 @@ __global__ void __launch_bounds__(BLOCK, 1) k_search_hw(const KeyLaunch L) {
         const int b = it & 1;
         if (it + 1 < iters && it + 1 < stop_iter) produce(it + 1);
         bar_sync(3 + b, B_PIPE);
-        backward<KPT, false>(L, ms, ms.narrow ? lane_masks : nullptr, first_of(it, gid), batch[b],
+        backward<KPT, false>(L, ms, ms.narrow ? lane_masks : nullptr, first_of(it, gid), true, batch[b],
                                         prod[b][tid], sink);
         if (it + 1 >= iters || it + 1 >= stop_iter) break;
     }
@@ -1081,7 +1087,7 @@ __global__ void __launch_bounds__(BLOCK, 512 / BLOCK) k_derive(const KeyLaunch L
     }
     prod[tid] = pre[NUM - 1];
     __syncthreads();
-    if (tid < 32) invert_pools(prod, scratch, BLOCK / 32);
+    if (tid < 32) invert_pools(prod, scratch, BLOCK);
     __syncthreads();
     fe inv = prod[tid];
 #pragma unroll 1
@@ -1119,8 +1125,7 @@ static size_t dyn_bytes(bool derive, bool incr, uint32_t block, uint32_t layout,
         const size_t ct = 352;
         return 4 * ct * fe_bytes + ct * sizeof(EntrySlot) + 2 * 4 * ct * 32;
     }
-    const size_t threads = derive ? block : search_threads(block, layout == LAYOUT_HASH_WARPS ? LAYOUT_INVERTER_WARP : layout);
-    // (the interleaved layout has the dedicated inverter's buffers)
+    const size_t threads = derive ? block : search_kernel_threads(incr, block, layout, table_smem);
     if (table_smem && !derive && !incr) return 4 * threads * fe_bytes + table_smem;  // the table in place of the slots
     return (derive ? 2 : 4) * threads * fe_bytes + (incr ? 0 : threads * sizeof(EntrySlot));
 }
@@ -1141,12 +1146,15 @@ static const void* stab_kernel_of(uint32_t kpt, uint32_t block) {
     return nullptr;
 }
 
-static const void* kernel_of(bool derive, bool incr, uint32_t kpt, uint32_t block, bool rot) {
-#define MK_FN(K, B)                                                                                            \
-    if (kpt == K && block == B) {                                                                              \
-        if (derive) return incr ? (const void*)k_derive<K, B, true> : (const void*)k_derive<K, B, false>;      \
-        if (rot) return incr ? (const void*)k_search<K, B, true, true> : (const void*)k_search<K, B, false, true>; \
-        return incr ? (const void*)k_search<K, B, true, false> : (const void*)k_search<K, B, false, false>;    \
+static const void* kernel_of(bool derive, bool incr, uint32_t kpt, uint32_t block) {
+    if (!derive && !incr)
+        return block == 512 ? (const void*)k_search<HASHED_KEYS, 512, false, true>
+               : block == 256 ? (const void*)k_search<HASHED_KEYS, 256, false, true>
+                              : nullptr;
+#define MK_FN(K, B)                                                                                       \
+    if (kpt == K && block == B) {                                                                         \
+        if (derive) return incr ? (const void*)k_derive<K, B, true> : (const void*)k_derive<K, B, false>; \
+        return (const void*)k_search<K, B, true, false>;                                                  \
     }
     MK_VARIANTS(MK_FN)
 #undef MK_FN
@@ -1172,7 +1180,7 @@ static const void* variant_kernel(bool derive, bool incr, uint32_t kpt, uint32_t
     if (layout == LAYOUT_INTERLEAVED && !derive && !incr) return table_smem ? nullptr : shai_kernel_of(kpt, block);
     const bool hw = layout == LAYOUT_HASH_WARPS && !derive && !incr;
     if (table_smem && !derive && !incr) return layout == LAYOUT_INVERTER_WARP ? stab_kernel_of(kpt, block) : nullptr;
-    return hw ? hw_kernel_of(kpt, block) : kernel_of(derive, incr, kpt, block, layout == LAYOUT_ROTATING);
+    return hw ? hw_kernel_of(kpt, block) : kernel_of(derive, incr, kpt, block);
 }
 
 cudaError_t launch_keys(const KeyLaunch& L, bool derive, uint32_t kpt, uint32_t block, uint32_t grid, cudaStream_t st) {

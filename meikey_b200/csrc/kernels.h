@@ -19,6 +19,7 @@ struct KeyLaunch {
     uint32_t key[8];
     uint32_t seed_src;     // 0 ChaCha20, 1 counter, 2 incremental
     uint32_t iters;
+    uint64_t chunks;       // search: runs of search_kernel_keys consecutive indices from base
     uint64_t base;
     // search
     const MatchSet* match; // device copy
@@ -33,31 +34,46 @@ struct KeyLaunch {
     // incremental source: index base + i stands for the point (s0 + base + i)·B
     const uint4* incr;     // INCR_WINDOWS·16 entries j·16^w·B, then INCR_STEPS entries j·B (table form)
     uint32_t start[32];    // (s0 + base)·B as x, y, 1, xy
-    uint32_t delta[24];    // keys_per_iter·B: one search thread's jump between iterations
+    uint32_t delta[24];    // CTAs·search_kernel_threads·keys·B: a search thread's jump between iterations
     // bytes of shared memory for the job's DFA tables (each 16-byte aligned; 0: read them
     // from global memory)
     uint32_t dfa_smem;
     // division of work inside a search CTA (LAYOUT_*)
     uint32_t layout;
-    // field inversions per CTA and iteration (0: 32, one per lane of the inverting warp): each
-    // pools the products of compute threads / inv_pools threads; a divisor of the compute
-    // threads, at most 32
+    // field inversions per CTA and iteration of a search, 1..32 (one per lane of the inverting
+    // warp): each pools the products of every inv_pools-th compute thread
     uint32_t inv_pools;
     // bytes of the comb table in shared memory (search kernels; 0: gathered from HBM): every CTA
     // copies the table there at the start, entries 96 bytes apart
     uint32_t table_smem;
 };
 
-// LAYOUT_INVERTER_WARP: the last warp inverts, the others compute keys; LAYOUT_ROTATING: every
-// warp computes keys and the inversion rotates over four warps; LAYOUT_INTERLEAVED: as
-// LAYOUT_INVERTER_WARP, with each iteration's SHA-512 of the next iteration's seeds inside the
+// LAYOUT_INVERTER_WARP, LAYOUT_ROTATING: the span of an iteration counts a CTA's threads without
+// or with the last warp; both run the same kernels (hashed seeds: every warp computes keys and the
+// inversion rotates over them; incremental source: the last warp inverts).  LAYOUT_INTERLEAVED: the
+// last warp inverts, and each iteration's SHA-512 of the next iteration's seeds runs inside the
 // comb rows (12 rows); LAYOUT_HASH_WARPS: 11 comb warps, 1 inverter, 4 hashing warps
 // (k_search_hw; ChaCha20 / counter seeds)
 constexpr uint32_t LAYOUT_INVERTER_WARP = 0, LAYOUT_ROTATING = 1, LAYOUT_INTERLEAVED = 2, LAYOUT_HASH_WARPS = 4;
 
-// compute threads of a search CTA
+// threads of a search CTA that the span of one iteration counts
 inline uint32_t search_threads(uint32_t block, uint32_t layout) {
     return layout == LAYOUT_HASH_WARPS ? 352u : layout == LAYOUT_ROTATING ? block : block - 32u;
+}
+
+// keys per thread and iteration of the hashed-seed search kernel
+constexpr uint32_t HASHED_KEYS = 8;
+
+inline bool search_rotates(bool incr, uint32_t layout, uint32_t table_smem) {
+    return !incr && !table_smem && (layout == LAYOUT_INVERTER_WARP || layout == LAYOUT_ROTATING);
+}
+// keys per thread and iteration, and compute threads per CTA, of the kernel that serves a search
+inline uint32_t search_kernel_keys(bool incr, uint32_t kpt, uint32_t layout, uint32_t table_smem) {
+    return search_rotates(incr, layout, table_smem) ? HASHED_KEYS : kpt;
+}
+inline uint32_t search_kernel_threads(bool incr, uint32_t block, uint32_t layout, uint32_t table_smem) {
+    if (layout == LAYOUT_HASH_WARPS && !incr) return 352u;
+    return search_rotates(incr, layout, table_smem) ? block : block - 32u;
 }
 
 constexpr uint32_t DFA_SMEM_MAX = 48u * 1024u;

@@ -444,8 +444,8 @@ def tune_space(rows=(11, 12, 13, 14, 16), variants=BUILT_VARIANTS, blocks_per_sm
                inverter_rotates=(0,), inversion_batch=(0,), table_in_smem=(0,)):
     """Candidate options: comb rows (table size against multiplications per key) x keys per
     thread and block x CTAs per SM x the hashing-warp layout (built for block 512, keys per
-    thread 8 and 16) x who inverts (a dedicated warp, or a duty rotating over four key warps;
-    not with hashing warps) x the inversion batch (keys per field inversion; 0 = 32 pools,
+    thread 8 and 16) x the counted threads (block - 32, or all with inverter_rotates; not with
+    hashing warps) x the inversion batch (keys per field inversion; 0 = 32 pools,
     "all" = every batch of 64..512 the layout can run)."""
     out = []
     for r in rows:
