@@ -1,5 +1,7 @@
 // GF(2^255 - 19) in eight 32-bit limbs (radix 2^32), values kept below 2^256
-// (congruent mod p, not canonical).  Products use hand-written mad.lo.cc /
+// (congruent mod p, not canonical).  "Tight" values are below 2^255 + 1500: canonical ones and
+// every product.  Sums and differences of tight values need half the carries (fe_add_t, fe_add_1,
+// fe_sub_t) and may reach 2^256; products take either.  Products use hand-written mad.lo.cc /
 // madc.hi.cc carry chains; 2^256 is folded back as 38.  Exact integer math, no FP.
 #pragma once
 #include <stdint.h>
@@ -97,6 +99,107 @@ __device__ __forceinline__ fe fe_sub(const fe& a, const fe& b) {
     return r;
 }
 
+// a + b, both tight: a carry out leaves less than 3000, so adding 38 stays in word 0
+__device__ __forceinline__ fe fe_add_t(const fe& a, const fe& b) {
+    fe r;
+    u32 c;
+    asm("add.cc.u32 %0, %9, %17;\n\t"
+        "addc.cc.u32 %1, %10, %18;\n\t"
+        "addc.cc.u32 %2, %11, %19;\n\t"
+        "addc.cc.u32 %3, %12, %20;\n\t"
+        "addc.cc.u32 %4, %13, %21;\n\t"
+        "addc.cc.u32 %5, %14, %22;\n\t"
+        "addc.cc.u32 %6, %15, %23;\n\t"
+        "addc.cc.u32 %7, %16, %24;\n\t"
+        "addc.u32 %8, 0, 0;"
+        : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]), "=r"(r.v[6]),
+          "=r"(r.v[7]), "=r"(c)
+        : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]), "r"(a.v[6]), "r"(a.v[7]),
+          "r"(b.v[0]), "r"(b.v[1]), "r"(b.v[2]), "r"(b.v[3]), "r"(b.v[4]), "r"(b.v[5]), "r"(b.v[6]), "r"(b.v[7]));
+    r.v[0] += 38u * c;
+    return r;
+}
+
+// a + b, b tight: a carry out leaves less than 2^255 + 1500, so adding 38 carries no further
+__device__ __forceinline__ fe fe_add_1(const fe& a, const fe& b) {
+    fe r;
+    u32 c;
+    asm("add.cc.u32 %0, %9, %17;\n\t"
+        "addc.cc.u32 %1, %10, %18;\n\t"
+        "addc.cc.u32 %2, %11, %19;\n\t"
+        "addc.cc.u32 %3, %12, %20;\n\t"
+        "addc.cc.u32 %4, %13, %21;\n\t"
+        "addc.cc.u32 %5, %14, %22;\n\t"
+        "addc.cc.u32 %6, %15, %23;\n\t"
+        "addc.cc.u32 %7, %16, %24;\n\t"
+        "addc.u32 %8, 0, 0;"
+        : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]), "=r"(r.v[6]),
+          "=r"(r.v[7]), "=r"(c)
+        : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]), "r"(a.v[6]), "r"(a.v[7]),
+          "r"(b.v[0]), "r"(b.v[1]), "r"(b.v[2]), "r"(b.v[3]), "r"(b.v[4]), "r"(b.v[5]), "r"(b.v[6]), "r"(b.v[7]));
+    const u32 add = 38u * c;
+    asm("add.cc.u32 %0, %0, %8;\n\t"
+        "addc.cc.u32 %1, %1, 0;\n\t"
+        "addc.cc.u32 %2, %2, 0;\n\t"
+        "addc.cc.u32 %3, %3, 0;\n\t"
+        "addc.cc.u32 %4, %4, 0;\n\t"
+        "addc.cc.u32 %5, %5, 0;\n\t"
+        "addc.cc.u32 %6, %6, 0;\n\t"
+        "addc.u32 %7, %7, 0;"
+        : "+r"(r.v[0]), "+r"(r.v[1]), "+r"(r.v[2]), "+r"(r.v[3]), "+r"(r.v[4]), "+r"(r.v[5]), "+r"(r.v[6]), "+r"(r.v[7])
+        : "r"(add));
+    return r;
+}
+
+// a - b, b tight: a borrow leaves at least 2^255 - 1500, so taking 38 off borrows no further
+__device__ __forceinline__ fe fe_sub_t(const fe& a, const fe& b) {
+    fe r;
+    u32 bw;
+    asm("sub.cc.u32 %0, %9, %17;\n\t"
+        "subc.cc.u32 %1, %10, %18;\n\t"
+        "subc.cc.u32 %2, %11, %19;\n\t"
+        "subc.cc.u32 %3, %12, %20;\n\t"
+        "subc.cc.u32 %4, %13, %21;\n\t"
+        "subc.cc.u32 %5, %14, %22;\n\t"
+        "subc.cc.u32 %6, %15, %23;\n\t"
+        "subc.cc.u32 %7, %16, %24;\n\t"
+        "subc.u32 %8, 0, 0;"
+        : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]), "=r"(r.v[6]),
+          "=r"(r.v[7]), "=r"(bw)
+        : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]), "r"(a.v[6]), "r"(a.v[7]),
+          "r"(b.v[0]), "r"(b.v[1]), "r"(b.v[2]), "r"(b.v[3]), "r"(b.v[4]), "r"(b.v[5]), "r"(b.v[6]), "r"(b.v[7]));
+    const u32 sub = 38u & bw;
+    asm("sub.cc.u32 %0, %0, %8;\n\t"
+        "subc.cc.u32 %1, %1, 0;\n\t"
+        "subc.cc.u32 %2, %2, 0;\n\t"
+        "subc.cc.u32 %3, %3, 0;\n\t"
+        "subc.cc.u32 %4, %4, 0;\n\t"
+        "subc.cc.u32 %5, %5, 0;\n\t"
+        "subc.cc.u32 %6, %6, 0;\n\t"
+        "subc.u32 %7, %7, 0;"
+        : "+r"(r.v[0]), "+r"(r.v[1]), "+r"(r.v[2]), "+r"(r.v[3]), "+r"(r.v[4]), "+r"(r.v[5]), "+r"(r.v[6]), "+r"(r.v[7])
+        : "r"(sub));
+    return r;
+}
+
+// a as a tight value: bit 255 comes back as 19
+__device__ __forceinline__ fe fe_tight(const fe& a) {
+    fe r = a;
+    const u32 add = 19u * (a.v[7] >> 31);
+    r.v[7] &= 0x7fffffffu;
+    asm("add.cc.u32 %0, %0, %8;\n\t"
+        "addc.cc.u32 %1, %1, 0;\n\t"
+        "addc.cc.u32 %2, %2, 0;\n\t"
+        "addc.cc.u32 %3, %3, 0;\n\t"
+        "addc.cc.u32 %4, %4, 0;\n\t"
+        "addc.cc.u32 %5, %5, 0;\n\t"
+        "addc.cc.u32 %6, %6, 0;\n\t"
+        "addc.u32 %7, %7, 0;"
+        : "+r"(r.v[0]), "+r"(r.v[1]), "+r"(r.v[2]), "+r"(r.v[3]), "+r"(r.v[4]), "+r"(r.v[5]), "+r"(r.v[6]), "+r"(r.v[7])
+        : "r"(add));
+    return r;
+}
+
 // ---- products in even/odd accumulators ----
 //
 // A product of two limbs a_i·b_j is added at words i+j, i+j+1.  The integer pipe adds a full
@@ -122,8 +225,9 @@ __device__ __forceinline__ void wide(u32* w, u32 x, u32 y) {
 
 // One chain of n products by the same limb y on consecutive pairs, w[2i..2i+1] += x_i·y:
 //   rown_carry  every pair holds a sum already; the carry starts the next pair, w[2n] = carry;
-//   rown_top    the last pair is new but for a carry `top` (0 or 1) of an earlier row; it cannot
-//               overflow (x·y + 2 < 2^64).
+//   rown_add    the same, the carry added to the next pair, which holds a sum;
+//   rown_open   the last pair is new, and rown_top new but for a carry `top` (0 or 1) of an earlier
+//               row; neither overflows (x·y + 2 < 2^64).
 __device__ __forceinline__ void row2_carry(u32* w, u32 x0, u32 x1, u32 y) {
     asm("mad.lo.cc.u32 %0, %5, %7, %0;\n\t"
         "madc.hi.cc.u32 %1, %5, %7, %1;\n\t"
@@ -158,17 +262,33 @@ __device__ __forceinline__ void row4_carry(u32* w, u32 x0, u32 x1, u32 x2, u32 x
         : "r"(x0), "r"(x1), "r"(x2), "r"(x3), "r"(y));
 }
 
-__device__ __forceinline__ void row4_top(u32* w, u32 x0, u32 x1, u32 x2, u32 x3, u32 y, u32 top) {
+__device__ __forceinline__ void row4_open(u32* w, u32 x0, u32 x1, u32 x2, u32 x3, u32 y) {
     asm("mad.lo.cc.u32 %0, %8, %12, %0;\n\t"
         "madc.hi.cc.u32 %1, %8, %12, %1;\n\t"
         "madc.lo.cc.u32 %2, %9, %12, %2;\n\t"
         "madc.hi.cc.u32 %3, %9, %12, %3;\n\t"
         "madc.lo.cc.u32 %4, %10, %12, %4;\n\t"
         "madc.hi.cc.u32 %5, %10, %12, %5;\n\t"
-        "madc.lo.cc.u32 %6, %11, %12, %13;\n\t"
+        "madc.lo.cc.u32 %6, %11, %12, 0;\n\t"
         "madc.hi.u32 %7, %11, %12, 0;"
         : "+r"(w[0]), "+r"(w[1]), "+r"(w[2]), "+r"(w[3]), "+r"(w[4]), "+r"(w[5]), "=&r"(w[6]), "=r"(w[7])
-        : "r"(x0), "r"(x1), "r"(x2), "r"(x3), "r"(y), "r"(top));
+        : "r"(x0), "r"(x1), "r"(x2), "r"(x3), "r"(y));
+}
+
+__device__ __forceinline__ void row4_add(u32* w, u32 x0, u32 x1, u32 x2, u32 x3, u32 y) {
+    asm("mad.lo.cc.u32 %0, %10, %14, %0;\n\t"
+        "madc.hi.cc.u32 %1, %10, %14, %1;\n\t"
+        "madc.lo.cc.u32 %2, %11, %14, %2;\n\t"
+        "madc.hi.cc.u32 %3, %11, %14, %3;\n\t"
+        "madc.lo.cc.u32 %4, %12, %14, %4;\n\t"
+        "madc.hi.cc.u32 %5, %12, %14, %5;\n\t"
+        "madc.lo.cc.u32 %6, %13, %14, %6;\n\t"
+        "madc.hi.cc.u32 %7, %13, %14, %7;\n\t"
+        "addc.cc.u32 %8, %8, 0;\n\t"
+        "addc.u32 %9, %9, 0;"
+        : "+r"(w[0]), "+r"(w[1]), "+r"(w[2]), "+r"(w[3]), "+r"(w[4]), "+r"(w[5]), "+r"(w[6]), "+r"(w[7]),
+          "+r"(w[8]), "+r"(w[9])
+        : "r"(x0), "r"(x1), "r"(x2), "r"(x3), "r"(y));
 }
 
 // t = e + o·2^32 over n+1 words (t[0] = e[0]); the sum fits
@@ -211,7 +331,7 @@ __device__ __forceinline__ void merge15(const u32* e, const u32* o, u32* t) {
           "r"(o[8]), "r"(o[9]), "r"(o[10]), "r"(o[11]), "r"(o[12]), "r"(o[13]), "r"(o[14]));
 }
 
-// Fold a 512-bit product t[0..15] to 8 words: t_lo + 38·t_hi, then the top word again.  The
+// Fold a 512-bit product t[0..15] to 8 words (tight): t_lo + 38·t_hi, then the bits from 255 up.  The
 // products 38·t[8+j] of even j extend the pairs of t_lo, those of odd j go one word up.
 __device__ __forceinline__ fe fe_reduce512(const u32 t[16]) {
     u32 s[8], w[9];
@@ -234,41 +354,40 @@ __device__ __forceinline__ fe fe_reduce512(const u32 t[16]) {
         "addc.u32 %7, %7, %15;"
         : "+r"(r.v[1]), "+r"(r.v[2]), "+r"(r.v[3]), "+r"(r.v[4]), "+r"(r.v[5]), "+r"(r.v[6]), "+r"(r.v[7]), "+r"(top)
         : "r"(s[0]), "r"(s[1]), "r"(s[2]), "r"(s[3]), "r"(s[4]), "r"(s[5]), "r"(s[6]), "r"(s[7]));
-    // top < 40: fold 38·top; one more carry is possible and is folded as 38 without further carry
-    u32 add = 38u * top, c2;
-    asm("add.cc.u32 %0, %0, %9;\n\t"
+    // top < 40: what stands above bit 255, below 78, comes back as 19 each and carries no further
+    const u32 add = 19u * __funnelshift_l(r.v[7], top, 1);
+    r.v[7] &= 0x7fffffffu;
+    asm("add.cc.u32 %0, %0, %8;\n\t"
         "addc.cc.u32 %1, %1, 0;\n\t"
         "addc.cc.u32 %2, %2, 0;\n\t"
         "addc.cc.u32 %3, %3, 0;\n\t"
         "addc.cc.u32 %4, %4, 0;\n\t"
         "addc.cc.u32 %5, %5, 0;\n\t"
         "addc.cc.u32 %6, %6, 0;\n\t"
-        "addc.cc.u32 %7, %7, 0;\n\t"
-        "addc.u32 %8, 0, 0;\n\t"
-        : "+r"(r.v[0]), "+r"(r.v[1]), "+r"(r.v[2]), "+r"(r.v[3]), "+r"(r.v[4]), "+r"(r.v[5]), "+r"(r.v[6]),
-          "+r"(r.v[7]), "=r"(c2)
+        "addc.u32 %7, %7, 0;"
+        : "+r"(r.v[0]), "+r"(r.v[1]), "+r"(r.v[2]), "+r"(r.v[3]), "+r"(r.v[4]), "+r"(r.v[5]), "+r"(r.v[6]), "+r"(r.v[7])
         : "r"(add));
-    r.v[0] += 38u * c2;
     return r;
 }
 
-// r = a·b mod p (as a value below 2^256), schoolbook: 64 products.  Limb b_i meets the limbs
-// a_j of its own parity on the even words and the others on the odd ones; each row's chain either
-// opens a new top pair or leaves its carry there for the next row.
+// r = a·b mod p (tight), schoolbook: 64 products.  Limb b_i meets the limbs a_j of its own parity
+// on the even words and the others on the odd ones.  Of two rows whose chains end on one pair, the
+// one that opens it goes first and the other's carry is added to it: a pair opened on top of a
+// waiting carry would need that carry moved into a pair with a zero.
 __device__ __forceinline__ fe fe_mul_schoolbook(const fe& a, const fe& b) {
     u32 e[16], o[16], t[16];
     const u32 a0 = a.v[0], a1 = a.v[1], a2 = a.v[2], a3 = a.v[3], a4 = a.v[4], a5 = a.v[5], a6 = a.v[6], a7 = a.v[7];
     wide(e, a0, b.v[0]); wide(e + 2, a2, b.v[0]); wide(e + 4, a4, b.v[0]); wide(e + 6, a6, b.v[0]);
     wide(o, a1, b.v[0]); wide(o + 2, a3, b.v[0]); wide(o + 4, a5, b.v[0]); wide(o + 6, a7, b.v[0]);
-    row4_top(e + 2, a1, a3, a5, a7, b.v[1], 0u);
-    row4_carry(o, a0, a2, a4, a6, b.v[1]);
+    row4_open(e + 2, a1, a3, a5, a7, b.v[1]);
 #pragma unroll
     for (int i = 2; i < 8; i += 2) {
-        row4_carry(e + i, a0, a2, a4, a6, b.v[i]);
-        row4_top(o + i, a1, a3, a5, a7, b.v[i], o[i + 6]);
-        row4_top(e + i + 2, a1, a3, a5, a7, b.v[i + 1], e[i + 8]);
-        row4_carry(o + i, a0, a2, a4, a6, b.v[i + 1]);
+        row4_open(e + i + 2, a1, a3, a5, a7, b.v[i + 1]);
+        row4_add(e + i, a0, a2, a4, a6, b.v[i]);
+        row4_open(o + i, a1, a3, a5, a7, b.v[i]);
+        row4_add(o + i - 2, a0, a2, a4, a6, b.v[i - 1]);
     }
+    row4_carry(o + 6, a0, a2, a4, a6, b.v[7]);
     merge15(e, o, t);
     return fe_reduce512(t);
 }
@@ -385,7 +504,7 @@ __device__ __forceinline__ fe fe_mul_karatsuba(const fe& a, const fe& b) {
     return fe_reduce512(t);
 }
 
-// r = a·b mod p (as a value below 2^256)
+// r = a·b mod p (tight) for any values below 2^256
 __device__ __forceinline__ fe fe_mul(const fe& a, const fe& b) { return fe_mul_schoolbook(a, b); }
 
 // Canonical value (mod p) as 8 words

@@ -19,26 +19,27 @@ struct niels {
     fe ypx, ymx, t2d;
 };
 
-__device__ __forceinline__ void fe_cswap(fe& a, fe& b, bool swap) {
+// -q when neg: swaps y+x and y-x and negates 2dxy
+__device__ __forceinline__ niels niels_signed(const niels& q, bool neg) {
+    const fe nt = fe_sub_t(fe_zero(), q.t2d);
+    niels r;
 #pragma unroll
     for (int i = 0; i < 8; i++) {
-        u32 x = a.v[i], y = b.v[i];
-        a.v[i] = swap ? y : x;
-        b.v[i] = swap ? x : y;
+        r.ypx.v[i] = neg ? q.ymx.v[i] : q.ypx.v[i];
+        r.ymx.v[i] = neg ? q.ypx.v[i] : q.ymx.v[i];
+        r.t2d.v[i] = neg ? nt.v[i] : q.t2d.v[i];
     }
+    return r;
 }
 
-// P + Q for a table point Q given with its digit sign: a negative digit uses -Q,
-// which swaps y+x / y-x and flips the sign of the 2dxy term (so F and G trade places).
-__device__ __forceinline__ ge ge_add_niels(const ge& p, niels q, bool neg) {
-    fe_cswap(q.ypx, q.ymx, neg);
-    fe a = fe_mul(fe_sub(p.Y, p.X), q.ymx);
-    fe b = fe_mul(fe_add(p.Y, p.X), q.ypx);
-    fe c = fe_mul(p.T, q.t2d);
-    fe d = fe_add(p.Z, p.Z);
-    fe e = fe_sub(b, a), h = fe_add(b, a);
-    fe f = fe_sub(d, c), g = fe_add(d, c);
-    fe_cswap(f, g, neg);
+// P + Q for a table point Q, P's coordinates tight (so are the sum's).
+__device__ __forceinline__ ge ge_add_niels(const ge& p, const niels& q) {
+    const fe a = fe_mul(fe_sub_t(p.Y, p.X), q.ymx);
+    const fe b = fe_mul(fe_add_t(p.Y, p.X), q.ypx);
+    const fe c = fe_mul(p.T, q.t2d);
+    const fe d = fe_add_t(p.Z, p.Z);
+    const fe e = fe_sub_t(b, a), h = fe_add_t(b, a);
+    const fe f = fe_sub_t(d, c), g = fe_add_1(d, c);
     ge r;
     r.X = fe_mul(e, f);
     r.Y = fe_mul(g, h);
@@ -47,17 +48,17 @@ __device__ __forceinline__ ge ge_add_niels(const ge& p, niels q, bool neg) {
     return r;
 }
 
-// Last addition (digit >= 0): the sum's y as a fraction yn/yd and, optionally, x as xn/xd.
+// The last addition (P tight): the sum's y as a fraction yn/yd and, optionally, x as xn/xd.
 __device__ __forceinline__ void ge_add_niels_frac(const ge& p, const niels& q, fe& yn, fe& yd, fe* xn, fe* xd) {
-    fe a = fe_mul(fe_sub(p.Y, p.X), q.ymx);
-    fe b = fe_mul(fe_add(p.Y, p.X), q.ypx);
-    fe c = fe_mul(p.T, q.t2d);
-    fe d = fe_add(p.Z, p.Z);
-    yn = fe_add(b, a);
-    yd = fe_sub(d, c);
+    const fe a = fe_mul(fe_sub_t(p.Y, p.X), q.ymx);
+    const fe b = fe_mul(fe_add_t(p.Y, p.X), q.ypx);
+    const fe c = fe_mul(p.T, q.t2d);
+    const fe d = fe_add_t(p.Z, p.Z);
+    yn = fe_add_t(b, a);
+    yd = fe_sub_t(d, c);
     if (xn) {
-        *xn = fe_sub(b, a);
-        *xd = fe_add(d, c);
+        *xn = fe_sub_t(b, a);
+        *xd = fe_add_1(d, c);
     }
 }
 

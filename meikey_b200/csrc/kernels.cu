@@ -1,7 +1,7 @@
 // sm_100a kernels of the candidate-key search path.
 //
 //   k_build_table  fills the comb table in HBM: entry (row, k) = k·2^(off_row)·8B
-//                  (+ 2^254·B on the top row), affine (y+x, y-x, 2dxy), row 0 holds 2xy.
+//                  (+ 2^254·B on the top row), affine (y+x, y-x, 2dxy, -2dxy), row 0 holds ±2xy.
 //   k_keys<…>      one fused pass per key: seed (ChaCha20 / counter) -> SHA-512 -> clamp
 //                  -> comb multiply from the table -> y as a fraction -> per-thread
 //                  Montgomery batch + per-CTA pooled inversion -> canonical y -> base64
@@ -49,16 +49,6 @@ __device__ __forceinline__ niels load_entry(const uint4* table, u64 idx) {
     return n;
 }
 
-// bits [off, off+w) of the 256-bit value m (w <= 32)
-__device__ __forceinline__ u32 bits_at(const u64 m[4], u32 off, u32 w) {
-    u32 q = off >> 6, r = off & 63;
-    u64 lo = q == 0 ? m[0] : q == 1 ? m[1] : q == 2 ? m[2] : m[3];
-    u64 hi = q == 0 ? m[1] : q == 1 ? m[2] : q == 2 ? m[3] : 0ull;
-    u64 v = lo >> r;
-    if (r != 0) v |= hi << (64 - r);
-    return (u32)(v & ((1ull << w) - 1ull));
-}
-
 // ---------------------------------------------------------------------------
 // comb table build
 // ---------------------------------------------------------------------------
@@ -96,15 +86,14 @@ __global__ void __launch_bounds__(256, 2) k_build_table(uint4* table, const Comb
     fe x = mk32::fe_mul(P.X, zi), y = mk32::fe_mul(P.Y, zi);
     fe xy = mk32::fe_mul(x, y);
     fe t = row == 0 ? mk32::fe_add(xy, xy) : mk32::fe_mul(xy, d2);
-    u32 w[24];
+    u32 w[32];
     mk32::fe_to_words(mk32::fe_add(y, x), w);
     mk32::fe_to_words(mk32::fe_sub(y, x), w + 8);
     mk32::fe_to_words(t, w + 16);
+    mk32::fe_to_words(mk32::fe_sub(mk32::fe_zero(), t), w + 24);
     uint4* out = table + e * (COMB_STRIDE_WORDS / 4);
 #pragma unroll
-    for (int q = 0; q < 6; q++) out[q] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
-#pragma unroll
-    for (int q = 6; q < COMB_STRIDE_WORDS / 4; q++) out[q] = make_uint4(0, 0, 0, 0);
+    for (int q = 0; q < 8; q++) out[q] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
 }
 
 // ---------------------------------------------------------------------------
@@ -117,12 +106,24 @@ struct EntrySlot {
     uint4 q[2][6];
 };
 
-__device__ __forceinline__ void fetch_entry(EntrySlot& slot, int which, const uint4* table, u64 idx) {
+// Fetches the entry of a signed digit as (y+x, y-x, 2dxy) of the digit's own point: a negative
+// digit swaps the first two on their way into the slot and takes -2dxy, which the entry holds as
+// its last 32 bytes, so the addition needs no selects (48 an addition).  With the tight sums of
+// ge_add_niels and the rows of fe_mul that open a pair first, one addition takes 2320 instead of
+// 2451 cycles of an SM sub-partition (16 warps per SM, the multiply pipe 93 % busy), and the search
+// of hashed seeds runs at 0.926 instead of 0.889 G keys/s.
+__device__ __forceinline__ void fetch_entry(EntrySlot& slot, int which, const uint4* table, u64 idx, bool neg) {
     const uint4* src = table + idx * (COMB_STRIDE_WORDS / 4);
-    u32 dst = (u32)__cvta_generic_to_shared(&slot.q[which][0]);
+    const u32 dst = (u32)__cvta_generic_to_shared(&slot.q[which][0]);
+    const u32 lo = neg ? 32u : 0u;
+    const uint4* t = src + (neg ? 6 : 4);
 #pragma unroll
-    for (int q = 0; q < 6; q++)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + 16 * q), "l"(src + q) : "memory");
+    for (int q = 0; q < 2; q++) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + lo + 16 * q), "l"(src + q) : "memory");
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + 32 - lo + 16 * q), "l"(src + 2 + q)
+                     : "memory");
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + 64 + 16 * q), "l"(t + q) : "memory");
+    }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
 }
 
@@ -144,37 +145,48 @@ __device__ __forceinline__ niels read_entry(const EntrySlot& slot, int which) {
     return n;
 }
 
-// signed digit of row `row` (rows before the top one), updating the carry
-__device__ __forceinline__ int next_digit(const CombGeom& g, const u64 m[4], u32 row, int& carry) {
-    u32 w = g.width[row];
-    int v = (int)bits_at(m, g.offset[row], w) + carry;
-    carry = (v + (1 << (w - 1))) >> w;
-    return v - (carry << w);
+// The digits of a clamped scalar's comb number m (bits 3..253 of s), lowest row first: m is
+// shifted down by each row's width.
+struct Digits {
+    u32 m[8];
+    int carry;
+};
+
+__device__ __forceinline__ Digits digits_of(const u64 s[4]) {
+    Digits d;
+    const u64 m[4] = {s[0] >> 3 | s[1] << 61, s[1] >> 3 | s[2] << 61, s[2] >> 3 | s[3] << 61,
+                      (s[3] >> 3) & ((1ull << (251 - 192)) - 1ull)};
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        d.m[2 * i] = (u32)m[i];
+        d.m[2 * i + 1] = (u32)(m[i] >> 32);
+    }
+    d.carry = 0;
+    return d;
+}
+
+// the next row's digit; `top` (the last row): unsigned, the carry lands in it unchanged
+__device__ __forceinline__ int next_digit(Digits& d, u32 w, bool top) {
+    const int v = (int)(d.m[0] & ((1u << w) - 1u)) + d.carry;
+#pragma unroll
+    for (int i = 0; i < 7; i++) d.m[i] = __funnelshift_r(d.m[i], d.m[i + 1], w);
+    d.m[7] >>= w;
+    d.carry = top ? 0 : (v + (1 << (w - 1))) >> w;
+    return v - (d.carry << w);
 }
 
 __device__ __forceinline__ u64 entry_index(const CombGeom& g, u32 row, int d) {
     return g.row_base[row] + (u64)(d < 0 ? -d : d);
 }
 
-// bits 3..253 of a clamped scalar s: the number whose digits the comb rows take
-__device__ __forceinline__ void comb_m(const u64 s[4], u64 m[4]) {
-    m[0] = s[0] >> 3 | s[1] << 61;
-    m[1] = s[1] >> 3 | s[2] << 61;
-    m[2] = s[2] >> 3 | s[3] << 61;
-    m[3] = (s[3] >> 3) & ((1ull << (251 - 192)) - 1ull);
-}
-
-// Row 0's entry (digit sign `neg`) in extended coordinates: X = 2x, Y = 2y, Z = 2, T = 2xy,
-// without a multiplication (row 0 stores 2xy).
-__device__ __forceinline__ ge comb_row0(niels n, bool neg) {
+// Row 0's entry in extended coordinates: X = 2x, Y = 2y, Z = 2, T = 2xy, without a multiplication
+// (row 0 stores 2xy).
+__device__ __forceinline__ ge comb_row0(const niels& n) {
     ge P;
-    mk32::fe_cswap(n.ypx, n.ymx, neg);
-    P.X = mk32::fe_sub(n.ypx, n.ymx);
-    P.Y = mk32::fe_add(n.ypx, n.ymx);
+    P.X = mk32::fe_tight(mk32::fe_sub_t(n.ypx, n.ymx));
+    P.Y = mk32::fe_tight(mk32::fe_add_t(n.ypx, n.ymx));
     P.Z = mk32::fe_small(2);
-    fe nt = mk32::fe_sub(mk32::fe_zero(), n.t2d);
-#pragma unroll
-    for (int i = 0; i < 8; i++) P.T.v[i] = neg ? nt.v[i] : n.t2d.v[i];
+    P.T = n.t2d;
     return P;
 }
 
@@ -182,30 +194,24 @@ __device__ __forceinline__ ge comb_row0(niels n, bool neg) {
 // Row r's entry is fetched while row r-1 is being added.
 __device__ __forceinline__ void comb_mul(const uint4* __restrict__ table, const CombGeom& g, const u64 s[4],
                                          EntrySlot& slot, fe& yn, fe& yd, fe* xn, fe* xd) {
-    u64 m[4];
-    comb_m(s, m);
+    Digits dg = digits_of(s);
     const u32 rows = g.rows;
-    int carry = 0;
-    int d0 = next_digit(g, m, 0, carry);
-    fetch_entry(slot, 0, table, entry_index(g, 0, d0));
-    int dn = next_digit(g, m, 1, carry);  // rows >= 3, so row 1 is not the top row
-    fetch_entry(slot, 1, table, entry_index(g, 1, dn));
+    auto fetch = [&](u32 row) {
+        const int d = next_digit(dg, g.width[row], row + 1 == rows);
+        fetch_entry(slot, row & 1, table, entry_index(g, row, d), d < 0);
+    };
+    fetch(0);
+    fetch(1);
     wait_entries<1>();
-    ge P = comb_row0(read_entry(slot, 0), d0 < 0);
+    ge P = comb_row0(read_entry(slot, 0));
 #pragma unroll 1
     for (u32 row = 1; row + 1 < rows; row++) {
-        const int d = dn;
-        // prefetch row+1 (the top row's digit is unsigned: the carry lands in it unchanged)
-        if (row + 2 < rows) dn = next_digit(g, m, row + 1, carry);
-        else dn = (int)bits_at(m, g.offset[row + 1], g.width[row + 1]) + carry;
-        fetch_entry(slot, (row + 1) & 1, table, entry_index(g, row + 1, dn));
+        fetch(row + 1);
         wait_entries<1>();
-        niels n = read_entry(slot, row & 1);
-        P = mk32::ge_add_niels(P, n, d < 0);
+        P = mk32::ge_add_niels(P, read_entry(slot, row & 1));
     }
     wait_entries<0>();
-    niels n = read_entry(slot, (rows - 1) & 1);
-    mk32::ge_add_niels_frac(P, n, yn, yd, xn, xd);
+    mk32::ge_add_niels_frac(P, read_entry(slot, (rows - 1) & 1), yn, yd, xn, xd);
 }
 
 // comb_mul with one 8-round step of the SHA-512 `run` (the next iteration's seed) in every
@@ -214,36 +220,26 @@ __device__ __forceinline__ void comb_mul(const uint4* __restrict__ table, const 
 // 10 full rows carry the 80 rounds.  y = yn/yd only.
 __device__ __forceinline__ void comb_mul_sha(const uint4* __restrict__ table, const CombGeom& g, const u64 s[4],
                                              EntrySlot& slot, fe& yn, fe& yd, mkh::ShaRun& run) {
-    u64 m[4];
-    comb_m(s, m);
+    Digits dg = digits_of(s);
     const u32 rows = g.rows;
-    int carry = 0;
-    int d0 = next_digit(g, m, 0, carry);
-    fetch_entry(slot, 0, table, entry_index(g, 0, d0));
-    int dn = next_digit(g, m, 1, carry);
-    fetch_entry(slot, 1, table, entry_index(g, 1, dn));
+    auto fetch = [&](u32 row) {
+        const int d = next_digit(dg, g.width[row], row + 1 == rows);
+        fetch_entry(slot, row & 1, table, entry_index(g, row, d), d < 0);
+    };
+    fetch(0);
+    fetch(1);
     wait_entries<1>();
-    ge P = comb_row0(read_entry(slot, 0), d0 < 0);
+    ge P = comb_row0(read_entry(slot, 0));
 #pragma unroll 1
     for (u32 row = 1; row + 1 < rows; row++) {
-        const int d = dn;
-        // the next row's digit without a branch (the top row's is unsigned: the carry lands
-        // in it unchanged)
-        int c2 = carry;
-        const int sd = next_digit(g, m, row + 1, c2);
-        const int td = (int)bits_at(m, g.offset[row + 1], g.width[row + 1]) + carry;
-        const bool top = row + 2 >= rows;
-        dn = top ? td : sd;
-        carry = top ? carry : c2;
-        fetch_entry(slot, (row + 1) & 1, table, entry_index(g, row + 1, dn));
+        fetch(row + 1);
         wait_entries<1>();
-        niels n = read_entry(slot, row & 1);
+        const niels n = read_entry(slot, row & 1);
         mkh::sha_run_step(run, 8u * (row - 1));
-        P = mk32::ge_add_niels(P, n, d < 0);
+        P = mk32::ge_add_niels(P, n);
     }
     wait_entries<0>();
-    niels n = read_entry(slot, (rows - 1) & 1);
-    mk32::ge_add_niels_frac(P, n, yn, yd, nullptr, nullptr);
+    mk32::ge_add_niels_frac(P, read_entry(slot, (rows - 1) & 1), yn, yd, nullptr, nullptr);
 }
 
 // 6-bit values of the 44-character base64 tail of the key blob (0x20 then the key),
@@ -438,20 +434,16 @@ __device__ __forceinline__ niels smem_niels(const uint4* q);
 // Comb multiply with the whole table in shared memory (entries 96 bytes apart, `stab`): every
 // row reads its entry there, with no staging; y = yn/yd only.
 __device__ __forceinline__ void comb_mul_smem(const uint4* stab, const CombGeom& g, const u64 s[4], fe& yn, fe& yd) {
-    u64 m[4];
-    comb_m(s, m);
+    Digits dg = digits_of(s);
     const u32 rows = g.rows;
-    int carry = 0;
-    int d = next_digit(g, m, 0, carry);
-    ge P = comb_row0(smem_niels(stab + entry_index(g, 0, d) * 6), d < 0);
+    auto entry = [&](u32 row) {
+        const int d = next_digit(dg, g.width[row], row + 1 == rows);
+        return mk32::niels_signed(smem_niels(stab + entry_index(g, row, d) * 6), d < 0);
+    };
+    ge P = comb_row0(entry(0));
 #pragma unroll 1
-    for (u32 row = 1; row + 1 < rows; row++) {
-        d = next_digit(g, m, row, carry);
-        P = mk32::ge_add_niels(P, smem_niels(stab + entry_index(g, row, d) * 6), d < 0);
-    }
-    // the top row's digit is unsigned: the carry lands in it unchanged
-    d = (int)bits_at(m, g.offset[rows - 1], g.width[rows - 1]) + carry;
-    mk32::ge_add_niels_frac(P, smem_niels(stab + entry_index(g, rows - 1, d) * 6), yn, yd, nullptr, nullptr);
+    for (u32 row = 1; row + 1 < rows; row++) P = mk32::ge_add_niels(P, entry(row));
+    mk32::ge_add_niels_frac(P, entry(rows - 1), yn, yd, nullptr, nullptr);
 }
 
 // Comb multiplies of the KPT scalars (IMAD work) into the batch; STAB: from the table in
@@ -628,7 +620,7 @@ __device__ __forceinline__ ge incr_start(const KeyLaunch& L, u64 offset) {
 #pragma unroll 1
     for (int w = 0; w < INCR_WINDOWS; w++) {
         const u32 d = (u32)(offset >> (4 * w)) & 15u;
-        if (d) P = mk32::ge_add_niels(P, load_entry(L.incr, (u64)w * 16 + d), false);
+        if (d) P = mk32::ge_add_niels(P, load_entry(L.incr, (u64)w * 16 + d));
     }
     return P;
 }
@@ -658,7 +650,7 @@ __device__ __forceinline__ void step_to_yx(uint4* steps, u32 j) {
 // The batch's slots are filled in the order Q, +1, -1, +2, -2, ..., -KPT/2 (incr_key).
 template <int KPT>
 __device__ __forceinline__ void incr_fracs(const ge& Q, const uint4* steps, Batch<KPT>& b) {
-    const fe z2 = mk32::fe_add(Q.Z, Q.Z);
+    const fe z2 = mk32::fe_add_t(Q.Z, Q.Z);
     b.a[0] = Q.Y;
     b.den[0] = Q.Z;
     fe run = Q.Z;
@@ -667,15 +659,15 @@ __device__ __forceinline__ void incr_fracs(const ge& Q, const uint4* steps, Batc
         const niels t = smem_niels(steps + d * (ENTRY_WORDS / 4));  // (2y, 2x, 2dxy)
         const fe yy = mk32::fe_mul(Q.Y, t.ypx), xx = mk32::fe_mul(Q.X, t.ymx), c = mk32::fe_mul(Q.T, t.t2d);
         if (d < KPT / 2) {
-            const fe den = mk32::fe_sub(z2, c);
+            const fe den = mk32::fe_sub_t(z2, c);
             b.den[2 * d - 1] = den;
-            b.a[2 * d - 1] = mk32::fe_mul(mk32::fe_add(yy, xx), run);
+            b.a[2 * d - 1] = mk32::fe_mul(mk32::fe_add_t(yy, xx), run);
             run = mk32::fe_mul(run, den);
         }
         const int s = d < KPT / 2 ? 2 * d : KPT - 1;
-        const fe den = mk32::fe_add(z2, c);
+        const fe den = mk32::fe_add_1(z2, c);
         b.den[s] = den;
-        b.a[s] = mk32::fe_mul(mk32::fe_sub(yy, xx), run);
+        b.a[s] = mk32::fe_mul(mk32::fe_sub_t(yy, xx), run);
         run = mk32::fe_mul(run, den);
     }
     b.prod = run;
@@ -824,7 +816,7 @@ __global__ void __launch_bounds__(BLOCK, 512 / BLOCK) k_search(const KeyLaunch L
                 batch[b].prod = mk32::fe_small(1);  // a warp past the last run
             } else if (INCR) {
                 incr_fracs<KPT>(Q, steps, batch[b]);
-                Q = mk32::ge_add_niels(Q, words_niels(L.delta), false);
+                Q = mk32::ge_add_niels(Q, words_niels(L.delta));
             } else if (SHAI) {
                 if (it == 0) scalars<KPT>(L, key, mid, first_of(0), sc);
                 combs_sha<KPT>(L, g, sc, slot, batch[b], key, mid, first_of(it + 1));
