@@ -329,7 +329,7 @@ int mk_ctx_create(int device, const mk_options* options, mk_ctx** out) try {
         c->table_smem = (uint32_t)bytes;
     }
     int occ = 0;
-    cudaError_t oe = mkb::keys_occupancy(false, false, c->kpt, c->block, c->layout, c->table_smem, &occ);
+    cudaError_t oe = mkb::search_occupancy(c->kpt, c->block, c->layout, c->table_smem, &occ);
     if (oe != cudaSuccess && c->table_smem) {
         cudaGetLastError();
         return fail(c, MK_ERR_OUT_OF_RANGE, "the comb table and the CTA's buffers do not fit in shared memory");
@@ -435,7 +435,8 @@ int mk_derive(mk_ctx* c, const uint8_t key[32], int seed_source, uint64_t first,
     const uint64_t per_launch = 1ull << 22;
     uint8_t* d_out = nullptr;
     uint64_t cap = std::min(n, per_launch);
-    MK_CUDA(c, cudaMalloc(&d_out, cap * 32));
+    // from the context's pool: cudaMalloc and cudaFree cost more than a short derive
+    if (!pool_alloc(c, &d_out, cap * 32)) return fail(c, MK_ERR_OUT_OF_MEMORY, "derive output");
     for (uint64_t done = 0; done < n; done += per_launch) {
         uint64_t cnt = std::min(per_launch, n - done);
         mkb::KeyLaunch L{};
@@ -448,17 +449,15 @@ int mk_derive(mk_ctx* c, const uint8_t key[32], int seed_source, uint64_t first,
         L.out = d_out;
         L.count = cnt;
         if (seed_source == MK_SEED_INCREMENTAL) set_incremental(c, key, L.base, L);
-        uint64_t threads = (cnt + c->kpt - 1) / c->kpt;
-        uint32_t grid = (uint32_t)((threads + c->block - 1) / c->block);
-        cudaError_t e = mkb::launch_keys(L, true, c->kpt, c->block, grid, c->stream);
+        cudaError_t e = mkb::launch_derive(L, c->info.sms, c->stream);
         if (e == cudaSuccess) e = cudaMemcpyAsync(out + 32 * done, d_out, cnt * 32, cudaMemcpyDeviceToHost, c->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
         if (e != cudaSuccess) {
-            cudaFree(d_out);
+            pool_free(c, d_out);
             return cuda_fail(c, e, "derive");
         }
     }
-    cudaFree(d_out);
+    pool_free(c, d_out);
     return MK_OK;
 } MK_ABI_CATCH(c ? &c->err : nullptr)
 
@@ -484,9 +483,7 @@ int mk_derive_noalloc(mk_ctx* c, const uint8_t key[32], int seed_source, uint64_
     L.base = first;
     L.out = staging;
     L.count = n;
-    uint64_t threads = (n + c->kpt - 1) / c->kpt;
-    uint32_t grid = (uint32_t)((threads + c->block - 1) / c->block);
-    MK_CUDA(c, mkb::launch_keys(L, true, c->kpt, c->block, grid, c->stream));
+    MK_CUDA(c, mkb::launch_derive(L, c->info.sms, c->stream));
     MK_CUDA(c, cudaMemcpyAsync(out, staging, n * 32, cudaMemcpyDeviceToHost, c->stream));
     MK_CUDA(c, cudaStreamSynchronize(c->stream));
     return MK_OK;
@@ -802,7 +799,7 @@ static int enqueue(mk_job* j, uint64_t base, uint32_t iters) {
     MK_CUDA(c, cudaSetDevice(c->device));
     MK_CUDA(c, cudaMemsetAsync(j->d_job, 0, 8, c->stream));  // hit_count and status; keep stop
     mkb::KeyLaunch L = search_params(j, base, iters);
-    MK_CUDA(c, mkb::launch_keys(L, false, c->kpt, c->block, c->grid, c->stream));
+    MK_CUDA(c, mkb::launch_search(L, c->kpt, c->block, c->grid, c->stream));
     j->h2d += sizeof L;  // kernel parameters
     return MK_OK;
 }
@@ -1071,9 +1068,9 @@ int mk_job_graph_create(mk_job* j, uint32_t iters, uint32_t launches, mk_graph**
     if (e != cudaSuccess) return bail(e, "cudaGraphAddMemsetNode");
     const void* func = nullptr;
     size_t dyn = 0;
-    e = mkb::keys_kernel(false, j->source == MK_SEED_INCREMENTAL, c->kpt, c->block, c->layout, dfa_smem_bytes(j),
+    e = mkb::search_kernel(j->source == MK_SEED_INCREMENTAL, c->kpt, c->block, c->layout, dfa_smem_bytes(j),
                          c->table_smem, &func, &dyn);
-    if (e != cudaSuccess) return bail(e, "keys_kernel");
+    if (e != cudaSuccess) return bail(e, "search_kernel");
     for (uint32_t i = 0; i < launches; i++) {
         g->params[i] = search_params(j, g->span * i, iters);
         void* args[] = {&g->params[i]};
@@ -1101,7 +1098,7 @@ static int graph_enqueue(mk_graph* g, uint64_t base) {
     mk_ctx* c = j->ctx;
     MK_CUDA(c, cudaSetDevice(c->device));
     // the job's needles may have changed since the graph was made: size the DFA staging anew
-    MK_CUDA(c, mkb::keys_kernel(false, j->source == MK_SEED_INCREMENTAL, c->kpt, c->block, c->layout, dfa_smem_bytes(j),
+    MK_CUDA(c, mkb::search_kernel(j->source == MK_SEED_INCREMENTAL, c->kpt, c->block, c->layout, dfa_smem_bytes(j),
                                 c->table_smem, &g->func,
                                 &g->dyn));
     for (size_t i = 0; i < g->nodes.size(); i++) {

@@ -1022,30 +1022,35 @@ __global__ void __launch_bounds__(BLOCK, 1) k_search_hw(const KeyLaunch L) {
     if (L.sink) L.sink[gid] = sink;
 }
 
-// Derive kernel: full public keys (x sign included) of indices base .. base+count-1;
-// one iteration, per-CTA pooled inversion of 2·KPT denominators per thread.  INCR: the
+constexpr int DERIVE_BLOCK = 128;
+constexpr uint32_t DERIVE_MAX_KEYS = 16;
+
+// Derive kernel: full public keys (x sign included) of indices base .. base+count-1, KPT
+// consecutive ones per thread, with one inversion of its 2·KPT denominators per thread.  INCR: the
 // thread's keys are Q + j·B with Q = (s0 + first)·B; key j gives y = (b+a)/(2Z-c) and
 // x = (b-a)/(2Z+c) of the mixed addition with step entry j (entry 0 is the identity).
-template <int KPT, int BLOCK, bool INCR>
-__global__ void __launch_bounds__(BLOCK, 512 / BLOCK) k_derive(const KeyLaunch L) {
+// Threads do not work together: with the division steps an inversion costs about two thirds of a
+// key, and a call of few keys is a single dependent chain per thread, so the keys go to as many
+// threads as one wave holds (launch_derive) instead of waiting behind each other.
+template <int KPT, bool INCR>
+__global__ void __launch_bounds__(DERIVE_BLOCK, 512 / DERIVE_BLOCK) k_derive(const KeyLaunch L) {
     constexpr int NUM = 2 * KPT;
     extern __shared__ uint4 dyn_smem[];
-    fe* prod = reinterpret_cast<fe*>(dyn_smem);
-    fe* scratch = prod + BLOCK;
-    EntrySlot* slots = reinterpret_cast<EntrySlot*>(scratch + BLOCK);
+    EntrySlot* slots = reinterpret_cast<EntrySlot*>(dyn_smem);
     __shared__ CombGeom g;
     __shared__ u32 key[8];
     __shared__ uint4 steps[INCR ? INCR_STEPS * (ENTRY_WORDS / 4) : 1];
     const u32 tid = threadIdx.x;
-    const u64 gid = (u64)blockIdx.x * BLOCK + tid;
-    if (INCR) load_steps(L, steps, tid, BLOCK);
+    const u64 gid = (u64)blockIdx.x * DERIVE_BLOCK + tid;
+    if (INCR) load_steps(L, steps, tid, DERIVE_BLOCK);
     {
         const u32* src = (const u32*)&L.geom;
         u32* dst = (u32*)&g;
-        for (u32 i = tid; i < sizeof(CombGeom) / 4; i += BLOCK) dst[i] = src[i];
+        for (u32 i = tid; i < sizeof(CombGeom) / 4; i += DERIVE_BLOCK) dst[i] = src[i];
         if (tid < 8) key[tid] = L.key[tid];
     }
     __syncthreads();
+    if (gid * KPT >= L.count) return;
     mkh::CounterMid mid;
     if (L.seed_src == 1) mid = mkh::counter_mid(key);
     const u64 first = L.base + gid * KPT;
@@ -1056,19 +1061,19 @@ __global__ void __launch_bounds__(BLOCK, 512 / BLOCK) k_derive(const KeyLaunch L
     fe ypx, ymx, z2;
     if (INCR) {
         Q = incr_start(L, gid * KPT);
-        ypx = mk32::fe_add(Q.Y, Q.X);
-        ymx = mk32::fe_sub(Q.Y, Q.X);
-        z2 = mk32::fe_add(Q.Z, Q.Z);
+        ypx = mk32::fe_add_t(Q.Y, Q.X);
+        ymx = mk32::fe_sub_t(Q.Y, Q.X);
+        z2 = mk32::fe_add_t(Q.Z, Q.Z);
     }
 #pragma unroll 1
     for (int j = 0; j < KPT; j++) {
         if (INCR) {
             const niels t = smem_niels(steps + j * (ENTRY_WORDS / 4));
             const fe A = mk32::fe_mul(ymx, t.ymx), B = mk32::fe_mul(ypx, t.ypx), C = mk32::fe_mul(Q.T, t.t2d);
-            num[2 * j] = mk32::fe_add(B, A);
-            den[2 * j] = mk32::fe_sub(z2, C);
-            num[2 * j + 1] = mk32::fe_sub(B, A);
-            den[2 * j + 1] = mk32::fe_add(z2, C);
+            num[2 * j] = mk32::fe_add_t(B, A);
+            den[2 * j] = mk32::fe_sub_t(z2, C);
+            num[2 * j + 1] = mk32::fe_sub_t(B, A);
+            den[2 * j + 1] = mk32::fe_add_1(z2, C);
         } else {
             u64 s[4];
             scalar_of(L.seed_src, key, mid, first + (u64)j, blk, blk_id, s);
@@ -1077,14 +1082,10 @@ __global__ void __launch_bounds__(BLOCK, 512 / BLOCK) k_derive(const KeyLaunch L
         pre[2 * j] = j == 0 ? den[0] : mk32::fe_mul(pre[2 * j - 1], den[2 * j]);
         pre[2 * j + 1] = mk32::fe_mul(pre[2 * j], den[2 * j + 1]);
     }
-    prod[tid] = pre[NUM - 1];
-    __syncthreads();
-    if (tid < 32) invert_pools(prod, scratch, BLOCK);
-    __syncthreads();
-    fe inv = prod[tid];
+    fe inv = mk32::fe_invert(pre[NUM - 1]);
 #pragma unroll 1
     for (int j = KPT - 1; j >= 0; j--) {
-        const u64 idx = first + (u64)j;
+        const u64 at = gid * KPT + (u64)j;
         const int ex = 2 * j + 1, ey = 2 * j;
         fe xinv = mk32::fe_mul(inv, pre[ex - 1]);
         inv = mk32::fe_mul(inv, den[ex]);
@@ -1094,8 +1095,8 @@ __global__ void __launch_bounds__(BLOCK, 512 / BLOCK) k_derive(const KeyLaunch L
         mk32::fe_to_words(mk32::fe_mul(num[ex], xinv), xw);
         mk32::fe_to_words(mk32::fe_mul(num[ey], yinv), pk);
         pk[7] |= (xw[0] & 1u) << 31;
-        if (idx - L.base < L.count) {
-            uint4* o = (uint4*)(L.out + (idx - L.base) * 32);
+        if (at < L.count) {
+            uint4* o = (uint4*)(L.out + at * 32);
             o[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
             o[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
         }
@@ -1108,18 +1109,17 @@ __global__ void __launch_bounds__(BLOCK, 512 / BLOCK) k_derive(const KeyLaunch L
 
 #define MK_VARIANTS(X) X(4, 256) X(8, 256) X(16, 256) X(4, 512) X(8, 512) X(16, 512)
 
-// dynamic shared memory: products and inversion scratch (two buffers each for the
-// search pipeline) and the per-thread table staging slots
-// (the incremental source reads no comb table and needs no staging slots)
-static size_t dyn_bytes(bool derive, bool incr, uint32_t block, uint32_t layout, uint32_t table_smem) {
+// dynamic shared memory of a search: products and inversion scratch (two buffers each) and the
+// per-thread table staging slots (the incremental source reads no comb table and needs none)
+static size_t dyn_bytes(bool incr, uint32_t block, uint32_t layout, uint32_t table_smem) {
     const size_t fe_bytes = 32;
-    if (layout == LAYOUT_HASH_WARPS && !derive && !incr) {  // k_search_hw: 352 comb threads, plus the two-slot scalar ring
+    if (layout == LAYOUT_HASH_WARPS && !incr) {  // k_search_hw: 352 comb threads, plus the two-slot scalar ring
         const size_t ct = 352;
         return 4 * ct * fe_bytes + ct * sizeof(EntrySlot) + 2 * 4 * ct * 32;
     }
-    const size_t threads = derive ? block : search_kernel_threads(incr, block, layout, table_smem);
-    if (table_smem && !derive && !incr) return 4 * threads * fe_bytes + table_smem;  // the table in place of the slots
-    return (derive ? 2 : 4) * threads * fe_bytes + (incr ? 0 : threads * sizeof(EntrySlot));
+    const size_t threads = search_kernel_threads(incr, block, layout, table_smem);
+    if (table_smem && !incr) return 4 * threads * fe_bytes + table_smem;  // the table in place of the slots
+    return 4 * threads * fe_bytes + (incr ? 0 : threads * sizeof(EntrySlot));
 }
 
 static const void* hw_kernel_of(uint32_t kpt, uint32_t block) {
@@ -1138,16 +1138,13 @@ static const void* stab_kernel_of(uint32_t kpt, uint32_t block) {
     return nullptr;
 }
 
-static const void* kernel_of(bool derive, bool incr, uint32_t kpt, uint32_t block) {
-    if (!derive && !incr)
+static const void* kernel_of(bool incr, uint32_t kpt, uint32_t block) {
+    if (!incr)
         return block == 512 ? (const void*)k_search<HASHED_KEYS, 512, false, true>
                : block == 256 ? (const void*)k_search<HASHED_KEYS, 256, false, true>
                               : nullptr;
-#define MK_FN(K, B)                                                                                       \
-    if (kpt == K && block == B) {                                                                         \
-        if (derive) return incr ? (const void*)k_derive<K, B, true> : (const void*)k_derive<K, B, false>; \
-        return (const void*)k_search<K, B, true, false>;                                                  \
-    }
+#define MK_FN(K, B) \
+    if (kpt == K && block == B) return (const void*)k_search<K, B, true, false>;
     MK_VARIANTS(MK_FN)
 #undef MK_FN
     return nullptr;
@@ -1166,52 +1163,65 @@ static const void* shai_kernel_of(uint32_t kpt, uint32_t block) {
     return nullptr;
 }
 
-// the kernel of a variant (the table-in-shared-memory search when table_smem > 0)
-static const void* variant_kernel(bool derive, bool incr, uint32_t kpt, uint32_t block, uint32_t layout,
-                                  uint32_t table_smem) {
-    if (layout == LAYOUT_INTERLEAVED && !derive && !incr) return table_smem ? nullptr : shai_kernel_of(kpt, block);
-    const bool hw = layout == LAYOUT_HASH_WARPS && !derive && !incr;
-    if (table_smem && !derive && !incr) return layout == LAYOUT_INVERTER_WARP ? stab_kernel_of(kpt, block) : nullptr;
-    return hw ? hw_kernel_of(kpt, block) : kernel_of(derive, incr, kpt, block);
+// the search kernel of a variant (the table-in-shared-memory search when table_smem > 0)
+static const void* variant_kernel(bool incr, uint32_t kpt, uint32_t block, uint32_t layout, uint32_t table_smem) {
+    if (layout == LAYOUT_INTERLEAVED && !incr) return table_smem ? nullptr : shai_kernel_of(kpt, block);
+    if (table_smem && !incr) return layout == LAYOUT_INVERTER_WARP ? stab_kernel_of(kpt, block) : nullptr;
+    return layout == LAYOUT_HASH_WARPS && !incr ? hw_kernel_of(kpt, block) : kernel_of(incr, kpt, block);
 }
 
-cudaError_t launch_keys(const KeyLaunch& L, bool derive, uint32_t kpt, uint32_t block, uint32_t grid, cudaStream_t st) {
+cudaError_t search_kernel(bool incr, uint32_t kpt, uint32_t block, uint32_t layout, uint32_t dfa_smem,
+                          uint32_t table_smem, const void** func, size_t* dyn) {
+    const bool hw = layout == LAYOUT_HASH_WARPS && !incr;
+    const uint32_t tsm = incr ? 0 : table_smem;
+    const void* f = variant_kernel(incr, kpt, block, layout, tsm);
+    // the hashing-warp kernel's scalar ring and a comb table take the shared memory of DFA tables
+    if (!f || dfa_smem > DFA_SMEM_MAX || ((hw || tsm) && dfa_smem)) return cudaErrorInvalidValue;
+    *func = f;
+    *dyn = dyn_bytes(incr, block, layout, tsm) + dfa_smem;
+    return prepare(f, *dyn);
+}
+
+cudaError_t launch_search(const KeyLaunch& L, uint32_t kpt, uint32_t block, uint32_t grid, cudaStream_t st) {
     const bool incr = L.seed_src == SEED_INCREMENTAL;
     if (incr && (kpt > (uint32_t)INCR_STEPS || !L.incr)) return cudaErrorInvalidValue;
-    if (L.dfa_smem > DFA_SMEM_MAX || (derive && L.dfa_smem)) return cudaErrorInvalidValue;
-    const bool hw = L.layout == LAYOUT_HASH_WARPS && !derive && !incr;
-    if (hw && L.dfa_smem) return cudaErrorInvalidValue;  // the scalar ring takes that shared memory
-    const uint32_t tsm = derive || incr ? 0 : L.table_smem;
-    if (tsm && L.dfa_smem) return cudaErrorInvalidValue;  // the table takes that shared memory
-    const void* f = variant_kernel(derive, incr, kpt, block, L.layout, tsm);
-    if (!f) return cudaErrorInvalidValue;
-    const size_t dyn = dyn_bytes(derive, incr, block, L.layout, tsm) + L.dfa_smem;
-    cudaError_t e = prepare(f, dyn);
+    const void* f = nullptr;
+    size_t dyn = 0;
+    cudaError_t e = search_kernel(incr, kpt, block, L.layout, L.dfa_smem, L.table_smem, &f, &dyn);
     if (e != cudaSuccess) return e;
     void* args[] = {const_cast<KeyLaunch*>(&L)};
     return cudaLaunchKernel(f, dim3(grid), dim3(block), args, dyn, st);
 }
 
-cudaError_t keys_kernel(bool derive, bool incr, uint32_t kpt, uint32_t block, uint32_t layout, uint32_t dfa_smem,
-                        uint32_t table_smem, const void** func, size_t* dyn) {
-    const bool hw = layout == LAYOUT_HASH_WARPS && !derive && !incr;
-    const uint32_t tsm = derive || incr ? 0 : table_smem;
-    const void* f = variant_kernel(derive, incr, kpt, block, layout, tsm);
-    if (!f || dfa_smem > DFA_SMEM_MAX || ((hw || tsm) && dfa_smem)) return cudaErrorInvalidValue;
-    *func = f;
-    *dyn = dyn_bytes(derive, incr, block, layout, tsm) + dfa_smem;
-    return prepare(f, *dyn);
-}
-
-cudaError_t keys_occupancy(bool derive, bool incr, uint32_t kpt, uint32_t block, uint32_t layout, uint32_t table_smem,
-                           int* blocks_per_sm) {
-    const uint32_t tsm = derive || incr ? 0 : table_smem;
-    const void* f = variant_kernel(derive, incr, kpt, block, layout, tsm);
-    if (!f) return cudaErrorInvalidValue;
-    const size_t dyn = dyn_bytes(derive, incr, block, layout, tsm);
-    cudaError_t e = prepare(f, dyn);
+cudaError_t search_occupancy(uint32_t kpt, uint32_t block, uint32_t layout, uint32_t table_smem, int* blocks_per_sm) {
+    const void* f = nullptr;
+    size_t dyn = 0;
+    cudaError_t e = search_kernel(false, kpt, block, layout, 0, table_smem, &f, &dyn);
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, f, (int)block, dyn);
+}
+
+// Keys per thread of a derive: the fewest that let one wave (512 threads per SM) hold them all, at
+// most DERIVE_MAX_KEYS.  On B200 a call of 257 keys takes 72 us (61 us in the kernel) where 16 keys
+// behind each other in a thread took 1286; 4099 keys 100 us against 726 at 8; 2^20 keys are 1.4 ms in
+// the kernel, at 16 keys per thread.
+cudaError_t launch_derive(const KeyLaunch& L, uint32_t sms, cudaStream_t st) {
+    const bool incr = L.seed_src == SEED_INCREMENTAL;
+    if (incr && !L.incr) return cudaErrorInvalidValue;
+    uint32_t k = 1;
+    while (k < DERIVE_MAX_KEYS && (L.count + k - 1) / k > (uint64_t)sms * 512) k *= 2;
+    const void* f = nullptr;
+#define MK_FN(K) \
+    if (k == K) f = incr ? (const void*)k_derive<K, true> : (const void*)k_derive<K, false>;
+    MK_FN(1) MK_FN(2) MK_FN(4) MK_FN(8) MK_FN(16)
+#undef MK_FN
+    const size_t dyn = incr ? 0 : DERIVE_BLOCK * sizeof(EntrySlot);
+    cudaError_t e = prepare(f, dyn);
+    if (e != cudaSuccess) return e;
+    const uint64_t threads = (L.count + k - 1) / k;
+    void* args[] = {const_cast<KeyLaunch*>(&L)};
+    return cudaLaunchKernel(f, dim3((uint32_t)((threads + DERIVE_BLOCK - 1) / DERIVE_BLOCK)), dim3(DERIVE_BLOCK), args,
+                            dyn, st);
 }
 
 cudaError_t launch_build_table(uint4* table, const CombGeom& g, const uint32_t* points, uint64_t first,

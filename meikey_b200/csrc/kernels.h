@@ -83,7 +83,9 @@ constexpr int INCR_WINDOWS = 8;   // 4-bit windows of a thread's offset (offsets
 constexpr int INCR_STEPS = 16;    // j·B for j = 0 .. keys per thread - 1
 constexpr int INCR_ENTRIES = INCR_WINDOWS * 16 + INCR_STEPS;
 
-cudaError_t launch_keys(const KeyLaunch& L, bool derive, uint32_t kpt, uint32_t block, uint32_t grid, cudaStream_t st);
+cudaError_t launch_search(const KeyLaunch& L, uint32_t kpt, uint32_t block, uint32_t grid, cudaStream_t st);
+// Public keys of L.base .. L.base + L.count - 1 (count > 0) into L.out.
+cudaError_t launch_derive(const KeyLaunch& L, uint32_t sms, cudaStream_t st);
 // Field multiplications per second in radix 2^32 (the search kernel's), radix 2^25.5 and
 // radix 2^51 in FP64; *radix51_exact tells whether radix-2^51 chains matched radix 2^32.
 cudaError_t measure_field_mul_rates(int sms, cudaStream_t st, double* radix32_per_s, double* radix26_per_s,
@@ -108,12 +110,11 @@ cudaError_t field_mul_pairs(const uint32_t* a, const uint32_t* b, uint32_t n, ui
 // each 6 products a step and 72 wide products on the limbs).
 constexpr double MADS_MUL_SCHOOLBOOK = 64 + 64 + 16;
 constexpr double MADS_INVERT = 18 * (30 * 6 + 2 * 72);
-// The kernel of a variant and its dynamic shared memory (for graph nodes); sets the
-// kernel's shared-memory limit like launch_keys does.
-cudaError_t keys_kernel(bool derive, bool incr, uint32_t kpt, uint32_t block, uint32_t layout, uint32_t dfa_smem,
-                        uint32_t table_smem, const void** func, size_t* dyn);
-cudaError_t keys_occupancy(bool derive, bool incr, uint32_t kpt, uint32_t block, uint32_t layout, uint32_t table_smem,
-                           int* blocks_per_sm);
+// The search kernel of a variant and its dynamic shared memory (for graph nodes); sets the
+// kernel's shared-memory limit like launch_search does.
+cudaError_t search_kernel(bool incr, uint32_t kpt, uint32_t block, uint32_t layout, uint32_t dfa_smem,
+                          uint32_t table_smem, const void** func, size_t* dyn);
+cudaError_t search_occupancy(uint32_t kpt, uint32_t block, uint32_t layout, uint32_t table_smem, int* blocks_per_sm);
 // multiply-adds per second of the carry-chain row microbenchmark and of plain mad.lo.u32
 cudaError_t measure_mad_peaks(int sms, cudaStream_t st, double* chain_per_s, double* lo_per_s);
 // multiply-adds per second of independent mad.hi.u32, independent mad.wide.u32, and rows of
