@@ -829,7 +829,7 @@ def main():
                          "and inversion amortise over more keys)")
     ap.add_argument("--block", type=int, default=512)
     ap.add_argument("--hash-warps", type=int, default=0, choices=[0, 4],
-                    help="4: search kernel with hashing warps (secure and multi workloads)")
+                    help="4: spans counted in 352 threads per CTA (secure and multi workloads)")
     ap.add_argument("--e2e-steps", type=int, default=0, help="end-to-end steps (default: --steps)")
     ap.add_argument("--workload", choices=sorted(WORKLOADS), default="secure")
     ap.add_argument("--serve-jobs", type=int, default=0, help="serving: number of jobs (default 1000)")

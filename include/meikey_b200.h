@@ -79,9 +79,9 @@ typedef struct mk_options {
     uint32_t blocks_per_sm;   /* resident CTAs per SM the grid is sized for (0 = occupancy maximum) */
     uint32_t self_check;      /* 1: derive keys at creation and compare with the host derivation */
     uint32_t hit_capacity;    /* hit-ring entries per job (0 = 65536) */
-    uint32_t hash_warps;      /* 4: search with hashing warps (block 512, keys per thread 8 or 16): 11 comb
-                                 warps, 1 inverter, 4 warps computing the SHA-512 scalars, so that hashing
-                                 overlaps the comb multiplies; ChaCha20 and counter seeds only.  0: off */
+    uint32_t hash_warps;      /* 4: the span of an iteration counts 352 threads of a CTA (block 512, keys per
+                                 thread 8 or 16); ChaCha20 and counter seeds only.  0: off.  Once a layout
+                                 with hashing warps of its own; every warp hashing is the faster one */
     uint32_t inverter_rotates;/* 0: the span of an iteration counts block - 32 threads of a CTA; 1: all of them.
                                  Who inverts no longer depends on it: with hashed seeds every warp derives
                                  keys and the inversion rotates over the warps, with the incremental source
@@ -99,12 +99,9 @@ typedef struct mk_options {
                                  40+ rows, e.g. 42 rows of 6-bit digits, 133 KB; block 512, keys per thread
                                  4 or 8, the dedicated inverter; regex tables then stay in global memory).
                                  MK_ERR_OUT_OF_RANGE when the table does not fit */
-    uint32_t hash_interleave; /* 1: each thread hashes the next iteration's seeds inside the current
-                                 iteration's comb rows, 8 SHA-512 rounds per row, so that the hashing
-                                 (ALU pipe) issues between the field multiplies (IMAD pipe) of one
-                                 warp; 12 rows, block 512, keys per thread 8 or 16, the dedicated
-                                 inverter, the table in HBM.  ChaCha20 and counter seeds (the
-                                 incremental source hashes nothing) */
+    uint32_t hash_interleave; /* 1 (12 rows, block 512, keys per thread 8 or 16, no other layout option): accepted
+                                 and without effect; once SHA-512 rounds inside the comb rows, which the
+                                 plain order of hashing first beats */
 } mk_options;
 
 /* One pattern as the reference's GPU needle (Needle, src/service/gpu.rs:618-660):

@@ -40,8 +40,8 @@ struct mk_ctx {
     uint4* incr = nullptr;           // incremental source: window table then step table
     uint32_t delta[24] = {};         // keys_per_iter·B (table form)
     uint32_t kpt = 8, block = 256, grid = 0;
-    uint32_t hash_warps = 0;  // 4: search kernel with hashing warps (ChaCha20 / counter seeds)
-    uint32_t layout = mkb::LAYOUT_INVERTER_WARP;  // division of work inside a search CTA
+    uint32_t hash_warps = 0;  // 4: hashed seed sources only
+    uint32_t layout = mkb::LAYOUT_INVERTER_WARP;  // which threads an iteration's span counts
     uint32_t inv_batch = 0;   // keys per field inversion asked for (0: 32 inversions per CTA and iteration)
     uint32_t table_smem = 0;  // bytes of the comb table each search CTA keeps in shared memory (0: HBM)
     uint32_t hit_capacity = 1u << 16;
@@ -268,8 +268,8 @@ int mk_ctx_create(int device, const mk_options* options, mk_ctx** out) try {
     const bool smem_ok = o.table_in_smem == 0 ||
                          (o.table_in_smem == 1 && o.block == 512 && (o.keys_per_thread == 4 || o.keys_per_thread == 8) &&
                           !o.hash_warps && !o.inverter_rotates);
-    // hashing inside the comb rows: 12 rows (10 full rows carry the 80 rounds), block 512, 8 or 16
-    // keys per thread, the dedicated inverter, the table in HBM
+    // accepted as it always was, without effect: 12 rows, block 512, 8 or 16 keys per thread, no other
+    // layout option
     const bool shai_ok = o.hash_interleave == 0 ||
                          (o.hash_interleave == 1 && o.table_rows == 12 && o.block == 512 &&
                           (o.keys_per_thread == 8 || o.keys_per_thread == 16) && !o.hash_warps &&
@@ -283,7 +283,6 @@ int mk_ctx_create(int device, const mk_options* options, mk_ctx** out) try {
     // the pools a divisor of the compute threads and at most 32 (one per lane of the inverting warp)
     const uint32_t layout = o.hash_warps         ? mkb::LAYOUT_HASH_WARPS
                             : o.inverter_rotates ? mkb::LAYOUT_ROTATING
-                            : o.hash_interleave  ? mkb::LAYOUT_INTERLEAVED
                                                  : mkb::LAYOUT_INVERTER_WARP;
     const uint32_t ct = mkb::search_threads(o.block, layout);
     uint32_t pools = 32;
@@ -329,7 +328,7 @@ int mk_ctx_create(int device, const mk_options* options, mk_ctx** out) try {
         c->table_smem = (uint32_t)bytes;
     }
     int occ = 0;
-    cudaError_t oe = mkb::search_occupancy(c->kpt, c->block, c->layout, c->table_smem, &occ);
+    cudaError_t oe = mkb::search_occupancy(c->kpt, c->block, c->table_smem, &occ);
     if (oe != cudaSuccess && c->table_smem) {
         cudaGetLastError();
         return fail(c, MK_ERR_OUT_OF_RANGE, "the comb table and the CTA's buffers do not fit in shared memory");
@@ -370,7 +369,7 @@ int mk_ctx_create(int device, const mk_options* options, mk_ctx** out) try {
             return fail(c, MK_ERR_OUT_OF_MEMORY, "incremental table allocation failed");
         }
         MK_CUDA(c, cudaMemcpy(c->incr, words.data(), words.size() * 4, cudaMemcpyHostToDevice));
-        mkh25519::niels_of_multiple((uint64_t)c->grid * mkb::search_kernel_threads(true, c->block, c->layout, 0) * c->kpt,
+        mkh25519::niels_of_multiple((uint64_t)c->grid * mkb::search_kernel_threads(true, c->block, 0) * c->kpt,
                                     c->delta);
     }
     // info
@@ -382,8 +381,7 @@ int mk_ctx_create(int device, const mk_options* options, mk_ctx** out) try {
     in.keys_per_thread = c->kpt;
     in.table_rows = c->geom.rows;
     in.table_bytes = bytes;
-    // the threads of a search CTA that derive keys (all but a dedicated inverter warp, unless the
-    // inversion rotates; 352 comb threads with hashing warps)
+    // the span of an iteration counts all threads of a CTA but the last warp, all of them, or 352
     in.keys_per_iter = (uint64_t)c->grid * mkb::search_threads(c->block, c->layout) * c->kpt;
     in.inversion_batch = mkb::search_threads(c->block, c->layout) * c->kpt / pools;
     in.table_in_smem = c->table_smem ? 1 : 0;
@@ -744,8 +742,7 @@ void mk_job_destroy(mk_job* j) try {
 
 // Shared memory for the job's DFA tables when they fit (the kernel then reads them there).
 static uint32_t dfa_smem_bytes(const mk_job* j) {
-    if (j->ctx->hash_warps) return 0;  // the hashing-warp kernel's scalar ring takes that shared memory
-    if (j->ctx->table_smem) return 0;  // so does a comb table kept in shared memory
+    if (j->ctx->table_smem) return 0;  // a comb table kept in shared memory takes that room
     uint64_t total = 0;
     for (const auto& h : j->needles)
         if (h.mode == MK_MODE_REGEX) total += ((uint64_t)h.len * 130 + 15) & ~15ull;
@@ -756,8 +753,8 @@ static uint32_t dfa_smem_bytes(const mk_job* j) {
 // source: the pools whose batches come nearest to the keys per inversion asked for.
 static uint32_t search_pools(const mk_ctx* c, bool incr) {
     if (!c->inv_batch) return 32;
-    const uint32_t keys = mkb::search_kernel_threads(incr, c->block, c->layout, c->table_smem) *
-                          mkb::search_kernel_keys(incr, c->kpt, c->layout, c->table_smem);
+    const uint32_t keys = mkb::search_kernel_threads(incr, c->block, c->table_smem) *
+                          mkb::search_kernel_keys(incr, c->kpt, c->table_smem);
     return std::min(32u, std::max(1u, (keys + c->inv_batch / 2) / c->inv_batch));
 }
 
@@ -772,7 +769,7 @@ static mkb::KeyLaunch search_params(const mk_job* j, uint64_t base, uint32_t ite
     L.seed_src = (uint32_t)j->source;
     L.iters = iters;
     const bool incr = j->source == MK_SEED_INCREMENTAL;
-    L.chunks = c->info.keys_per_iter / mkb::search_kernel_keys(incr, c->kpt, c->layout, c->table_smem) * iters;
+    L.chunks = c->info.keys_per_iter / mkb::search_kernel_keys(incr, c->kpt, c->table_smem) * iters;
     L.base = base;
     L.match = j->d_match;
     L.hits = j->d_hits;
@@ -782,7 +779,6 @@ static mkb::KeyLaunch search_params(const mk_job* j, uint64_t base, uint32_t ite
     L.sink = j->d_sink;
     if (incr) set_incremental(c, j->key, base, L);
     L.dfa_smem = dfa_smem_bytes(j);
-    L.layout = c->layout;
     L.inv_pools = search_pools(c, incr);
     L.table_smem = c->table_smem;
     return L;
@@ -993,8 +989,8 @@ int mk_ctx_work_per_key(const mk_ctx* c, int seed_source, double* field_muls, do
     // (fold by 38).
     const double MUL = mkb::MADS_MUL_SCHOOLBOOK;
     const bool incr = seed_source == MK_SEED_INCREMENTAL;
-    const double kpt = mkb::search_kernel_keys(incr, c->kpt, c->layout, c->table_smem), rows = c->geom.rows;
-    const double ct = mkb::search_kernel_threads(incr, c->block, c->layout, c->table_smem);
+    const double kpt = mkb::search_kernel_keys(incr, c->kpt, c->table_smem), rows = c->geom.rows;
+    const double ct = mkb::search_kernel_threads(incr, c->block, c->table_smem);
     // comb: row 0 is free, full additions cost 7 multiplications, the last one 3
     double comb = 7.0 * (rows - 2) + 3.0;
     // Montgomery batch inside a thread: a_j and the running product (2 each for j > 0),
@@ -1068,7 +1064,7 @@ int mk_job_graph_create(mk_job* j, uint32_t iters, uint32_t launches, mk_graph**
     if (e != cudaSuccess) return bail(e, "cudaGraphAddMemsetNode");
     const void* func = nullptr;
     size_t dyn = 0;
-    e = mkb::search_kernel(j->source == MK_SEED_INCREMENTAL, c->kpt, c->block, c->layout, dfa_smem_bytes(j),
+    e = mkb::search_kernel(j->source == MK_SEED_INCREMENTAL, c->kpt, c->block, dfa_smem_bytes(j),
                          c->table_smem, &func, &dyn);
     if (e != cudaSuccess) return bail(e, "search_kernel");
     for (uint32_t i = 0; i < launches; i++) {
@@ -1098,7 +1094,7 @@ static int graph_enqueue(mk_graph* g, uint64_t base) {
     mk_ctx* c = j->ctx;
     MK_CUDA(c, cudaSetDevice(c->device));
     // the job's needles may have changed since the graph was made: size the DFA staging anew
-    MK_CUDA(c, mkb::search_kernel(j->source == MK_SEED_INCREMENTAL, c->kpt, c->block, c->layout, dfa_smem_bytes(j),
+    MK_CUDA(c, mkb::search_kernel(j->source == MK_SEED_INCREMENTAL, c->kpt, c->block, dfa_smem_bytes(j),
                                 c->table_smem, &g->func,
                                 &g->dyn));
     for (size_t i = 0; i < g->nodes.size(); i++) {

@@ -188,49 +188,4 @@ __device__ __forceinline__ void counter_scalar(const CounterMid& m, u64 index, u
     sha512_scalar_from<3>(m.st, w4, s_out);
 }
 
-// SHA-512 of one padded 32-byte message advanced 8 rounds at a time with the same code for
-// every step, so that a caller can interleave the steps with other work (the search kernel
-// puts one step into each comb row).  The ring w[0..15] holds W[t0-16 .. t0-1] before the step
-// of rounds t0..t0+7, t0 >= 16 (the first two steps take the message words, which start in
-// the ring); each step writes W[t0..t0+7] into w[0..7] and swaps the halves.
-struct ShaRun {
-    u64 s[8];
-    u64 w[16];
-};
-
-__device__ __forceinline__ void sha_run_start(ShaRun& r, const u64 w4[4]) {
-    r.s[0] = MKH_IV0; r.s[1] = MKH_IV1; r.s[2] = MKH_IV2; r.s[3] = MKH_IV3;
-    r.s[4] = MKH_IV4; r.s[5] = MKH_IV5; r.s[6] = MKH_IV6; r.s[7] = MKH_IV7;
-#pragma unroll
-    for (int i = 0; i < 4; i++) r.w[i] = w4[i];
-    r.w[4] = 0x8000000000000000ull;
-#pragma unroll
-    for (int i = 5; i < 15; i++) r.w[i] = 0;
-    r.w[15] = 256;
-}
-
-// rounds t0..t0+7 (t0 = 0, 8, ..., 72)
-__device__ __forceinline__ void sha_run_step(ShaRun& r, u32 t0) {
-    const bool sched = t0 >= 16;
-    u64 a = r.s[0], b = r.s[1], c = r.s[2], d = r.s[3], e = r.s[4], f = r.s[5], g = r.s[6], h = r.s[7];
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const u64 x2 = i < 2 ? r.w[i + 14] : r.w[i - 2];   // W[t-2]
-        const u64 x7 = i < 7 ? r.w[i + 9] : r.w[0];        // W[t-7]
-        const u64 x15 = r.w[i + 1];                         // W[t-15]
-        const u64 s0 = rotr64(x15, 1) ^ rotr64(x15, 8) ^ (x15 >> 7);
-        const u64 s1 = rotr64(x2, 19) ^ rotr64(x2, 61) ^ (x2 >> 6);
-        const u64 wt = sched ? r.w[i] + s0 + x7 + s1 : r.w[i];
-        r.w[i] = wt;
-        sha512_round(a, b, c, d, e, f, g, h, wt, SHA512_K[t0 + i]);
-    }
-    r.s[0] = a; r.s[1] = b; r.s[2] = c; r.s[3] = d; r.s[4] = e; r.s[5] = f; r.s[6] = g; r.s[7] = h;
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const u64 t = r.w[i];
-        r.w[i] = r.w[i + 8];
-        r.w[i + 8] = t;
-    }
-}
-
 }  // namespace mkh

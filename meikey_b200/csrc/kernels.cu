@@ -214,34 +214,6 @@ __device__ __forceinline__ void comb_mul(const uint4* __restrict__ table, const 
     mk32::ge_add_niels_frac(P, read_entry(slot, (rows - 1) & 1), yn, yd, xn, xd);
 }
 
-// comb_mul with one 8-round step of the SHA-512 `run` (the next iteration's seed) in every
-// full-addition row, in the same straight-line block as the row's field multiplies, so that
-// the hashing (ALU pipe) issues between the multiplies (IMAD pipe).  Built for 12 rows: the
-// 10 full rows carry the 80 rounds.  y = yn/yd only.
-__device__ __forceinline__ void comb_mul_sha(const uint4* __restrict__ table, const CombGeom& g, const u64 s[4],
-                                             EntrySlot& slot, fe& yn, fe& yd, mkh::ShaRun& run) {
-    Digits dg = digits_of(s);
-    const u32 rows = g.rows;
-    auto fetch = [&](u32 row) {
-        const int d = next_digit(dg, g.width[row], row + 1 == rows);
-        fetch_entry(slot, row & 1, table, entry_index(g, row, d), d < 0);
-    };
-    fetch(0);
-    fetch(1);
-    wait_entries<1>();
-    ge P = comb_row0(read_entry(slot, 0));
-#pragma unroll 1
-    for (u32 row = 1; row + 1 < rows; row++) {
-        fetch(row + 1);
-        wait_entries<1>();
-        const niels n = read_entry(slot, row & 1);
-        mkh::sha_run_step(run, 8u * (row - 1));
-        P = mk32::ge_add_niels(P, n);
-    }
-    wait_entries<0>();
-    mk32::ge_add_niels_frac(P, read_entry(slot, (rows - 1) & 1), yn, yd, nullptr, nullptr);
-}
-
 // 6-bit values of the 44-character base64 tail of the key blob (0x20 then the key),
 // from the key's 8 little-endian words; only positions 1..43 are searched.
 __device__ __forceinline__ u32 tail_value(const u32 pk[8], int pos) {
@@ -468,57 +440,6 @@ __device__ __forceinline__ void combs(const KeyLaunch& L, const CombGeom& g, con
     b.prod = run;
 }
 
-// Comb multiplies of this iteration's KPT scalars (sc) with the SHA-512 of the next
-// iteration's seeds (indices next_first + j) carried through their rows: key j's comb reads
-// sc[j] at its start and leaves the next iteration's scalar of key j there.  ChaCha20 blocks
-// serve an even index and the next odd one (the other half is kept).
-template <int KPT>
-__device__ __forceinline__ void combs_sha(const KeyLaunch& L, const CombGeom& g, u64 sc[KPT][4], EntrySlot& slot,
-                                          Batch<KPT>& b, const u32 key[8], const mkh::CounterMid& mid,
-                                          u64 next_first) {
-    fe run;
-    u32 other[8];
-    u64 other_id = ~0ull;
-#pragma unroll 1
-    for (int j = 0; j < KPT; j++) {
-        const u64 idx = next_first + (u64)j;
-        u64 w4[4];
-        if (L.seed_src == 1) {
-            mkh::counter_words(mid, idx, w4);
-        } else {
-            u32 sw[8];
-            if ((idx >> 1) == other_id) {
-#pragma unroll
-                for (int i = 0; i < 8; i++) sw[i] = other[i];
-            } else {
-                u32 blk[16];
-                mkh::chacha20_block(key, idx >> 1, blk);
-                const bool odd = idx & 1;
-#pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    sw[i] = odd ? blk[8 + i] : blk[i];
-                    other[i] = odd ? blk[i] : blk[8 + i];
-                }
-                other_id = idx >> 1;
-            }
-            mkh::seed_words(sw, w4);
-        }
-        mkh::ShaRun shr;
-        mkh::sha_run_start(shr, w4);
-        fe num;
-        comb_mul_sha(L.table, g, sc[j], slot, num, b.den[j], shr);
-        mkh::digest_scalar(shr.s[0], shr.s[1], shr.s[2], shr.s[3], sc[j]);
-        if (j == 0) {
-            b.a[0] = num;
-            run = b.den[0];
-        } else {
-            b.a[j] = mk32::fe_mul(num, run);
-            run = mk32::fe_mul(run, b.den[j]);
-        }
-    }
-    b.prod = run;
-}
-
 // The key (0 .. KPT-1) in slot s of an incremental batch.
 template <int KPT>
 __device__ __forceinline__ int incr_key(int s) {
@@ -706,9 +627,7 @@ __device__ __forceinline__ void incr_fracs(const ge& Q, const uint4* steps, Batc
 // keys_per_iter·B (one mixed addition) per iteration.  No comb table is read.
 // STAB: the comb table lives in shared memory (copied by every CTA at the start, in place of
 // the staging slots; tables of a few hundred to a few thousand entries, 40+ rows).
-// SHAI: the SHA-512 of iteration it+1's seeds runs inside iteration it's comb rows (12 rows;
-// the first iteration's scalars are hashed up front).
-template <int KPT, int BLOCK, bool INCR, bool ROT, bool STAB = false, bool SHAI = false>
+template <int KPT, int BLOCK, bool INCR, bool ROT, bool STAB = false>
 __global__ void __launch_bounds__(BLOCK, 512 / BLOCK) k_search(const KeyLaunch L) {
     constexpr int CT = ROT ? BLOCK : BLOCK - 32;  // compute threads
     constexpr int CW = CT / 32;                   // compute warps
@@ -817,9 +736,6 @@ __global__ void __launch_bounds__(BLOCK, 512 / BLOCK) k_search(const KeyLaunch L
             } else if (INCR) {
                 incr_fracs<KPT>(Q, steps, batch[b]);
                 Q = mk32::ge_add_niels(Q, words_niels(L.delta));
-            } else if (SHAI) {
-                if (it == 0) scalars<KPT>(L, key, mid, first_of(0), sc);
-                combs_sha<KPT>(L, g, sc, slot, batch[b], key, mid, first_of(it + 1));
             } else {
                 scalars<KPT>(L, key, mid, first_of(it), sc);
                 combs<KPT, STAB>(L, g, sc, slot, stab, batch[b]);
@@ -848,178 +764,6 @@ __global__ void __launch_bounds__(BLOCK, 512 / BLOCK) k_search(const KeyLaunch L
     // the decision of the iteration that ended the loop is visible here (its inverses were waited for)
     if (ROT && tid == 0 && stop_iter < iters) atomicOr(&L.job->status, 1u);
     if (L.sink) L.sink[(u64)blockIdx.x * CT + tid] = sink;
-}
-
-// Search kernel with hashing warps (ChaCha20 / counter seeds).  Warps 0..10 run the comb
-// multiplies, warp 11 inverts, warps 12..15 (one per SM sub-partition) compute the seeds'
-// SHA-512 scalars: hashing is ALU work and the comb is IMAD work, so the two pipes overlap
-// instead of the compute warps alternating between them.  The index layout and results are
-// those of k_search; only the division of work inside a CTA differs.
-//
-// Scalars go from the hashing warps to the comb warps through a two-slot shared ring of
-// chunks (4 keys of every comb thread per chunk).  Named barriers:
-//   1+b / 3+b  products / inverses of pipeline buffer b (comb warps and the inverter, 384)
-//   5+s / 7+s  ring slot s full / empty (hashing and comb warps, 480)
-//   9+(it&1)   the inverter's stop decision after iteration it (inverter and hashing warps, 160)
-// Whether iteration X is computed is decided, by every role, from the stop word as it stands
-// after the inverter's decision of iteration X-2; the inverter arrives on a decision barrier
-// only when the hashing warps will wait on it, and the hashing warps drain the last two ring
-// releases before they return, so no barrier phase is left open (model-checked in
-// tests/test_pipeline_protocol.py).
-template <int KPT, int BLOCK>
-__global__ void __launch_bounds__(BLOCK, 1) k_search_hw(const KeyLaunch L) {
-    static_assert(BLOCK == 512 && KPT % 4 == 0 && KPT >= 8, "layout of 11 comb, 1 inverter, 4 hashing warps");
-    constexpr int CW = 11, CT = CW * 32;     // comb warps / threads
-    constexpr int INV_WARP = 11;
-    constexpr int HT = 128;                  // hashing threads
-    constexpr int CPI = KPT / 4;             // ring chunks per iteration
-    constexpr int PAIRS = CT * 2;            // index pairs per chunk
-    constexpr int B_PIPE = CT + 32, B_RING = CT + HT, B_STOP = 32 + HT;
-    extern __shared__ uint4 dyn_smem[];
-    fe (*prod)[CT] = reinterpret_cast<fe (*)[CT]>(dyn_smem);
-    fe (*scratch)[CT] = prod + 2;
-    EntrySlot* slots = reinterpret_cast<EntrySlot*>(scratch + 2);
-    u64 (*ring)[4][CT][4] = reinterpret_cast<u64 (*)[4][CT][4]>(slots + CT);  // [slot][key][thread][word]
-    __shared__ CombGeom g;
-    __shared__ MatchSet ms;
-    __shared__ u32 lane_masks[64 * 32];  // see match_key
-    __shared__ u32 key[8];
-    __shared__ mkh::CounterMid mid;
-    __shared__ volatile u32 stop_iter;
-    const u32 tid = threadIdx.x;
-    const u32 warp = tid >> 5;
-    {
-        const u32* src = (const u32*)&L.geom;
-        u32* dst = (u32*)&g;
-        for (u32 i = tid; i < sizeof(CombGeom) / 4; i += BLOCK) dst[i] = src[i];
-        const u32* s2 = (const u32*)L.match;
-        u32* d2 = (u32*)&ms;
-        for (u32 i = tid; i < sizeof(MatchSet) / 4; i += BLOCK) d2[i] = s2[i];
-        if (tid < 8) key[tid] = L.key[tid];
-        if (tid == 0) stop_iter = L.iters;
-    }
-    __syncthreads();
-    if (ms.narrow)
-        for (u32 i = tid; i < 64u * 32u; i += BLOCK) lane_masks[i] = (u32)ms.mask[0][i >> 5];
-    if (tid == 0 && L.seed_src == 1) mid = mkh::counter_mid(key);
-    __syncthreads();
-    const u32 iters = L.iters;
-    if (iters == 0) return;
-    const u64 nthreads = (u64)gridDim.x * CT;
-    auto first_of = [&](u32 it, u64 gid) { return L.base + ((u64)it * nthreads + gid) * KPT; };
-    const int pools = (int)L.inv_pools;  // 1..32
-
-    if (warp > (u32)INV_WARP) {
-        // ---- hashing warps ----
-        const u32 p = tid - (INV_WARP + 1) * 32;
-        u32 X = 0;
-        for (;; X++) {
-            if (X >= iters) break;
-            if (X >= 2) {
-                bar_sync(9 + (X & 1), B_STOP);
-                if (X >= stop_iter) break;
-            }
-#pragma unroll 1
-            for (u32 c = 0; c < (u32)CPI; c++) {
-                const u32 gc = X * CPI + c, slot = gc & 1;
-                if (gc >= 2) bar_sync(7 + slot, B_RING);
-#pragma unroll 1
-                for (u32 v = p; v < (u32)PAIRS; v += HT) {
-                    const u32 t = v >> 1, k0 = (v & 1) * 2;
-                    const u64 idx = first_of(X, (u64)blockIdx.x * CT + t) + c * 4 + k0;
-                    u32 blk[16];
-                    u64 blk_id = ~0ull;
-#pragma unroll 1
-                    for (u32 q = 0; q < 2; q++) {
-                        u64 sc[4];
-                        scalar_of(L.seed_src, key, mid, idx + q, blk, blk_id, sc);
-                        uint4* d = reinterpret_cast<uint4*>(ring[slot][k0 + q][t]);
-                        d[0] = make_uint4((u32)sc[0], (u32)(sc[0] >> 32), (u32)sc[1], (u32)(sc[1] >> 32));
-                        d[1] = make_uint4((u32)sc[2], (u32)(sc[2] >> 32), (u32)sc[3], (u32)(sc[3] >> 32));
-                    }
-                }
-                bar_arrive(5 + slot, B_RING);
-            }
-        }
-        // the comb warps release every chunk they take: wait for the last two releases
-        const u32 G = X * CPI;
-        bar_sync(7 + ((G - 2) & 1), B_RING);
-        bar_sync(7 + ((G - 1) & 1), B_RING);
-        return;
-    }
-
-    if (warp == (u32)INV_WARP) {
-        // ---- inverter warp ----
-        for (u32 it = 0;; it++) {
-            const int b = it & 1;
-            bar_sync(1 + b, B_PIPE);
-            if ((tid & 31) == 0) {
-                const volatile JobDevice* jd = L.job;
-                if (jd->stop != 0 || (L.stop_on_hit && jd->hit_count != 0)) {
-                    u32 s = it + 2;
-                    if (s < stop_iter) stop_iter = s;
-                }
-            }
-            __syncwarp();
-            const bool more = it + 1 < iters && it + 1 < stop_iter;
-            // the hashing warps wait on this decision only when they will consider iteration it+2
-            if (it + 2 < iters && more) bar_arrive(9 + (it & 1), B_STOP);
-            invert_pools(prod[b], scratch[b], CT, pools);
-            __syncwarp();
-            bar_arrive(3 + b, B_PIPE);
-            if (!more) break;
-        }
-        if ((tid & 31) == 0 && stop_iter < iters) atomicOr(&L.job->status, 1u);
-        return;
-    }
-
-    // ---- comb warps ----
-    const u64 gid = (u64)blockIdx.x * CT + tid;
-    EntrySlot& slot = slots[tid];
-    Batch<KPT> batch[2];
-    u32 sink = 0;
-    auto produce = [&](u32 it) {
-        const int b = it & 1;
-        Batch<KPT>& bt = batch[b];
-        fe run;
-#pragma unroll 1
-        for (int j = 0; j < KPT; j++) {
-            const u32 gc = it * CPI + (u32)(j >> 2), rs = gc & 1;
-            if ((j & 3) == 0) bar_sync(5 + rs, B_RING);
-            u64 sc[4];
-            {
-                const uint4* q = reinterpret_cast<const uint4*>(ring[rs][j & 3][tid]);
-                const uint4 a = q[0], c = q[1];
-                sc[0] = (u64)a.y << 32 | a.x;
-                sc[1] = (u64)a.w << 32 | a.z;
-                sc[2] = (u64)c.y << 32 | c.x;
-                sc[3] = (u64)c.w << 32 | c.z;
-            }
-            if ((j & 3) == 3) bar_arrive(7 + rs, B_RING);
-            fe num;
-            comb_mul(L.table, g, sc, slot, num, bt.den[j], nullptr, nullptr);
-            if (j == 0) {
-                bt.a[0] = num;
-                run = bt.den[0];
-            } else {
-                bt.a[j] = mk32::fe_mul(num, run);
-                run = mk32::fe_mul(run, bt.den[j]);
-            }
-        }
-        bt.prod = run;
-        prod[b][tid] = bt.prod;
-        bar_arrive(1 + b, B_PIPE);
-    };
-    produce(0);
-    for (u32 it = 0;; it++) {
-        const int b = it & 1;
-        if (it + 1 < iters && it + 1 < stop_iter) produce(it + 1);
-        bar_sync(3 + b, B_PIPE);
-        backward<KPT, false>(L, ms, ms.narrow ? lane_masks : nullptr, first_of(it, gid), true, batch[b],
-                                        prod[b][tid], sink);
-        if (it + 1 >= iters || it + 1 >= stop_iter) break;
-    }
-    if (L.sink) L.sink[gid] = sink;
 }
 
 constexpr int DERIVE_BLOCK = 128;
@@ -1111,22 +855,10 @@ __global__ void __launch_bounds__(DERIVE_BLOCK, 512 / DERIVE_BLOCK) k_derive(con
 
 // dynamic shared memory of a search: products and inversion scratch (two buffers each) and the
 // per-thread table staging slots (the incremental source reads no comb table and needs none)
-static size_t dyn_bytes(bool incr, uint32_t block, uint32_t layout, uint32_t table_smem) {
-    const size_t fe_bytes = 32;
-    if (layout == LAYOUT_HASH_WARPS && !incr) {  // k_search_hw: 352 comb threads, plus the two-slot scalar ring
-        const size_t ct = 352;
-        return 4 * ct * fe_bytes + ct * sizeof(EntrySlot) + 2 * 4 * ct * 32;
-    }
-    const size_t threads = search_kernel_threads(incr, block, layout, table_smem);
+static size_t dyn_bytes(bool incr, uint32_t block, uint32_t table_smem) {
+    const size_t fe_bytes = 32, threads = search_kernel_threads(incr, block, table_smem);
     if (table_smem && !incr) return 4 * threads * fe_bytes + table_smem;  // the table in place of the slots
     return 4 * threads * fe_bytes + (incr ? 0 : threads * sizeof(EntrySlot));
-}
-
-static const void* hw_kernel_of(uint32_t kpt, uint32_t block) {
-    if (block != 512) return nullptr;
-    if (kpt == 8) return (const void*)k_search_hw<8, 512>;
-    if (kpt == 16) return (const void*)k_search_hw<16, 512>;
-    return nullptr;
 }
 
 // search kernels with the comb table in shared memory: the dedicated-inverter layout, block
@@ -1154,31 +886,19 @@ static cudaError_t prepare(const void* f, size_t dyn) {
     return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
 }
 
-// search kernels with the SHA-512 interleaved into the comb rows: the dedicated-inverter layout,
-// block 512, keys per thread 8 and 16
-static const void* shai_kernel_of(uint32_t kpt, uint32_t block) {
-    if (block != 512) return nullptr;
-    if (kpt == 8) return (const void*)k_search<8, 512, false, false, false, true>;
-    if (kpt == 16) return (const void*)k_search<16, 512, false, false, false, true>;
-    return nullptr;
-}
-
 // the search kernel of a variant (the table-in-shared-memory search when table_smem > 0)
-static const void* variant_kernel(bool incr, uint32_t kpt, uint32_t block, uint32_t layout, uint32_t table_smem) {
-    if (layout == LAYOUT_INTERLEAVED && !incr) return table_smem ? nullptr : shai_kernel_of(kpt, block);
-    if (table_smem && !incr) return layout == LAYOUT_INVERTER_WARP ? stab_kernel_of(kpt, block) : nullptr;
-    return layout == LAYOUT_HASH_WARPS && !incr ? hw_kernel_of(kpt, block) : kernel_of(incr, kpt, block);
+static const void* variant_kernel(bool incr, uint32_t kpt, uint32_t block, uint32_t table_smem) {
+    return table_smem && !incr ? stab_kernel_of(kpt, block) : kernel_of(incr, kpt, block);
 }
 
-cudaError_t search_kernel(bool incr, uint32_t kpt, uint32_t block, uint32_t layout, uint32_t dfa_smem,
-                          uint32_t table_smem, const void** func, size_t* dyn) {
-    const bool hw = layout == LAYOUT_HASH_WARPS && !incr;
+cudaError_t search_kernel(bool incr, uint32_t kpt, uint32_t block, uint32_t dfa_smem, uint32_t table_smem,
+                          const void** func, size_t* dyn) {
     const uint32_t tsm = incr ? 0 : table_smem;
-    const void* f = variant_kernel(incr, kpt, block, layout, tsm);
-    // the hashing-warp kernel's scalar ring and a comb table take the shared memory of DFA tables
-    if (!f || dfa_smem > DFA_SMEM_MAX || ((hw || tsm) && dfa_smem)) return cudaErrorInvalidValue;
+    const void* f = variant_kernel(incr, kpt, block, tsm);
+    // a comb table takes the shared memory of DFA tables
+    if (!f || dfa_smem > DFA_SMEM_MAX || (tsm && dfa_smem)) return cudaErrorInvalidValue;
     *func = f;
-    *dyn = dyn_bytes(incr, block, layout, tsm) + dfa_smem;
+    *dyn = dyn_bytes(incr, block, tsm) + dfa_smem;
     return prepare(f, *dyn);
 }
 
@@ -1187,16 +907,16 @@ cudaError_t launch_search(const KeyLaunch& L, uint32_t kpt, uint32_t block, uint
     if (incr && (kpt > (uint32_t)INCR_STEPS || !L.incr)) return cudaErrorInvalidValue;
     const void* f = nullptr;
     size_t dyn = 0;
-    cudaError_t e = search_kernel(incr, kpt, block, L.layout, L.dfa_smem, L.table_smem, &f, &dyn);
+    cudaError_t e = search_kernel(incr, kpt, block, L.dfa_smem, L.table_smem, &f, &dyn);
     if (e != cudaSuccess) return e;
     void* args[] = {const_cast<KeyLaunch*>(&L)};
     return cudaLaunchKernel(f, dim3(grid), dim3(block), args, dyn, st);
 }
 
-cudaError_t search_occupancy(uint32_t kpt, uint32_t block, uint32_t layout, uint32_t table_smem, int* blocks_per_sm) {
+cudaError_t search_occupancy(uint32_t kpt, uint32_t block, uint32_t table_smem, int* blocks_per_sm) {
     const void* f = nullptr;
     size_t dyn = 0;
-    cudaError_t e = search_kernel(false, kpt, block, layout, 0, table_smem, &f, &dyn);
+    cudaError_t e = search_kernel(false, kpt, block, 0, table_smem, &f, &dyn);
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, f, (int)block, dyn);
 }

@@ -38,8 +38,6 @@ struct KeyLaunch {
     // bytes of shared memory for the job's DFA tables (each 16-byte aligned; 0: read them
     // from global memory)
     uint32_t dfa_smem;
-    // division of work inside a search CTA (LAYOUT_*)
-    uint32_t layout;
     // field inversions per CTA and iteration of a search, 1..32 (one per lane of the inverting
     // warp): each pools the products of every inv_pools-th compute thread
     uint32_t inv_pools;
@@ -48,13 +46,14 @@ struct KeyLaunch {
     uint32_t table_smem;
 };
 
-// LAYOUT_INVERTER_WARP, LAYOUT_ROTATING: the span of an iteration counts a CTA's threads without
-// or with the last warp; both run the same kernels (hashed seeds: every warp computes keys and the
-// inversion rotates over them; incremental source: the last warp inverts).  LAYOUT_INTERLEAVED: the
-// last warp inverts, and each iteration's SHA-512 of the next iteration's seeds runs inside the
-// comb rows (12 rows); LAYOUT_HASH_WARPS: 11 comb warps, 1 inverter, 4 hashing warps
-// (k_search_hw; ChaCha20 / counter seeds)
-constexpr uint32_t LAYOUT_INVERTER_WARP = 0, LAYOUT_ROTATING = 1, LAYOUT_INTERLEAVED = 2, LAYOUT_HASH_WARPS = 4;
+// How many threads of a search CTA the span of one iteration counts: all but the last warp, all
+// (LAYOUT_ROTATING), or 352 (LAYOUT_HASH_WARPS, hashed seeds only).  The kernels are the same:
+// hashed seeds rotate the inversion over every warp, the incremental source and comb tables in
+// shared memory leave it to the last one.  (Warps that only hash beside comb warps, 0.877 G keys/s
+// on B200 and 0.908 with all 16 other warps at the comb, and SHA-512 rounds inside the comb rows,
+// 0.69, lose to hashing in every warp, 0.926: operations of the ALU and of the multiply pipe from
+// different warps compete for register reads instead of overlapping.)
+constexpr uint32_t LAYOUT_INVERTER_WARP = 0, LAYOUT_ROTATING = 1, LAYOUT_HASH_WARPS = 4;
 
 // threads of a search CTA that the span of one iteration counts
 inline uint32_t search_threads(uint32_t block, uint32_t layout) {
@@ -64,16 +63,12 @@ inline uint32_t search_threads(uint32_t block, uint32_t layout) {
 // keys per thread and iteration of the hashed-seed search kernel
 constexpr uint32_t HASHED_KEYS = 8;
 
-inline bool search_rotates(bool incr, uint32_t layout, uint32_t table_smem) {
-    return !incr && !table_smem && (layout == LAYOUT_INVERTER_WARP || layout == LAYOUT_ROTATING);
-}
 // keys per thread and iteration, and compute threads per CTA, of the kernel that serves a search
-inline uint32_t search_kernel_keys(bool incr, uint32_t kpt, uint32_t layout, uint32_t table_smem) {
-    return search_rotates(incr, layout, table_smem) ? HASHED_KEYS : kpt;
+inline uint32_t search_kernel_keys(bool incr, uint32_t kpt, uint32_t table_smem) {
+    return incr || table_smem ? kpt : HASHED_KEYS;
 }
-inline uint32_t search_kernel_threads(bool incr, uint32_t block, uint32_t layout, uint32_t table_smem) {
-    if (layout == LAYOUT_HASH_WARPS && !incr) return 352u;
-    return search_rotates(incr, layout, table_smem) ? block : block - 32u;
+inline uint32_t search_kernel_threads(bool incr, uint32_t block, uint32_t table_smem) {
+    return incr || table_smem ? block - 32u : block;
 }
 
 constexpr uint32_t DFA_SMEM_MAX = 48u * 1024u;
@@ -112,9 +107,9 @@ constexpr double MADS_MUL_SCHOOLBOOK = 64 + 64 + 16;
 constexpr double MADS_INVERT = 18 * (30 * 6 + 2 * 72);
 // The search kernel of a variant and its dynamic shared memory (for graph nodes); sets the
 // kernel's shared-memory limit like launch_search does.
-cudaError_t search_kernel(bool incr, uint32_t kpt, uint32_t block, uint32_t layout, uint32_t dfa_smem,
-                          uint32_t table_smem, const void** func, size_t* dyn);
-cudaError_t search_occupancy(uint32_t kpt, uint32_t block, uint32_t layout, uint32_t table_smem, int* blocks_per_sm);
+cudaError_t search_kernel(bool incr, uint32_t kpt, uint32_t block, uint32_t dfa_smem, uint32_t table_smem,
+                          const void** func, size_t* dyn);
+cudaError_t search_occupancy(uint32_t kpt, uint32_t block, uint32_t table_smem, int* blocks_per_sm);
 // multiply-adds per second of the carry-chain row microbenchmark and of plain mad.lo.u32
 cudaError_t measure_mad_peaks(int sms, cudaStream_t st, double* chain_per_s, double* lo_per_s);
 // multiply-adds per second of independent mad.hi.u32, independent mad.wide.u32, and rows of
