@@ -423,6 +423,29 @@ static int check_source(mk_ctx* c, const uint8_t key[32], int seed_source) {
     return MK_OK;
 }
 
+// Makes the pages of a large output buffer present, on several host threads while the GPU works:
+// the buffer is usually fresh memory, and left to the copy its page faults come one after another
+// on one thread.  Every byte is written by the copy afterwards.
+static void touch_pages(uint8_t* out, size_t bytes) {
+    const size_t MIN = 8u << 20, PAGE = 4096;
+    if (bytes < MIN) return;
+    const uint32_t threads = std::min(8u, std::max(1u, std::thread::hardware_concurrency()));
+    auto work = [&](uint32_t t) {
+        const size_t lo = bytes / threads * t, hi = t + 1 == threads ? bytes : bytes / threads * (t + 1);
+        volatile uint8_t* p = out;
+        for (size_t i = lo; i < hi; i += PAGE) p[i] = 0;
+    };
+    std::vector<std::thread> pool;
+    try {
+        pool.reserve(threads);
+        for (uint32_t t = 1; t < threads; t++) pool.emplace_back(work, t);
+    } catch (...) {
+        // the host would not start another thread: the copy faults the remaining pages in
+    }
+    work(0);
+    for (auto& t : pool) t.join();
+}
+
 int mk_derive(mk_ctx* c, const uint8_t key[32], int seed_source, uint64_t first, uint64_t n, uint8_t* out) try {
     if (!c || !key || (!out && n)) return fail(c, MK_ERR_BAD_ARG, "bad argument");
     if (int st = check_source(c, key, seed_source)) return st;
@@ -448,6 +471,7 @@ int mk_derive(mk_ctx* c, const uint8_t key[32], int seed_source, uint64_t first,
         L.count = cnt;
         if (seed_source == MK_SEED_INCREMENTAL) set_incremental(c, key, L.base, L);
         cudaError_t e = mkb::launch_derive(L, c->info.sms, c->stream);
+        if (e == cudaSuccess) touch_pages(out + 32 * done, cnt * 32);
         if (e == cudaSuccess) e = cudaMemcpyAsync(out + 32 * done, d_out, cnt * 32, cudaMemcpyDeviceToHost, c->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
         if (e != cudaSuccess) {

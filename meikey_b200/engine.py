@@ -112,6 +112,19 @@ def _check(lib, ctx_ptr, status: int):
         raise GpuError(status, buf.value.decode(errors="replace"))
 
 
+_bytes_from_size = ctypes.pythonapi.PyBytes_FromStringAndSize
+_bytes_from_size.restype = ctypes.py_object
+_bytes_from_size.argtypes = [ctypes.c_char_p, ctypes.c_ssize_t]
+
+
+def _new_bytes(n: int) -> bytes:
+    """A new bytes object of n bytes for the library to fill before anyone else sees it (what
+    PyBytes_FromStringAndSize without a string is for); not cleared first and not copied after."""
+    if n < 0:
+        raise ValueError("Array length must be >= 0")
+    return _bytes_from_size(None, n)
+
+
 class Context:
     """A device with the comb table built on it (Gpu::new / Kernel::load)."""
 
@@ -144,9 +157,9 @@ class Context:
 
     def derive(self, key: bytes, source: int, first: int, n: int) -> bytes:
         """n full public keys (32 bytes each) of indices first..first+n-1."""
-        out = ctypes.create_string_buffer(32 * n)
+        out = _new_bytes(32 * n)
         _check(self._lib, self._ptr, self._lib.mk_derive(self._ptr, bytes(key), source, first, n, out))
-        return out.raw
+        return out
 
     def derive_noalloc(self, key: bytes, source: int, first: int, n: int) -> bytes:
         """As derive, through the entry point that allocates no device memory (n <= 65536).
@@ -155,9 +168,9 @@ class Context:
         device memory is committed at start-up, or one whose memory a host framework's pool
         owns); the first call on a device should come before any stream capture, and calls
         that overlap on the GPU share, and race on, the library's fixed staging array."""
-        out = ctypes.create_string_buffer(32 * n)
+        out = _new_bytes(32 * n)
         _check(self._lib, self._ptr, self._lib.mk_derive_noalloc(self._ptr, bytes(key), source, first, n, out))
-        return out.raw
+        return out
 
     def table_entry(self, row: int, col: int) -> List[int]:
         out = (ctypes.c_uint32 * 24)()
