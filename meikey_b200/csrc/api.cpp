@@ -57,6 +57,7 @@ struct mk_job {
     std::vector<mkh25519::Needle> needles;
     mkb::MatchSet* d_match = nullptr;
     std::vector<uint8_t*> d_dfa;
+    bool light = true;            // neither regex needles nor the 4-gram prefilter
     uint32_t* d_gram4 = nullptr;  // 4-gram prefilter bitmap (2 MB), allocated on first use
     mkb::HitRecord* d_hits = nullptr;
     uint32_t cap = 1u << 16;
@@ -602,6 +603,35 @@ static int pack_needles(mk_ctx* c, const mk_needle* needles, uint32_t n_needles,
         for (uint32_t i = 0; i < n_needles; i++)
             if (is_text(i) && hosts[i].len >= 4)
                 if (int st = place(i)) return st;
+        // buckets: needles of 4 characters apart from the longer ones (their fifth character is
+        // free), neighbours in the alphabet together so that a bucket's first characters agree
+        std::vector<uint32_t> four, five;
+        for (uint32_t i = 0; i < n_needles; i++)
+            if (is_text(i) && hosts[i].len >= 4) (hosts[i].len == 4 ? four : five).push_back(i);
+        const uint32_t all = (uint32_t)(four.size() + five.size());
+        uint32_t n4 = (uint32_t)((four.size() * mkb::BUCKETS + all / 2) / all);
+        if (!four.empty()) n4 = std::max(n4, 1u);
+        if (!five.empty()) n4 = std::min(n4, mkb::BUCKETS - 1);
+        auto fill = [&](std::vector<uint32_t>& list, uint32_t first, uint32_t count) {
+            std::sort(list.begin(), list.end(), [&](uint32_t a, uint32_t b) { return hosts[a].bytes < hosts[b].bytes; });
+            for (size_t q = 0; q < list.size(); q++) {
+                const mkh25519::Needle& h = hosts[list[q]];
+                const uint32_t b = first + (uint32_t)(q * count / list.size());
+                for (uint32_t k = 0; k < mkb::BUCKET_CHARS; k++) {
+                    const uint64_t bitk = 1ull << (mkb::BUCKETS * k + b);
+                    if (k >= h.len) {
+                        for (auto& m : ms.bucket) m |= bitk;
+                        ms.bucket_end |= bitk;
+                        continue;
+                    }
+                    const uint8_t ch = h.bytes[k];
+                    ms.bucket[b64_value(ch)] |= bitk;
+                    if (h.fold && ch >= 'a' && ch <= 'z') ms.bucket[b64_value(ch) - 26] |= bitk;
+                }
+            }
+        };
+        fill(four, 0, n4);
+        fill(five, n4, mkb::BUCKETS - n4);
         if (gram4) gram4->assign(mkb::GRAM4_WORDS, 0u);
         for (uint32_t i = 0; gram4 && i < n_needles; i++) {
             if (!is_text(i) || hosts[i].len < 4) continue;
@@ -633,6 +663,27 @@ static int pack_needles(mk_ctx* c, const mk_needle* needles, uint32_t n_needles,
     ms.sa_words = ms.n_text ? (bit + 63) / 64 : 0;
     if (!prefilter) ms.short_words = ms.sa_words;
     ms.narrow = ms.n_text && !prefilter && bit <= 32;
+    // quick compare (see MatchSet)
+    ms.quick = ms.n_text > 0;
+    for (uint32_t i = 0; i < n_needles && ms.quick; i++) {
+        if (!is_text(i)) continue;
+        const mkh25519::Needle& h = hosts[i];
+        const bool end = h.mode == MK_MODE_SUFFIX;
+        uint32_t& n = end ? ms.n_quick_suffix : ms.n_quick_contains;
+        bool letters = false;
+        for (uint8_t ch : h.bytes) letters = letters || (ch >= 'a' && ch <= 'z');
+        if ((h.fold && letters) || n >= (end ? mkb::QUICK_SUFFIX : mkb::QUICK_CONTAINS) || (!end && h.len < 3)) {
+            ms.quick = 0;
+            break;
+        }
+        const uint32_t chars = std::min<uint32_t>(h.len, 5u), at = end ? mkb::QUICK_CONTAINS + n : n;
+        uint32_t v = 0;
+        for (uint32_t k = 0; k < chars; k++) v = v << 6 | (uint32_t)b64_value(h.bytes[end ? h.len - chars + k : k]);
+        const uint32_t mask = (1u << (6 * chars)) - 1u, up = end ? 0u : 32u - 6u * chars;
+        ms.quick_value[at] = v << up;
+        ms.quick_mask[at] = mask << up;
+        n++;
+    }
     return MK_OK;
 }
 
@@ -674,6 +725,7 @@ static int upload_needles(mk_job* j, mkb::MatchSet& ms, std::vector<mkh25519::Ne
     MK_CUDA(c, cudaMemcpyAsync(j->d_match, &ms, sizeof ms, cudaMemcpyHostToDevice, c->stream));
     MK_CUDA(c, cudaStreamSynchronize(c->stream));
     j->h2d += sizeof ms;
+    j->light = ms.n_regex == 0 && !ms.gram4;
     j->needles = std::move(hosts);
     return MK_OK;
 }
@@ -802,6 +854,7 @@ static mkb::KeyLaunch search_params(const mk_job* j, uint64_t base, uint32_t ite
     L.job = j->d_job;
     L.sink = j->d_sink;
     if (incr) set_incremental(c, j->key, base, L);
+    L.light = j->light;
     L.dfa_smem = dfa_smem_bytes(j);
     L.inv_pools = search_pools(c, incr);
     L.table_smem = c->table_smem;
@@ -1088,7 +1141,7 @@ int mk_job_graph_create(mk_job* j, uint32_t iters, uint32_t launches, mk_graph**
     if (e != cudaSuccess) return bail(e, "cudaGraphAddMemsetNode");
     const void* func = nullptr;
     size_t dyn = 0;
-    e = mkb::search_kernel(j->source == MK_SEED_INCREMENTAL, c->kpt, c->block, dfa_smem_bytes(j),
+    e = mkb::search_kernel(j->source == MK_SEED_INCREMENTAL, c->kpt, c->block, j->light, dfa_smem_bytes(j),
                          c->table_smem, &func, &dyn);
     if (e != cudaSuccess) return bail(e, "search_kernel");
     for (uint32_t i = 0; i < launches; i++) {
@@ -1118,7 +1171,7 @@ static int graph_enqueue(mk_graph* g, uint64_t base) {
     mk_ctx* c = j->ctx;
     MK_CUDA(c, cudaSetDevice(c->device));
     // the job's needles may have changed since the graph was made: size the DFA staging anew
-    MK_CUDA(c, mkb::search_kernel(j->source == MK_SEED_INCREMENTAL, c->kpt, c->block, dfa_smem_bytes(j),
+    MK_CUDA(c, mkb::search_kernel(j->source == MK_SEED_INCREMENTAL, c->kpt, c->block, j->light, dfa_smem_bytes(j),
                                 c->table_smem, &g->func,
                                 &g->dyn));
     for (size_t i = 0; i < g->nodes.size(); i++) {

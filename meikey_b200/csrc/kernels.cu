@@ -229,42 +229,93 @@ __device__ __forceinline__ u32 tail_value(const u32 pk[8], int pos) {
 
 #define MK_SIGN_POS 42
 
+// Whether some text needle of a quick-compare job (MatchSet::quick) may match the key: 3 operations a
+// position instead of a table lookup and 6 (one needle on B200: 0.924 -> 0.929 G keys/s, incremental
+// 11.5 -> 12.6, a suffix 13.2).  The bit of position 42 that the x sign decides is left
+// out of every comparison.
+__device__ __forceinline__ bool quick_match(const MatchSet& ms, const u32 pk[8]) {
+    // the key as a big-endian bit string; character p starts at bit 6p - 8 (p = 1 with two zero bits
+    // of the byte before the key)
+    u32 k[9];
+#pragma unroll
+    for (int i = 0; i < 8; i++) k[i] = mkh::bswap32(pk[i]);
+    k[8] = 0;
+    bool any = false;
+    for (u32 n = 0; n < ms.n_quick_contains; n++) {
+        const u32 value = ms.quick_value[n], mask = ms.quick_mask[n];
+#pragma unroll
+        for (int p = 1; p <= 41; p++) {  // 3 characters fit at 41; a longer needle only passes too often
+            const int bit = 6 * p - 8;
+            const u32 w = p == 1 ? k[0] >> 2 : __funnelshift_l(k[bit / 32 + 1], k[bit / 32], bit % 32);
+            const int sign = 248 - bit;  // the sign's place in the window
+            const u32 m = sign < 32 ? mask & ~(0x80000000u >> (sign & 31)) : mask;
+            any |= ((w ^ value) & m) == 0;
+        }
+    }
+    for (u32 n = 0; n < ms.n_quick_suffix; n++)
+        any |= ((k[7] ^ ms.quick_value[QUICK_CONTAINS + n]) & ms.quick_mask[QUICK_CONTAINS + n] & ~0x80u) == 0;
+    return any;
+}
+
 // Tests one key (y only; the character at position 42 is tried with both x signs, as
 // kernel.cu:1804-1875 does) and sets bit `id` of hit_words for every needle that may match.
-// `lane_masks` (null: none) holds, for jobs whose text needles fit in 32 bits of state, the
-// low half of mask word 0 once per lane (value v of lane l at v * 32 + l): every lane reads
-// its own bank.
-__device__ __forceinline__ void match_key(const MatchSet& ms, const u32* lane_masks, const u32 pk[8],
+// `lane_masks` (null: none) is a table with every value's entry once per lane (value v of lane l at
+// v * 32 + l), so that every lane reads its own banks: for jobs whose text needles fit in 32 bits of
+// state the low half of mask word 0 (u32), for jobs with the 4-gram prefilter the bucket filter
+// (u64).  LIGHT: the job has neither the prefilter nor regex needles; their code costs the kernel
+// registers (spills) that a job of a few needles runs faster without (one needle on B200: 0.929 ->
+// 0.936 G keys/s, incremental 12.6 -> 12.9).
+template <bool LIGHT>
+__device__ __forceinline__ void match_key(const MatchSet& ms, const u64* lane_masks, const u32 pk[8],
                                           u64 hit_words[2]) {
     hit_words[0] = hit_words[1] = 0;
-    u32 vals[44];
-#pragma unroll
-    for (int pos = 1; pos < 44; pos++) vals[pos] = tail_value(pk, pos);
+    u32 words = ms.sa_words;
+    if (ms.quick && !quick_match(ms, pk)) {
+        if (LIGHT || ms.n_regex == 0) return;
+        words = 0;
+    }
+    auto value = [&](int pos) { return tail_value(pk, pos); };  // cut out where used: 43 of them do not stay in registers
     // text needles: shift-and over sa_words words of state.  With the 4-gram prefilter, the
     // words of the needles of 4+ characters are scanned only when one of the key's 4-character
-    // windows (position 42 with both values) is the start of such a needle.
-    u32 words = ms.sa_words;
-    if (ms.gram4) {
-        u32 any = 0, gw = vals[1] << 12 | vals[2] << 6 | vals[3];
+    // windows (position 42 with both values) is the start of such a needle.  The bitmap's lookups
+    // are a cache line per lane, 32 a load, and bound the L1 tag stage (5200 of 46700 cycles a key
+    // for 58 needles on B200), so the bucket filter in shared memory lets about one key in a hundred
+    // through to them (58 needles; half of them at 128).
+    if (!LIGHT && ms.gram4) {
+        const u64* lm = lane_masks + (threadIdx.x & 31u);
+        u64 D = 0;
+        u32 acc = 0;
 #pragma unroll
-        for (int p = 1; p + 3 < 44; p++) {
-            gw = (gw << 6 | vals[p + 3]) & 0xffffffu;
-            any |= __ldg(ms.gram4 + (gw >> 5)) >> (gw & 31);
-            if (p <= MK_SIGN_POS && MK_SIGN_POS <= p + 3) {
-                const u32 g2 = gw | 2u << (6 * (p + 3 - MK_SIGN_POS));
-                any |= __ldg(ms.gram4 + (g2 >> 5)) >> (g2 & 31);
+        for (int pos = 1; pos < 44; pos++) {
+            u64 mk = lm[value(pos) * 32u];
+            if (pos == MK_SIGN_POS) mk |= lm[(value(pos) | 2u) * 32u];
+            D = (D << BUCKETS | ((1ull << BUCKETS) - 1)) & mk;
+            acc |= (u32)(D >> 32);
+        }
+        acc |= (u32)((D << BUCKETS & ms.bucket_end) >> 32);
+        u32 any = 0;
+        if (acc >> (BUCKETS * (BUCKET_CHARS - 1) - 32)) {
+            u32 gw = value(1) << 12 | value(2) << 6 | value(3);
+#pragma unroll
+            for (int p = 1; p + 3 < 44; p++) {
+                gw = (gw << 6 | value(p + 3)) & 0xffffffu;
+                any |= __ldg(ms.gram4 + (gw >> 5)) >> (gw & 31);
+                if (p <= MK_SIGN_POS && MK_SIGN_POS <= p + 3) {
+                    const u32 g2 = gw | 2u << (6 * (p + 3 - MK_SIGN_POS));
+                    any |= __ldg(ms.gram4 + (g2 >> 5)) >> (g2 & 31);
+                }
             }
         }
         if (!(any & 1u)) words = ms.short_words;
     }
-    if (lane_masks && words) {
-        const u32* lm = lane_masks + (threadIdx.x & 31u);
+    if (ms.narrow && words) {
+        const u32* lm = reinterpret_cast<const u32*>(lane_masks) + (threadIdx.x & 31u);
         u32 D = 0, acc = 0;
         const u32 first = (u32)ms.first_bit[0], last = (u32)ms.last_bit[0];
 #pragma unroll
         for (int pos = 1; pos < 44; pos++) {
-            u32 mk = lm[vals[pos] * 32u];
-            if (pos == MK_SIGN_POS) mk |= lm[(vals[pos] | 2u) * 32u];
+            u32 mk = lm[value(pos) * 32u];
+            if (pos == MK_SIGN_POS) mk |= lm[(value(pos) | 2u) * 32u];
             D = ((D << 1) | first) & mk;
             acc |= D & last;
         }
@@ -283,8 +334,8 @@ __device__ __forceinline__ void match_key(const MatchSet& ms, const u32* lane_ma
         u64 first = ms.first_bit[wi], last = ms.last_bit[wi];
 #pragma unroll
         for (int pos = 1; pos < 44; pos++) {
-            u64 mk = ms.mask[wi][vals[pos]];
-            if (pos == MK_SIGN_POS) mk |= ms.mask[wi][vals[pos] | 2u];
+            u64 mk = ms.mask[wi][value(pos)];
+            if (pos == MK_SIGN_POS) mk |= ms.mask[wi][value(pos) | 2u];
             D = ((D << 1) | first) & mk;
             acc |= D & last;
         }
@@ -302,7 +353,7 @@ __device__ __forceinline__ void match_key(const MatchSet& ms, const u32* lane_ma
     }
     // regex needles: eight DFA walks side by side, so that their table lookups (shared
     // memory when the launch staged the tables there, else global) overlap
-    for (u32 r0 = 0; r0 < ms.n_regex; r0 += 8) {
+    for (u32 r0 = 0; !LIGHT && r0 < ms.n_regex; r0 += 8) {
         const uint16_t* t[8];
         u32 s[8], alt[8];
 #pragma unroll
@@ -312,7 +363,7 @@ __device__ __forceinline__ void match_key(const MatchSet& ms, const u32* lane_ma
         }
 #pragma unroll 1
         for (int pos = 1; pos < 44; pos++) {
-            const u32 v = tail_value(pk, pos);
+            const u32 v = value(pos);
 #pragma unroll
             for (int q = 0; q < 8; q++) {
                 if (pos == MK_SIGN_POS) alt[q] = t[q][s[q] * 65u + (v | 2u)];
@@ -450,8 +501,8 @@ __device__ __forceinline__ int incr_key(int s) {
 // Backward pass: `inv` is 1/(product of the batch's denominators); yields each key's
 // canonical y (sign bit 0), tests the needles and reports candidate hits (none when `valid` is
 // false: a run past the launch's last one).  INCR: slot j holds key incr_key(j).
-template <int KPT, bool INCR>
-__device__ __forceinline__ void backward(const KeyLaunch& L, const MatchSet& ms, const u32* lane_masks, u64 first,
+template <int KPT, bool INCR, bool LIGHT>
+__device__ __forceinline__ void backward(const KeyLaunch& L, const MatchSet& ms, const u64* lane_masks, u64 first,
                                          bool valid, const Batch<KPT>& b, fe inv, u32& sink) {
 #pragma unroll 1
     for (int j = KPT - 1; j >= 0; j--) {
@@ -460,7 +511,7 @@ __device__ __forceinline__ void backward(const KeyLaunch& L, const MatchSet& ms,
         if (j > 0) inv = mk32::fe_mul(inv, b.den[j]);
         sink ^= pk[7];
         u64 hw[2];
-        match_key(ms, lane_masks, pk, hw);
+        match_key<LIGHT>(ms, lane_masks, pk, hw);
         if (!valid) hw[0] = hw[1] = 0;
         const bool any = (hw[0] | hw[1]) != 0;
         // warp ballot: the (rare) warps with a hit compact their records into the ring
@@ -627,18 +678,18 @@ __device__ __forceinline__ void incr_fracs(const ge& Q, const uint4* steps, Batc
 // keys_per_iter·B (one mixed addition) per iteration.  No comb table is read.
 // STAB: the comb table lives in shared memory (copied by every CTA at the start, in place of
 // the staging slots; tables of a few hundred to a few thousand entries, 40+ rows).
-template <int KPT, int BLOCK, bool INCR, bool ROT, bool STAB = false>
+template <int KPT, int BLOCK, bool INCR, bool ROT, bool LIGHT, bool STAB = false>
 __global__ void __launch_bounds__(BLOCK, 512 / BLOCK) k_search(const KeyLaunch L) {
     constexpr int CT = ROT ? BLOCK : BLOCK - 32;  // compute threads
     constexpr int CW = CT / 32;                   // compute warps
     extern __shared__ uint4 dyn_smem[];
     fe (*prod)[CT] = reinterpret_cast<fe (*)[CT]>(dyn_smem);
-    fe (*scratch)[CT] = prod + 2;
-    EntrySlot* slots = reinterpret_cast<EntrySlot*>(scratch + 2);
-    uint4* stab = reinterpret_cast<uint4*>(scratch + 2);  // STAB: the table in place of the slots
+    fe* scratch = prod[2];  // one inversion runs at a time: the next one waits for this one's warp
+    EntrySlot* slots = reinterpret_cast<EntrySlot*>(scratch + CT);
+    uint4* stab = reinterpret_cast<uint4*>(scratch + CT);  // STAB: the table in place of the slots
     __shared__ CombGeom g;
     __shared__ MatchSet ms;
-    __shared__ u32 lane_masks[64 * 32];  // see match_key
+    __shared__ u64 lane_masks[64 * 32];  // see match_key
     __shared__ u32 key[8];
     __shared__ mkh::CounterMid mid;
     __shared__ volatile u64 stop_iter;
@@ -663,8 +714,8 @@ __global__ void __launch_bounds__(BLOCK, 512 / BLOCK) k_search(const KeyLaunch L
 #pragma unroll
             for (int q = 0; q < 6; q++) stab[e * 6 + q] = L.table[(u64)e * (COMB_STRIDE_WORDS / 4) + q];
     u32 dfa_need = 0;
-    for (u32 r = 0; r < ms.n_regex; r++) dfa_need += (ms.dfa_states[r] * 130u + 15u) & ~15u;
-    if (L.dfa_smem && dfa_need <= L.dfa_smem) {
+    for (u32 r = 0; !LIGHT && r < ms.n_regex; r++) dfa_need += (ms.dfa_states[r] * 130u + 15u) & ~15u;
+    if (!LIGHT && L.dfa_smem && dfa_need <= L.dfa_smem) {
         // stage the job's DFA tables behind the other dynamic buffers (only when the launch
         // reserved room for all of them) and point the matcher at the copies (16-byte
         // aligned tables, copied in u16 units)
@@ -687,7 +738,9 @@ __global__ void __launch_bounds__(BLOCK, 512 / BLOCK) k_search(const KeyLaunch L
         }
     }
     if (ms.narrow)
-        for (u32 i = tid; i < 64u * 32u; i += BLOCK) lane_masks[i] = (u32)ms.mask[0][i >> 5];
+        for (u32 i = tid; i < 64u * 32u; i += BLOCK) reinterpret_cast<u32*>(lane_masks)[i] = (u32)ms.mask[0][i >> 5];
+    else if (!LIGHT && ms.gram4)
+        for (u32 i = tid; i < 64u * 32u; i += BLOCK) lane_masks[i] = ms.bucket[i >> 5];
     if (INCR && tid < (u32)INCR_STEPS) step_to_yx(steps, tid);
     if (tid == 0 && L.seed_src == 1) mid = mkh::counter_mid(key);
     __syncthreads();
@@ -707,7 +760,7 @@ __global__ void __launch_bounds__(BLOCK, 512 / BLOCK) k_search(const KeyLaunch L
             const int b = it & 1;
             bar_sync(1 + b, BLOCK);
             read_stop(it);
-            invert_pools(prod[b], scratch[b], CT, pools);
+            invert_pools(prod[b], scratch, CT, pools);
             __syncwarp();
             bar_arrive(3 + b, BLOCK);
             if (it + 1 >= iters || it + 1 >= stop_iter) break;
@@ -744,7 +797,7 @@ __global__ void __launch_bounds__(BLOCK, 512 / BLOCK) k_search(const KeyLaunch L
             if (inverts(it)) {
                 bar_sync(1 + b, BLOCK);
                 read_stop(it);
-                invert_pools(prod[b], scratch[b], CT, pools);
+                invert_pools(prod[b], scratch, CT, pools);
                 __syncwarp();
                 bar_arrive(3 + b, BLOCK);
             } else {
@@ -757,7 +810,7 @@ __global__ void __launch_bounds__(BLOCK, 512 / BLOCK) k_search(const KeyLaunch L
         const int b = p & 1;
         if (!inverts(p)) bar_sync(3 + b, BLOCK);
         if (chunk_of(p) - (tid & 31u) < L.chunks)
-            backward<KPT, INCR>(L, ms, ms.narrow ? lane_masks : nullptr, first_of(p), chunk_of(p) < L.chunks, batch[b],
+            backward<KPT, INCR, LIGHT>(L, ms, lane_masks, first_of(p), chunk_of(p) < L.chunks, batch[b],
                                 prod[b][tid], sink);
         if (it >= iters || it >= stop_iter) break;
     }
@@ -853,30 +906,31 @@ __global__ void __launch_bounds__(DERIVE_BLOCK, 512 / DERIVE_BLOCK) k_derive(con
 
 #define MK_VARIANTS(X) X(4, 256) X(8, 256) X(16, 256) X(4, 512) X(8, 512) X(16, 512)
 
-// dynamic shared memory of a search: products and inversion scratch (two buffers each) and the
+// dynamic shared memory of a search: products (two buffers), inversion scratch and the
 // per-thread table staging slots (the incremental source reads no comb table and needs none)
 static size_t dyn_bytes(bool incr, uint32_t block, uint32_t table_smem) {
     const size_t fe_bytes = 32, threads = search_kernel_threads(incr, block, table_smem);
-    if (table_smem && !incr) return 4 * threads * fe_bytes + table_smem;  // the table in place of the slots
-    return 4 * threads * fe_bytes + (incr ? 0 : threads * sizeof(EntrySlot));
+    if (table_smem && !incr) return 3 * threads * fe_bytes + table_smem;  // the table in place of the slots
+    return 3 * threads * fe_bytes + (incr ? 0 : threads * sizeof(EntrySlot));
 }
 
 // search kernels with the comb table in shared memory: the dedicated-inverter layout, block
 // 512, keys per thread 4 and 8
 static const void* stab_kernel_of(uint32_t kpt, uint32_t block) {
     if (block != 512) return nullptr;
-    if (kpt == 4) return (const void*)k_search<4, 512, false, false, true>;
-    if (kpt == 8) return (const void*)k_search<8, 512, false, false, true>;
+    if (kpt == 4) return (const void*)k_search<4, 512, false, false, false, true>;
+    if (kpt == 8) return (const void*)k_search<8, 512, false, false, false, true>;
     return nullptr;
 }
 
+template <bool LIGHT>
 static const void* kernel_of(bool incr, uint32_t kpt, uint32_t block) {
     if (!incr)
-        return block == 512 ? (const void*)k_search<HASHED_KEYS, 512, false, true>
-               : block == 256 ? (const void*)k_search<HASHED_KEYS, 256, false, true>
+        return block == 512 ? (const void*)k_search<HASHED_KEYS, 512, false, true, LIGHT>
+               : block == 256 ? (const void*)k_search<HASHED_KEYS, 256, false, true, LIGHT>
                               : nullptr;
 #define MK_FN(K, B) \
-    if (kpt == K && block == B) return (const void*)k_search<K, B, true, false>;
+    if (kpt == K && block == B) return (const void*)k_search<K, B, true, false, LIGHT>;
     MK_VARIANTS(MK_FN)
 #undef MK_FN
     return nullptr;
@@ -886,15 +940,12 @@ static cudaError_t prepare(const void* f, size_t dyn) {
     return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
 }
 
-// the search kernel of a variant (the table-in-shared-memory search when table_smem > 0)
-static const void* variant_kernel(bool incr, uint32_t kpt, uint32_t block, uint32_t table_smem) {
-    return table_smem && !incr ? stab_kernel_of(kpt, block) : kernel_of(incr, kpt, block);
-}
-
-cudaError_t search_kernel(bool incr, uint32_t kpt, uint32_t block, uint32_t dfa_smem, uint32_t table_smem,
+cudaError_t search_kernel(bool incr, uint32_t kpt, uint32_t block, bool light, uint32_t dfa_smem, uint32_t table_smem,
                           const void** func, size_t* dyn) {
     const uint32_t tsm = incr ? 0 : table_smem;
-    const void* f = variant_kernel(incr, kpt, block, tsm);
+    const void* f = tsm ? stab_kernel_of(kpt, block)
+                    : light ? kernel_of<true>(incr, kpt, block)
+                            : kernel_of<false>(incr, kpt, block);
     // a comb table takes the shared memory of DFA tables
     if (!f || dfa_smem > DFA_SMEM_MAX || (tsm && dfa_smem)) return cudaErrorInvalidValue;
     *func = f;
@@ -907,7 +958,7 @@ cudaError_t launch_search(const KeyLaunch& L, uint32_t kpt, uint32_t block, uint
     if (incr && (kpt > (uint32_t)INCR_STEPS || !L.incr)) return cudaErrorInvalidValue;
     const void* f = nullptr;
     size_t dyn = 0;
-    cudaError_t e = search_kernel(incr, kpt, block, L.dfa_smem, L.table_smem, &f, &dyn);
+    cudaError_t e = search_kernel(incr, kpt, block, L.light, L.dfa_smem, L.table_smem, &f, &dyn);
     if (e != cudaSuccess) return e;
     void* args[] = {const_cast<KeyLaunch*>(&L)};
     return cudaLaunchKernel(f, dim3(grid), dim3(block), args, dyn, st);
@@ -916,7 +967,7 @@ cudaError_t launch_search(const KeyLaunch& L, uint32_t kpt, uint32_t block, uint
 cudaError_t search_occupancy(uint32_t kpt, uint32_t block, uint32_t table_smem, int* blocks_per_sm) {
     const void* f = nullptr;
     size_t dyn = 0;
-    cudaError_t e = search_kernel(false, kpt, block, 0, table_smem, &f, &dyn);
+    cudaError_t e = search_kernel(false, kpt, block, false, 0, table_smem, &f, &dyn);
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, f, (int)block, dyn);
 }

@@ -35,6 +35,8 @@ struct KeyLaunch {
     const uint4* incr;     // INCR_WINDOWS·16 entries j·16^w·B, then INCR_STEPS entries j·B (table form)
     uint32_t start[32];    // (s0 + base)·B as x, y, 1, xy
     uint32_t delta[24];    // CTAs·search_kernel_threads·keys·B: a search thread's jump between iterations
+    // the job has neither regex needles nor the 4-gram prefilter (picks the kernel)
+    bool light;
     // bytes of shared memory for the job's DFA tables (each 16-byte aligned; 0: read them
     // from global memory)
     uint32_t dfa_smem;
@@ -107,7 +109,7 @@ constexpr double MADS_MUL_SCHOOLBOOK = 64 + 64 + 16;
 constexpr double MADS_INVERT = 18 * (30 * 6 + 2 * 72);
 // The search kernel of a variant and its dynamic shared memory (for graph nodes); sets the
 // kernel's shared-memory limit like launch_search does.
-cudaError_t search_kernel(bool incr, uint32_t kpt, uint32_t block, uint32_t dfa_smem, uint32_t table_smem,
+cudaError_t search_kernel(bool incr, uint32_t kpt, uint32_t block, bool light, uint32_t dfa_smem, uint32_t table_smem,
                           const void** func, size_t* dyn);
 cudaError_t search_occupancy(uint32_t kpt, uint32_t block, uint32_t table_smem, int* blocks_per_sm);
 // multiply-adds per second of the carry-chain row microbenchmark and of plain mad.lo.u32

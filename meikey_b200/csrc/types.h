@@ -51,6 +51,18 @@ struct MatchSet {
     uint64_t suffix_bit[SA_WORDS];// last bit of every suffix-needle (tested at the end only)
     uint16_t text_id[MAX_NEEDLES];// caller's needle index per text needle
     uint16_t text_last[MAX_NEEDLES]; // global bit index of each text needle's last bit
+    // quick compare: when every text needle is case-sensitive (or holds no letter) and they are at
+    // most QUICK_CONTAINS contains-needles of 3+ characters and QUICK_SUFFIX suffixes, a key is
+    // compared as a bit string first: the first 30 bits (5 characters) of a contains-needle, left
+    // aligned, at every position, the last 30 of a suffix, right aligned, at the end
+    uint32_t quick;               // 1: on
+    uint32_t n_quick_contains, n_quick_suffix;
+    uint32_t quick_value[6], quick_mask[6];  // the contains-needles, then from QUICK_CONTAINS the suffixes
+    // bucket filter of the needles gram4 holds: bit 12·k + b of bucket[v] is set when some needle of
+    // bucket b takes value v as its character k (k < 5; of a 4-character needle every value as its
+    // fifth, and bucket_end has that bit for the end of the key)
+    uint64_t bucket[64];
+    uint64_t bucket_end;
     // regex needles
     const uint8_t* dfa[16];
     uint32_t dfa_states[16];
@@ -61,6 +73,8 @@ struct MatchSet {
     const uint32_t* gram4;
 };
 
+constexpr uint32_t QUICK_CONTAINS = 2, QUICK_SUFFIX = 4;
+constexpr uint32_t BUCKETS = 12, BUCKET_CHARS = 5;
 constexpr uint32_t GRAM4_WORDS = 1u << 19;  // 2^24 bits
 constexpr uint32_t GRAM4_MIN_NEEDLES = 8;   // long text needles from which a job uses the prefilter
 
