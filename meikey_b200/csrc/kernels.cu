@@ -655,7 +655,10 @@ __device__ __forceinline__ void incr_fracs(const ge& Q, const uint4* steps, Batc
 //     warp it mod the CTA's warps, so that consecutive inversions run on different SM
 //     sub-partitions and every warp carries the same share.  A dedicated inverter leaves its
 //     sub-partition with three compute warps against four (warp w runs on sub-partition w % 4):
-//     on B200, 8 keys per thread, 0.82 G keys/s against 0.89 with the rotating duty;
+//     on B200, 8 keys per thread, 0.82 G keys/s against 0.89 with the rotating duty.  The inverting
+//     warp does its backward pass of it-1 first: by then the others have arrived, so it does not
+//     wait for the slowest of them, and they still have a whole forward pass to run before they need
+//     the inverses (0.936 -> 0.974 G keys/s; 0.916 -> 0.966 at 16 pools, whose chain is longer);
 //   ROT false (the incremental source, whose iterations are an order shorter): the CTA's last warp,
 //     which does nothing else (BLOCK-32 compute threads), so the inversion's dependent chain runs
 //     beside the other warps' work (11.0 against 8.8 G keys/s with the rotating duty).
@@ -794,25 +797,27 @@ __global__ void __launch_bounds__(BLOCK, 512 / BLOCK) k_search(const KeyLaunch L
                 combs<KPT, STAB>(L, g, sc, slot, stab, batch[b]);
             }
             prod[b][tid] = batch[b].prod;
-            if (inverts(it)) {
-                bar_sync(1 + b, BLOCK);
-                read_stop(it);
-                invert_pools(prod[b], scratch, CT, pools);
-                __syncwarp();
-                bar_arrive(3 + b, BLOCK);
-            } else {
-                bar_arrive(1 + b, BLOCK);
-            }
+            if (!inverts(it)) bar_arrive(1 + b, BLOCK);
         }
-        if (it == 0) continue;
-        // backward pass of iteration it - 1
-        const u64 p = it - 1;
-        const int b = p & 1;
-        if (!inverts(p)) bar_sync(3 + b, BLOCK);
-        if (chunk_of(p) - (tid & 31u) < L.chunks)
-            backward<KPT, INCR, LIGHT>(L, ms, lane_masks, first_of(p), chunk_of(p) < L.chunks, batch[b],
-                                prod[b][tid], sink);
-        if (it >= iters || it >= stop_iter) break;
+        if (it > 0) {
+            // backward pass of iteration it - 1
+            const u64 p = it - 1;
+            const int b = p & 1;
+            if (!inverts(p)) bar_sync(3 + b, BLOCK);
+            if (chunk_of(p) - (tid & 31u) < L.chunks)
+                backward<KPT, INCR, LIGHT>(L, ms, lane_masks, first_of(p), chunk_of(p) < L.chunks, batch[b],
+                                           prod[b][tid], sink);
+            if (it >= iters || it >= stop_iter) break;
+        }
+        if (inverts(it)) {
+            // iteration it was run: the loop ends above otherwise
+            const int b = it & 1;
+            bar_sync(1 + b, BLOCK);
+            read_stop(it);
+            invert_pools(prod[b], scratch, CT, pools);
+            __syncwarp();
+            bar_arrive(3 + b, BLOCK);
+        }
     }
     // the decision of the iteration that ended the loop is visible here (its inverses were waited for)
     if (ROT && tid == 0 && stop_iter < iters) atomicOr(&L.job->status, 1u);
