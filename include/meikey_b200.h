@@ -71,9 +71,9 @@ enum mk_mode { MK_MODE_CONTAINS = 0, MK_MODE_SUFFIX = 1, MK_MODE_REGEX = 2 };
 typedef struct mk_options {
     uint32_t table_rows;      /* 10..63; default 12 (rows 10-20 are HBM tables of 26 GB down to 11 MB, 32-63 the
                                  comb windows of 8 down to 4 bits) */
-    uint32_t keys_per_thread; /* keys per counted thread of one iteration's span (default 16), and the incremental
-                                 source's and mk_derive's batch per thread; searches of hashed seeds
-                                 invert in batches of 8 keys per thread, the fastest, whatever the span */
+    uint32_t keys_per_thread; /* keys per counted thread of one iteration's span (default 16).  Searches batch 8
+                                 keys per thread (hashed seeds) or 16 (incremental source), the fastest,
+                                 whatever the span; with table_in_smem as many as given */
     uint32_t block;           /* threads per CTA (default 512): 256 or 512, keys per thread 4, 8 or 16;
                                  see inverter_rotates for who inverts */
     uint32_t blocks_per_sm;   /* resident CTAs per SM the grid is sized for (0 = occupancy maximum) */

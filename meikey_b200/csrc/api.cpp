@@ -370,7 +370,7 @@ int mk_ctx_create(int device, const mk_options* options, mk_ctx** out) try {
             return fail(c, MK_ERR_OUT_OF_MEMORY, "incremental table allocation failed");
         }
         MK_CUDA(c, cudaMemcpy(c->incr, words.data(), words.size() * 4, cudaMemcpyHostToDevice));
-        mkh25519::niels_of_multiple((uint64_t)c->grid * mkb::search_kernel_threads(true, c->block, 0) * c->kpt,
+        mkh25519::niels_of_multiple((uint64_t)c->grid * mkb::search_kernel_threads(true, c->block, 0) * mkb::INCR_KEYS,
                                     c->delta);
     }
     // info

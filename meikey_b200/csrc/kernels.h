@@ -62,12 +62,12 @@ inline uint32_t search_threads(uint32_t block, uint32_t layout) {
     return layout == LAYOUT_HASH_WARPS ? 352u : layout == LAYOUT_ROTATING ? block : block - 32u;
 }
 
-// keys per thread and iteration of the hashed-seed search kernel
-constexpr uint32_t HASHED_KEYS = 8;
+// keys per thread and iteration of the search kernels of hashed seeds and of the incremental source
+constexpr uint32_t HASHED_KEYS = 8, INCR_KEYS = 16;
 
 // keys per thread and iteration, and compute threads per CTA, of the kernel that serves a search
 inline uint32_t search_kernel_keys(bool incr, uint32_t kpt, uint32_t table_smem) {
-    return incr || table_smem ? kpt : HASHED_KEYS;
+    return incr ? INCR_KEYS : table_smem ? kpt : HASHED_KEYS;
 }
 inline uint32_t search_kernel_threads(bool incr, uint32_t block, uint32_t table_smem) {
     return incr || table_smem ? block - 32u : block;
