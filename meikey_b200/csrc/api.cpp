@@ -525,8 +525,8 @@ int mk_table_entry(mk_ctx* c, uint32_t row, uint64_t col, uint32_t out[24]) {
 // straddles a 64-bit word; fold lowercases the needle and accepts the uppercase value too),
 // DFA tables are validated and kept for upload.  A job with GRAM4_MIN_NEEDLES or more text
 // needles of 4+ characters also gets the 4-gram prefilter: needles shorter than 4 are packed
-// first (the words every key scans), and `gram4` receives the bitmap of the long needles'
-// first 4-grams in every case variant.  No device work.
+// first (the words every key scans), and `gram4` receives the long needles' first 4-grams in
+// every case variant, at most 16 a needle.  No device work.
 static int pack_needles(mk_ctx* c, const mk_needle* needles, uint32_t n_needles, mkb::MatchSet& ms,
                         std::vector<mkh25519::Needle>& hosts, std::vector<uint32_t>* gram4) {
     if (n_needles && !needles) return fail(c, MK_ERR_BAD_ARG, "bad argument");
@@ -568,7 +568,7 @@ static int pack_needles(mk_ctx* c, const mk_needle* needles, uint32_t n_needles,
             return fail(c, MK_ERR_BAD_ARG, "unknown needle mode");
         }
     }
-    // the packing is the same whether or not the bitmap is wanted (gram4 null: check only)
+    // the packing is the same whether or not the filters are wanted (gram4 null: check only)
     const bool prefilter = long_text >= mkb::GRAM4_MIN_NEEDLES;
     uint32_t bit = 0;  // next free bit in the shift-and state
     auto place = [&](uint32_t i) -> int {
@@ -630,9 +630,10 @@ static int pack_needles(mk_ctx* c, const mk_needle* needles, uint32_t n_needles,
                 }
             }
         };
-        fill(four, 0, n4);
-        fill(five, n4, mkb::BUCKETS - n4);
-        if (gram4) gram4->assign(mkb::GRAM4_WORDS, 0u);
+        if (gram4) {
+            fill(four, 0, n4);
+            fill(five, n4, mkb::BUCKETS - n4);
+        }
         for (uint32_t i = 0; gram4 && i < n_needles; i++) {
             if (!is_text(i) || hosts[i].len < 4) continue;
             const mkh25519::Needle& h = hosts[i];
@@ -652,7 +653,7 @@ static int pack_needles(mk_ctx* c, const mk_needle* needles, uint32_t n_needles,
                     if (pick >= nv[k]) ok = false;
                     g = g << 6 | (uint32_t)vals[k][pick];
                 }
-                if (ok) (*gram4)[g >> 5] |= 1u << (g & 31);
+                if (ok) gram4->push_back(g);
             }
         }
     } else {
@@ -698,9 +699,13 @@ static int upload_needles(mk_job* j, mkb::MatchSet& ms, std::vector<mkh25519::Ne
     // all copies are ordered on the context's stream after the allocations; the stream is
     // drained before returning, while the host vectors are still alive
     if (!gram4.empty()) {
-        if (!j->d_gram4 && !pool_alloc(c, &j->d_gram4, gram4.size() * 4))
+        // the bitmap is cleared and its few set bits written on the device: building its 2 MB here and
+        // copying them took most of a server tick's needle update
+        if (!j->d_gram4 && !pool_alloc(c, &j->d_gram4, (mkb::GRAM4_WORDS + 16u * mkb::MAX_NEEDLES) * 4))
             return fail(c, MK_ERR_OUT_OF_MEMORY, "prefilter allocation");
-        MK_CUDA(c, cudaMemcpyAsync(j->d_gram4, gram4.data(), gram4.size() * 4, cudaMemcpyHostToDevice, c->stream));
+        uint32_t* list = j->d_gram4 + mkb::GRAM4_WORDS;
+        MK_CUDA(c, cudaMemcpyAsync(list, gram4.data(), gram4.size() * 4, cudaMemcpyHostToDevice, c->stream));
+        MK_CUDA(c, mkb::launch_set_grams(j->d_gram4, list, (uint32_t)gram4.size(), c->stream));
         j->h2d += gram4.size() * 4;
         ms.gram4 = j->d_gram4;
     }

@@ -1005,6 +1005,18 @@ cudaError_t launch_derive(const KeyLaunch& L, uint32_t sms, cudaStream_t st) {
                             dyn, st);
 }
 
+__global__ void k_set_grams(uint32_t* bitmap, const uint32_t* grams, uint32_t n) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) atomicOr(bitmap + (grams[i] >> 5), 1u << (grams[i] & 31u));
+}
+
+cudaError_t launch_set_grams(uint32_t* bitmap, const uint32_t* grams, uint32_t n, cudaStream_t st) {
+    const cudaError_t e = cudaMemsetAsync(bitmap, 0, GRAM4_WORDS * sizeof(uint32_t), st);
+    if (e != cudaSuccess) return e;
+    k_set_grams<<<(n + 255) / 256, 256, 0, st>>>(bitmap, grams, n);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_build_table(uint4* table, const CombGeom& g, const uint32_t* points, uint64_t first,
                                uint64_t count, cudaStream_t st) {
     uint32_t blocks = (uint32_t)((count + 255) / 256);

@@ -122,6 +122,8 @@ cudaError_t measure_imad_rates(int sms, cudaStream_t st, double rates[4]);
 // current device (looked up when a context is created).
 constexpr uint64_t NOALLOC_MAX_KEYS = 1ull << 16;
 cudaError_t noalloc_staging(uint8_t** ptr);
+// Clears the GRAM4_WORDS words of the bitmap and sets the bits of n 24-bit values.
+cudaError_t launch_set_grams(uint32_t* bitmap, const uint32_t* grams, uint32_t n, cudaStream_t st);
 cudaError_t launch_build_table(uint4* table, const CombGeom& g, const uint32_t* points, uint64_t first,
                                uint64_t count, cudaStream_t st);
 
