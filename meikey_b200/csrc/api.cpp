@@ -520,6 +520,57 @@ int mk_table_entry(mk_ctx* c, uint32_t row, uint64_t col, uint32_t out[24]) {
     return MK_OK;
 }
 
+// What a key that matches a DFA must hold: on the last way from the start state to the match, which
+// does not come back to it, the values possible as characters 0..4, and whether the key may end there
+// after 3 or 4 of them.  The chance of a random key to hold some such values in a row, or 1 when
+// the DFA can match without (or within two characters).
+struct DfaFilter {
+    uint64_t values[mkb::BUCKET_CHARS];
+    bool end[mkb::BUCKET_CHARS + 1];
+    double chance;
+};
+
+static DfaFilter dfa_filter(const uint8_t* table, uint32_t states) {
+    DfaFilter f{};
+    f.chance = 1.0;
+    auto at = [&](uint32_t s, uint32_t v) {
+        const size_t i = ((size_t)s * 65 + v) * 2;
+        return (uint32_t)table[i] | (uint32_t)table[i + 1] << 8;
+    };
+    auto accepts = [&](uint32_t s) { return s == 0 || at(s, 64) != 0; };  // at the end of the key
+    if (states < 2 || accepts(1)) return f;
+    // states from which the key can still match
+    std::vector<char> live(states);
+    for (uint32_t s = 0; s < states; s++) live[s] = accepts(s);
+    for (bool more = true; more;) {
+        more = false;
+        for (uint32_t s = 0; s < states; s++)
+            for (uint32_t v = 0; v < 64 && !live[s]; v++)
+                if (live[at(s, v)]) live[s] = more = true;
+    }
+    std::vector<char> now(states, 0), next(states);
+    now[1] = 1;
+    double chance = 43.0;
+    for (uint32_t k = 0; k < mkb::BUCKET_CHARS; k++) {
+        std::fill(next.begin(), next.end(), 0);
+        int n = 0;
+        for (uint32_t v = 0; v < 64; v++) {
+            bool any = false;
+            for (uint32_t s = 0; s < states; s++)
+                if (now[s] && at(s, v) != 1 && live[at(s, v)]) next[at(s, v)] = any = true;
+            if (any) {
+                f.values[k] |= 1ull << v;
+                n++;
+            }
+        }
+        now.swap(next);
+        chance *= n / 64.0;
+        for (uint32_t s = 0; s < states; s++) f.end[k + 1] = f.end[k + 1] || (now[s] && accepts(s));
+    }
+    if (!f.end[1] && !f.end[2]) f.chance = chance;
+    return f;
+}
+
 // Compiles needles into a MatchSet on the host (src/service/gpu.rs:618-660 Needle::new,
 // dfa.rs:189-200): text needles become bit ranges of the shift-and state (a needle never
 // straddles a 64-bit word; fold lowercases the needle and accepts the uppercase value too),
@@ -570,6 +621,36 @@ static int pack_needles(mk_ctx* c, const mk_needle* needles, uint32_t n_needles,
     }
     // the packing is the same whether or not the filters are wanted (gram4 null: check only)
     const bool prefilter = long_text >= mkb::GRAM4_MIN_NEEDLES;
+    // regexes that few keys can match by the bucket filter; alone (without needles that need the filter
+    // anyway) it costs about one DFA walk, so it takes two of them to pay
+    ms.regex_always = (1u << ms.n_regex) - 1u;
+    if (gram4 && ms.n_regex) {
+        std::vector<std::pair<double, uint32_t>> rare;
+        std::vector<DfaFilter> filters(ms.n_regex);
+        for (uint32_t q = 0; q < ms.n_regex; q++) {
+            const mkh25519::Needle& h = hosts[ms.regex_id[q]];
+            if (h.len > 256) continue;  // keeps the search for its values short
+            filters[q] = dfa_filter(h.bytes.data(), h.len);
+            if (filters[q].chance <= 0.01) rare.push_back({filters[q].chance, q});
+        }
+        std::sort(rare.begin(), rare.end());
+        if (rare.size() >= 2 || (prefilter && !rare.empty())) {
+            ms.buckets = 1;
+            ms.n_filtered = std::min<uint32_t>((uint32_t)rare.size(), prefilter ? mkb::REGEX_BUCKETS : mkb::BUCKETS);
+            for (uint32_t i = 0; i < ms.n_filtered; i++) {
+                const DfaFilter& f = filters[rare[i].second];
+                ms.filtered[i] = (uint8_t)rare[i].second;
+                ms.regex_always &= ~(1u << rare[i].second);
+                for (uint32_t k = 0; k < mkb::BUCKET_CHARS; k++) {
+                    const uint64_t bitk = 1ull << (mkb::BUCKETS * k + mkb::BUCKETS - 1 - i);
+                    for (uint32_t v = 0; v < 64; v++)
+                        if ((f.values[k] >> v) & 1) ms.bucket[v] |= bitk;
+                    for (uint32_t e = 3; e <= k; e++)
+                        if (f.end[e]) ms.bucket_end |= bitk;
+                }
+            }
+        }
+    }
     uint32_t bit = 0;  // next free bit in the shift-and state
     auto place = [&](uint32_t i) -> int {
         const mkh25519::Needle& h = hosts[i];
@@ -609,9 +690,10 @@ static int pack_needles(mk_ctx* c, const mk_needle* needles, uint32_t n_needles,
         for (uint32_t i = 0; i < n_needles; i++)
             if (is_text(i) && hosts[i].len >= 4) (hosts[i].len == 4 ? four : five).push_back(i);
         const uint32_t all = (uint32_t)(four.size() + five.size());
-        uint32_t n4 = (uint32_t)((four.size() * mkb::BUCKETS + all / 2) / all);
+        const uint32_t n_text = mkb::BUCKETS - ms.n_filtered;
+        uint32_t n4 = (uint32_t)((four.size() * n_text + all / 2) / all);
         if (!four.empty()) n4 = std::max(n4, 1u);
-        if (!five.empty()) n4 = std::min(n4, mkb::BUCKETS - 1);
+        if (!five.empty()) n4 = std::min(n4, n_text - 1);
         auto fill = [&](std::vector<uint32_t>& list, uint32_t first, uint32_t count) {
             std::sort(list.begin(), list.end(), [&](uint32_t a, uint32_t b) { return hosts[a].bytes < hosts[b].bytes; });
             for (size_t q = 0; q < list.size(); q++) {
@@ -631,8 +713,10 @@ static int pack_needles(mk_ctx* c, const mk_needle* needles, uint32_t n_needles,
             }
         };
         if (gram4) {
+            ms.buckets = 1;
+            ms.text_buckets = (1u << n_text) - 1u;
             fill(four, 0, n4);
-            fill(five, n4, mkb::BUCKETS - n4);
+            fill(five, n4, n_text - n4);
         }
         for (uint32_t i = 0; gram4 && i < n_needles; i++) {
             if (!is_text(i) || hosts[i].len < 4) continue;

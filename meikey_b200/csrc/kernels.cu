@@ -229,6 +229,38 @@ __device__ __forceinline__ u32 tail_value(const u32 pk[8], int pos) {
 
 #define MK_SIGN_POS 42
 
+// Walks the next N (or fewer) DFAs of the set `need` and takes them out of it, side by side so that
+// their table lookups (shared memory when the launch staged the tables there, else global)
+// overlap; sets the bits of those that may match.
+template <int N>
+__device__ __forceinline__ void dfa_walks(const MatchSet& ms, const u32 pk[8], u32& need, u64 hit_words[2]) {
+    const uint16_t* t[N];
+    u32 r[N], s[N], alt[N];
+#pragma unroll
+    for (int q = 0; q < N; q++) {
+        r[q] = need ? (u32)__ffs((int)need) - 1u : r[0];
+        need &= need - 1u;
+        t[q] = reinterpret_cast<const uint16_t*>(ms.dfa[r[q]]);
+        s[q] = alt[q] = 1;
+    }
+#pragma unroll 1
+    for (int pos = 1; pos < 44; pos++) {
+        const u32 v = tail_value(pk, pos);
+#pragma unroll
+        for (int q = 0; q < N; q++) {
+            if (pos == MK_SIGN_POS) alt[q] = t[q][s[q] * 65u + (v | 2u)];
+            else if (pos > MK_SIGN_POS) alt[q] = t[q][alt[q] * 65u + v];
+            s[q] = t[q][s[q] * 65u + v];
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < N; q++) {
+        const bool ok = s[q] == 0 || t[q][s[q] * 65u + 64u] != 0 || alt[q] == 0 || t[q][alt[q] * 65u + 64u] != 0;
+        const u32 id = ms.regex_id[r[q]];
+        if (ok) hit_words[id >> 6] |= 1ull << (id & 63);
+    }
+}
+
 // Whether some text needle of a quick-compare job (MatchSet::quick) may match the key: 3 operations a
 // position instead of a table lookup and 6 (one needle on B200: 0.924 -> 0.929 G keys/s, incremental
 // 11.5 -> 12.6, a suffix 13.2).  The bit of position 42 that the x sign decides is left
@@ -259,15 +291,15 @@ __device__ __forceinline__ bool quick_match(const MatchSet& ms, const u32 pk[8])
 
 // Tests one key (y only; the character at position 42 is tried with both x signs, as
 // kernel.cu:1804-1875 does) and sets bit `id` of hit_words for every needle that may match.
-// `lane_masks` (null: none) is a table with every value's entry once per lane (value v of lane l at
-// v * 32 + l), so that every lane reads its own banks: for jobs whose text needles fit in 32 bits of
-// state the low half of mask word 0 (u32), for jobs with the 4-gram prefilter the bucket filter
-// (u64).  LIGHT: the job has neither the prefilter nor regex needles; their code costs the kernel
+// `lane_masks` and `lane_buckets` are tables with every value's entry once per lane (value v of lane
+// l at v * 32 + l), so that every lane reads its own banks: the low half of mask word 0 for jobs whose
+// text needles fit in 32 bits of state, and the bucket filter.  Called by all 32 lanes of a warp.
+// LIGHT: the job has neither the prefilter nor regex needles; their code costs the kernel
 // registers (spills) that a job of a few needles runs faster without (one needle on B200: 0.929 ->
 // 0.936 G keys/s, incremental 12.6 -> 12.9).
 template <bool LIGHT>
-__device__ __forceinline__ void match_key(const MatchSet& ms, const u64* lane_masks, const u32 pk[8],
-                                          u64 hit_words[2]) {
+__device__ __forceinline__ void match_key(const MatchSet& ms, const u32* lane_masks, const u64* lane_buckets,
+                                          const u32 pk[8], u64 hit_words[2]) {
     hit_words[0] = hit_words[1] = 0;
     u32 words = ms.sa_words;
     if (ms.quick && !quick_match(ms, pk)) {
@@ -281,8 +313,9 @@ __device__ __forceinline__ void match_key(const MatchSet& ms, const u64* lane_ma
     // are a cache line per lane, 32 a load, and bound the L1 tag stage (5200 of 46700 cycles a key
     // for 58 needles on B200), so the bucket filter in shared memory lets about one key in a hundred
     // through to them (58 needles; half of them at 128).
-    if (!LIGHT && ms.gram4) {
-        const u64* lm = lane_masks + (threadIdx.x & 31u);
+    u32 flags = ~0u;  // the buckets the key may hold something of
+    if (!LIGHT && ms.buckets) {
+        const u64* lm = lane_buckets + (threadIdx.x & 31u);
         u64 D = 0;
         u32 acc = 0;
 #pragma unroll
@@ -292,9 +325,13 @@ __device__ __forceinline__ void match_key(const MatchSet& ms, const u64* lane_ma
             D = (D << BUCKETS | ((1ull << BUCKETS) - 1)) & mk;
             acc |= (u32)(D >> 32);
         }
-        acc |= (u32)((D << BUCKETS & ms.bucket_end) >> 32);
+        D = D << BUCKETS & ms.bucket_end;
+        acc |= (u32)((D | (D << BUCKETS & ms.bucket_end)) >> 32);
+        flags = acc >> (BUCKETS * (BUCKET_CHARS - 1) - 32);
+    }
+    if (!LIGHT && ms.gram4) {
         u32 any = 0;
-        if (acc >> (BUCKETS * (BUCKET_CHARS - 1) - 32)) {
+        if (flags & ms.text_buckets) {
             u32 gw = value(1) << 12 | value(2) << 6 | value(3);
 #pragma unroll
             for (int p = 1; p + 3 < 44; p++) {
@@ -309,7 +346,7 @@ __device__ __forceinline__ void match_key(const MatchSet& ms, const u64* lane_ma
         if (!(any & 1u)) words = ms.short_words;
     }
     if (ms.narrow && words) {
-        const u32* lm = reinterpret_cast<const u32*>(lane_masks) + (threadIdx.x & 31u);
+        const u32* lm = lane_masks + (threadIdx.x & 31u);
         u32 D = 0, acc = 0;
         const u32 first = (u32)ms.first_bit[0], last = (u32)ms.last_bit[0];
 #pragma unroll
@@ -351,35 +388,16 @@ __device__ __forceinline__ void match_key(const MatchSet& ms, const u64* lane_ma
             }
         }
     }
-    // regex needles: eight DFA walks side by side, so that their table lookups (shared
-    // memory when the launch staged the tables there, else global) overlap
-    for (u32 r0 = 0; !LIGHT && r0 < ms.n_regex; r0 += 8) {
-        const uint16_t* t[8];
-        u32 s[8], alt[8];
-#pragma unroll
-        for (int q = 0; q < 8; q++) {
-            t[q] = reinterpret_cast<const uint16_t*>(ms.dfa[r0 + q < ms.n_regex ? r0 + q : r0]);
-            s[q] = alt[q] = 1;
-        }
-#pragma unroll 1
-        for (int pos = 1; pos < 44; pos++) {
-            const u32 v = value(pos);
-#pragma unroll
-            for (int q = 0; q < 8; q++) {
-                if (pos == MK_SIGN_POS) alt[q] = t[q][s[q] * 65u + (v | 2u)];
-                else if (pos > MK_SIGN_POS) alt[q] = t[q][alt[q] * 65u + v];
-                s[q] = t[q][s[q] * 65u + v];
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < 8; q++) {
-            const u32 r = r0 + q;
-            if (r >= ms.n_regex) break;
-            const bool ok = s[q] == 0 || t[q][s[q] * 65u + 64u] != 0 || alt[q] == 0 || t[q][alt[q] * 65u + 64u] != 0;
-            if (!ok) continue;
-            u32 id = ms.regex_id[r];
-            hit_words[id >> 6] |= 1ull << (id & 63);
-        }
+    // regex needles: the walks of those that the warp's keys cannot be told from by the buckets (8 DFAs
+    // of the multi-pattern workload on B200: 5 have buckets and are walked by every seventh warp, 0.850 ->
+    // 0.865 G keys/s alone and 0.807 -> 0.818 beside 64 text needles)
+    if (!LIGHT && ms.n_regex) {
+        u32 need = ms.regex_always;
+        for (u32 i = 0; i < ms.n_filtered; i++) need |= ((flags >> (BUCKETS - 1 - i)) & 1u) << ms.filtered[i];
+        need = __reduce_or_sync(0xffffffffu, need);
+        while (need)
+            if (__popc(need) > 4) dfa_walks<8>(ms, pk, need, hit_words);
+            else dfa_walks<4>(ms, pk, need, hit_words);
     }
 }
 
@@ -502,7 +520,7 @@ __device__ __forceinline__ int incr_key(int s) {
 // canonical y (sign bit 0), tests the needles and reports candidate hits (none when `valid` is
 // false: a run past the launch's last one).  INCR: slot j holds key incr_key(j).
 template <int KPT, bool INCR, bool LIGHT>
-__device__ __forceinline__ void backward(const KeyLaunch& L, const MatchSet& ms, const u64* lane_masks, u64 first,
+__device__ __forceinline__ void backward(const KeyLaunch& L, const MatchSet& ms, const u32* lane_masks, const u64* lane_buckets, u64 first,
                                          bool valid, const Batch<KPT>& b, fe inv, u32& sink) {
     // a key's two elements are loaded while the one before is tested (they have gone to the L2 cache
     // and further since the forward pass): on B200 incremental 13.0 -> 14.5, hashed 0.974 -> 0.980 G keys/s
@@ -518,7 +536,7 @@ __device__ __forceinline__ void backward(const KeyLaunch& L, const MatchSet& ms,
         den = den_next;
         sink ^= pk[7];
         u64 hw[2];
-        match_key<LIGHT>(ms, lane_masks, pk, hw);
+        match_key<LIGHT>(ms, lane_masks, lane_buckets, pk, hw);
         if (!valid) hw[0] = hw[1] = 0;
         const bool any = (hw[0] | hw[1]) != 0;
         // warp ballot: the (rare) warps with a hit compact their records into the ring
@@ -702,7 +720,8 @@ __global__ void __launch_bounds__(BLOCK, 512 / BLOCK) k_search(const KeyLaunch L
     uint4* stab = reinterpret_cast<uint4*>(scratch + CT);  // STAB: the table in place of the slots
     __shared__ CombGeom g;
     __shared__ MatchSet ms;
-    __shared__ u64 lane_masks[64 * 32];  // see match_key
+    __shared__ u32 lane_masks[64 * 32];  // see match_key
+    __shared__ u64 lane_buckets[LIGHT ? 1 : 64 * 32];
     __shared__ u32 key[8];
     __shared__ mkh::CounterMid mid;
     __shared__ volatile u64 stop_iter;
@@ -751,9 +770,9 @@ __global__ void __launch_bounds__(BLOCK, 512 / BLOCK) k_search(const KeyLaunch L
         }
     }
     if (ms.narrow)
-        for (u32 i = tid; i < 64u * 32u; i += BLOCK) reinterpret_cast<u32*>(lane_masks)[i] = (u32)ms.mask[0][i >> 5];
-    else if (!LIGHT && ms.gram4)
-        for (u32 i = tid; i < 64u * 32u; i += BLOCK) lane_masks[i] = ms.bucket[i >> 5];
+        for (u32 i = tid; i < 64u * 32u; i += BLOCK) lane_masks[i] = (u32)ms.mask[0][i >> 5];
+    if (!LIGHT && ms.buckets)
+        for (u32 i = tid; i < 64u * 32u; i += BLOCK) lane_buckets[i] = ms.bucket[i >> 5];
     if (INCR && tid < (u32)INCR_STEPS) step_to_yx(steps, tid);
     if (tid == 0 && L.seed_src == 1) mid = mkh::counter_mid(key);
     __syncthreads();
@@ -815,7 +834,7 @@ __global__ void __launch_bounds__(BLOCK, 512 / BLOCK) k_search(const KeyLaunch L
             const int b = p & 1;
             if (!inverts(p)) bar_sync(3 + b, BLOCK);
             if (chunk_of(p) - (tid & 31u) < L.chunks)
-                backward<KPT, INCR, LIGHT>(L, ms, lane_masks, first_of(p), chunk_of(p) < L.chunks, batch[b],
+                backward<KPT, INCR, LIGHT>(L, ms, lane_masks, lane_buckets, first_of(p), chunk_of(p) < L.chunks, batch[b],
                                            prod[b][tid], sink);
             if (it >= iters || it >= stop_iter) break;
         }

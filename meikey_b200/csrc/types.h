@@ -58,11 +58,17 @@ struct MatchSet {
     uint32_t quick;               // 1: on
     uint32_t n_quick_contains, n_quick_suffix;
     uint32_t quick_value[6], quick_mask[6];  // the contains-needles, then from QUICK_CONTAINS the suffixes
-    // bucket filter of the needles gram4 holds: bit 12·k + b of bucket[v] is set when some needle of
-    // bucket b takes value v as its character k (k < 5; of a 4-character needle every value as its
-    // fifth, and bucket_end has that bit for the end of the key)
+    // bucket filter: bit 12·k + b of bucket[v] is set when something in bucket b takes value v as its
+    // character k (k < 5): a needle that gram4 holds, or a regex on its last way from its start state to
+    // a match.  What may end with the key after k < 5 characters has bits 12·k + b and up in
+    // bucket_end (a 4-character needle takes every value as its fifth)
+    uint32_t buckets;             // 1: on
+    uint32_t text_buckets;        // the buckets of needles
     uint64_t bucket[64];
     uint64_t bucket_end;
+    uint32_t regex_always;        // the regex needles without a bucket: every key walks their DFAs
+    uint32_t n_filtered;          // regex needles with one: filtered[i] has bucket BUCKETS - 1 - i
+    uint8_t filtered[16];
     // regex needles
     const uint8_t* dfa[16];
     uint32_t dfa_states[16];
@@ -75,6 +81,7 @@ struct MatchSet {
 
 constexpr uint32_t QUICK_CONTAINS = 2, QUICK_SUFFIX = 4;
 constexpr uint32_t BUCKETS = 12, BUCKET_CHARS = 5;
+constexpr uint32_t REGEX_BUCKETS = 6;  // at most, beside text needles in the filter
 constexpr uint32_t GRAM4_WORDS = 1u << 19;  // 2^24 bits
 constexpr uint32_t GRAM4_MIN_NEEDLES = 8;   // long text needles from which a job uses the prefilter
 

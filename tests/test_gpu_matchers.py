@@ -66,3 +66,26 @@ def test_bucket_filter(gpu_ctx, oracle, tails, count, lo, hi):
     if count == 9:
         needles.append(mk.Needle.contains(tails[200][5:8]))  # scanned for every key, beside the filter
     check(gpu_ctx, oracle, needles)
+
+
+REGEXES = ["ab[0-9]", "(ab|cd|ef)[+/]", "(?:xyz|XY|q[a-c])z$", "aa?b[xy]c?d$", "z[0-9]{2}z", "(?:a[ab]b|bab)[cd]", "qq+w",
+           "(?i)hij", "[a-f][0-9]{2}$", "(?i)k.l.m", "zz$", "^K..x", "(ab){2}", "/[+]/", "[xyz]{5}", "(?i)[a-c]{4}$"]
+
+
+@pytest.mark.parametrize("texts", [0, 1, 20])
+@pytest.mark.parametrize("which", [slice(0, 16), slice(0, 5), slice(5, 10), slice(9, 11)])
+def test_regexes_together_find_what_each_finds_alone(gpu_ctx, tails, which, texts):
+    """A job of one regex walks its DFA for every key; several take the bucket filter."""
+    def hits_of(needles):
+        with gpu_ctx.job(KEY, mk.SEED_COUNTER, needles) as job:
+            job.launch(BASE, 1)
+            hits, total = job.hits(cap=1 << 18)
+        assert total == len(hits)
+        return hits
+
+    rx = [mk.Needle.regex(r) for r in REGEXES[which]]
+    text = [mk.Needle.contains(tails[q][3:8]) for q in range(texts)]
+    got = hits_of(rx + text)
+    for k, n in enumerate(rx):
+        assert [i for i, q in got if q == k] == [i for i, _ in hits_of([n])], REGEXES[which][k]
+    assert {q for _, q in got} >= set(range(len(rx), len(rx) + texts))
