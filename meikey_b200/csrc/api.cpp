@@ -652,6 +652,7 @@ static int pack_needles(mk_ctx* c, const mk_needle* needles, uint32_t n_needles,
         }
     }
     uint32_t bit = 0;  // next free bit in the shift-and state
+    uint32_t short_bits = 0;  // with the prefilter: bits of the needles shorter than 4
     auto place = [&](uint32_t i) -> int {
         const mkh25519::Needle& h = hosts[i];
         const uint32_t len = h.len;
@@ -679,6 +680,7 @@ static int pack_needles(mk_ctx* c, const mk_needle* needles, uint32_t n_needles,
         for (uint32_t i = 0; i < n_needles; i++)
             if (is_text(i) && hosts[i].len < 4)
                 if (int st = place(i)) return st;
+        short_bits = bit;
         bit = (bit + 63) & ~63u;
         ms.short_words = bit / 64;
         for (uint32_t i = 0; i < n_needles; i++)
@@ -747,7 +749,7 @@ static int pack_needles(mk_ctx* c, const mk_needle* needles, uint32_t n_needles,
     }
     ms.sa_words = ms.n_text ? (bit + 63) / 64 : 0;
     if (!prefilter) ms.short_words = ms.sa_words;
-    ms.narrow = ms.n_text && !prefilter && bit <= 32;
+    ms.narrow = prefilter ? short_bits && short_bits <= 32 : ms.n_text && bit <= 32;
     // quick compare (see MatchSet)
     ms.quick = ms.n_text > 0;
     for (uint32_t i = 0; i < n_needles && ms.quick; i++) {

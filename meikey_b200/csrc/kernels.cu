@@ -345,6 +345,7 @@ __device__ __forceinline__ void match_key(const MatchSet& ms, const u32* lane_ma
         }
         if (!(any & 1u)) words = ms.short_words;
     }
+    u32 scanned = 0;
     if (ms.narrow && words) {
         const u32* lm = lane_masks + (threadIdx.x & 31u);
         u32 D = 0, acc = 0;
@@ -359,14 +360,14 @@ __device__ __forceinline__ void match_key(const MatchSet& ms, const u32* lane_ma
         acc |= D & (u32)ms.suffix_bit[0];
         for (u32 t = 0; acc && t < ms.n_text; t++) {
             const u32 b = ms.text_last[t];
-            if ((acc >> b) & 1u) {
+            if (b < 32u && ((acc >> b) & 1u)) {
                 const u32 id = ms.text_id[t];
                 hit_words[id >> 6] |= 1ull << (id & 63);
             }
         }
-        words = 0;
+        scanned = 1;
     }
-    for (u32 wi = 0; wi < words; wi++) {
+    for (u32 wi = scanned; wi < words; wi++) {
         u64 D = 0, acc = 0;
         u64 first = ms.first_bit[wi], last = ms.last_bit[wi];
 #pragma unroll

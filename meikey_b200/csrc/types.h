@@ -41,7 +41,8 @@ struct MatchSet {
     uint32_t sa_words;            // words of shift-and state in use
     uint32_t short_words;         // with gram4: the leading words, holding the needles shorter than 4
                                   // characters, that every key scans; the rest only when gram4 fires
-    uint32_t narrow;              // 1: the text needles fit in 32 bits of state (word 0, low half)
+    uint32_t narrow;              // 1: word 0 has its needles in its low 32 bits (all text needles, or with
+                                  // gram4 the short ones)
     // shift-and: per word and value v (0..63) the bits of needle positions accepting v.  Word
     // major, so that the 32 lanes' reads of one word at different values spread over the
     // shared-memory banks (value major, a row of 64 bytes put every lane on bank 0 or 16)
