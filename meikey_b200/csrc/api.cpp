@@ -317,6 +317,10 @@ int mk_ctx_create(int device, const mk_options* options, mk_ctx** out) try {
         MK_CUDA(c, cudaMemPoolCreate(&c->pool, &pp));
         uint64_t keep = ~0ull;  // freed blocks stay in the pool until the context goes
         MK_CUDA(c, cudaMemPoolSetAttribute(c->pool, cudaMemPoolAttrReleaseThreshold, &keep));
+        // the pool's first memory is mapped now, not in the first short call
+        void* first = nullptr;
+        MK_CUDA(c, cudaMallocFromPoolAsync(&first, 2u << 20, c->pool, c->stream));
+        MK_CUDA(c, cudaFreeAsync(first, c->stream));
     }
     for (auto& ev : c->ev) MK_CUDA(c, cudaEventCreate(&ev));
     cudaDeviceProp prop;
