@@ -842,12 +842,10 @@ def main():
     ap.add_argument("--ref-step-seconds", type=float, default=2.0, help="reference arm: seconds per step")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--inverter-rotates", action=argparse.BooleanOptionalAction, default=None,
-                    help="every warp derives keys and the inversion rotates over four warps "
-                         "(mk_options.inverter_rotates; default: on for the multi-pattern workload, "
-                         "the layout mk_autotune_job picks for it, off otherwise)")
+                    help="spans counted in all threads of a CTA (mk_options.inverter_rotates; default: on "
+                         "for the multi-pattern workload, off otherwise)")
     ap.add_argument("--hash-interleave", type=int, default=0, choices=[0, 1],
-                    help="1: hash the next iteration's seeds inside the comb rows (mk_options.hash_interleave; "
-                         "ChaCha20 and counter workloads, 12 rows)")
+                    help="1: mk_options.hash_interleave (accepted, without effect; 12 rows)")
     ap.add_argument("--autotune", action="store_true",
                     help="instead of the benchmark: mk_autotune_job over the tuning space on the workload's job "
                          "(comb windows, keys per thread, layouts, inversion batches); prints every candidate")

@@ -470,7 +470,6 @@ int mk_derive(mk_ctx* c, const uint8_t key[32], int seed_source, uint64_t first,
         L.geom = c->geom;
         for (int i = 0; i < 8; i++) L.key[i] = (uint32_t)key[4 * i] | (uint32_t)key[4 * i + 1] << 8 | (uint32_t)key[4 * i + 2] << 16 | (uint32_t)key[4 * i + 3] << 24;
         L.seed_src = (uint32_t)seed_source;
-        L.iters = 1;
         L.base = first + done;
         L.out = d_out;
         L.count = cnt;
@@ -506,7 +505,6 @@ int mk_derive_noalloc(mk_ctx* c, const uint8_t key[32], int seed_source, uint64_
     for (int i = 0; i < 8; i++)
         L.key[i] = (uint32_t)key[4 * i] | (uint32_t)key[4 * i + 1] << 8 | (uint32_t)key[4 * i + 2] << 16 | (uint32_t)key[4 * i + 3] << 24;
     L.seed_src = (uint32_t)seed_source;
-    L.iters = 1;
     L.base = first;
     L.out = staging;
     L.count = n;
@@ -938,7 +936,6 @@ static mkb::KeyLaunch search_params(const mk_job* j, uint64_t base, uint32_t ite
     for (int i = 0; i < 8; i++)
         L.key[i] = (uint32_t)j->key[4 * i] | (uint32_t)j->key[4 * i + 1] << 8 | (uint32_t)j->key[4 * i + 2] << 16 | (uint32_t)j->key[4 * i + 3] << 24;
     L.seed_src = (uint32_t)j->source;
-    L.iters = iters;
     const bool incr = j->source == MK_SEED_INCREMENTAL;
     L.chunks = c->info.keys_per_iter / mkb::search_kernel_keys(incr, c->kpt, c->table_smem) * iters;
     L.base = base;

@@ -2,14 +2,14 @@
 //
 //   k_build_table  fills the comb table in HBM: entry (row, k) = k·2^(off_row)·8B
 //                  (+ 2^254·B on the top row), affine (y+x, y-x, 2dxy, -2dxy), row 0 holds ±2xy.
-//   k_keys<…>      one fused pass per key: seed (ChaCha20 / counter) -> SHA-512 -> clamp
+//   k_search<…>    one fused pass per key: seed (ChaCha20 / counter) -> SHA-512 -> clamp
 //                  -> comb multiply from the table -> y as a fraction -> per-thread
 //                  Montgomery batch + per-CTA pooled inversion -> canonical y -> base64
-//                  values -> shift-and / DFA match -> warp-ballot hit compaction.
-//                  The DERIVE instantiation also computes x and writes full public keys.
+//                  values -> compare / shift-and / DFA match -> warp-ballot hit compaction.
+//   k_derive<…>    full public keys (x too), an inversion per thread.
 //
 // Reference behaviour: src/service/gpu/kernel.cu:1898-2069 (meikey_search / meikey_derive).
-// The index layout matches it: index = base + ((it·nthreads + gid)·KPT + j).
+// A launch covers the same consecutive indices from its base.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -521,8 +521,9 @@ __device__ __forceinline__ int incr_key(int s) {
 // canonical y (sign bit 0), tests the needles and reports candidate hits (none when `valid` is
 // false: a run past the launch's last one).  INCR: slot j holds key incr_key(j).
 template <int KPT, bool INCR, bool LIGHT>
-__device__ __forceinline__ void backward(const KeyLaunch& L, const MatchSet& ms, const u32* lane_masks, const u64* lane_buckets, u64 first,
-                                         bool valid, const Batch<KPT>& b, fe inv, u32& sink) {
+__device__ __forceinline__ void backward(const KeyLaunch& L, const MatchSet& ms, const u32* lane_masks,
+                                         const u64* lane_buckets, u64 first, bool valid, const Batch<KPT>& b, fe inv,
+                                         u32& sink) {
     // a key's two elements are loaded while the one before is tested (they have gone to the L2 cache
     // and further since the forward pass): on B200 incremental 13.0 -> 14.5, hashed 0.974 -> 0.980 G keys/s
     fe a = b.a[KPT - 1], den = b.den[KPT - 1];
@@ -704,7 +705,7 @@ __device__ __forceinline__ void incr_fracs(const ge& Q, const uint4* steps, Batc
 // waits, the others arrive; inverses of buffer b ready (3 + b): the inverting warp arrives,
 // the others wait.  Stop requests (host stop word, or a hit with stop_on_hit) are read by
 // the inverting warp and take effect two iterations later, at a point every warp agrees on
-// (tests/test_pipeline_protocol.py model-checks both forms).
+// (tests/test_rotating_duty.py and tests/test_pipeline_protocol.py model-check the two forms).
 // INCR: the incremental source.  A compute thread keeps the point Q of its middle index (key
 // KPT/2) in the current iteration; its keys are Q ± d·B from the step table, and Q advances by
 // keys_per_iter·B (one mixed addition) per iteration.  No comb table is read.

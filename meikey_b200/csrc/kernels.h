@@ -18,7 +18,6 @@ struct KeyLaunch {
     CombGeom geom;
     uint32_t key[8];
     uint32_t seed_src;     // 0 ChaCha20, 1 counter, 2 incremental
-    uint32_t iters;
     uint64_t chunks;       // search: runs of search_kernel_keys consecutive indices from base
     uint64_t base;
     // search
