@@ -5,6 +5,7 @@
 ``Engine::launch``.  Everything runs through the C ABI of libmeikey_b200.so.
 """
 import ctypes
+import sys
 from dataclasses import dataclass
 from typing import List, Optional, Sequence, Tuple
 
@@ -119,9 +120,15 @@ _bytes_from_size.argtypes = [ctypes.c_char_p, ctypes.c_ssize_t]
 
 def _new_bytes(n: int) -> bytes:
     """A new bytes object of n bytes for the library to fill before anyone else sees it (what
-    PyBytes_FromStringAndSize without a string is for); not cleared first and not copied after."""
+    PyBytes_FromStringAndSize without a string is for); not cleared first and not copied after.
+    Sizes are refused as ctypes.create_string_buffer refuses them: ctypes cuts an argument to 64
+    bits, so 2^64 would give an object of no bytes."""
+    if not isinstance(n, int):
+        raise TypeError(n)
+    if not -sys.maxsize - 1 <= n <= sys.maxsize:
+        raise OverflowError("cannot fit 'int' into an index-sized integer")
     if n < 0:
-        raise ValueError("Array length must be >= 0")
+        raise ValueError(f"Array length must be >= 0, not {n}")
     return _bytes_from_size(None, n)
 
 
