@@ -113,9 +113,9 @@ def _check(lib, ctx_ptr, status: int):
         raise GpuError(status, buf.value.decode(errors="replace"))
 
 
-_bytes_from_size = ctypes.pythonapi.PyBytes_FromStringAndSize
-_bytes_from_size.restype = ctypes.py_object
-_bytes_from_size.argtypes = [ctypes.c_char_p, ctypes.c_ssize_t]
+# a prototype of its own: the attributes of ctypes.pythonapi's functions are shared by the process
+_bytes_from_size = ctypes.PYFUNCTYPE(ctypes.py_object, ctypes.c_char_p, ctypes.c_ssize_t)(
+    ("PyBytes_FromStringAndSize", ctypes.pythonapi))
 
 
 def _new_bytes(n: int) -> bytes:

@@ -18,3 +18,13 @@ def test_sizes_are_refused_as_by_create_string_buffer(n):
 @pytest.mark.parametrize("n", [0, 1, 32, 65536])
 def test_sizes_are_exact(n):
     assert len(engine._new_bytes(n)) == n
+
+
+def test_other_users_of_the_python_api_are_left_alone(monkeypatch):
+    """ctypes.pythonapi's functions belong to the whole process: another module may declare
+    PyBytes_FromStringAndSize as it likes, and finds what it declared."""
+    shared = ctypes.pythonapi.PyBytes_FromStringAndSize
+    monkeypatch.setattr(shared, "restype", ctypes.c_void_p)
+    monkeypatch.setattr(shared, "argtypes", [ctypes.c_void_p, ctypes.c_size_t])
+    got = engine._new_bytes(32)
+    assert type(got) is bytes and len(got) == 32
