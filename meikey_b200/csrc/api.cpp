@@ -430,10 +430,14 @@ static int check_source(mk_ctx* c, const uint8_t key[32], int seed_source) {
 
 // Makes the pages of a large output buffer present, on several host threads while the GPU works:
 // the buffer is usually fresh memory, and left to the copy its page faults come one after another
-// on one thread.  Every byte is written by the copy afterwards.
+// on one thread.  Every byte is written by the copy afterwards.  Memory that CUDA knows is left
+// alone: pinned pages are present, and the host cannot write to device memory, which the copy takes too.
 static void touch_pages(uint8_t* out, size_t bytes) {
     const size_t MIN = 8u << 20, PAGE = 4096;
     if (bytes < MIN) return;
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, out) != cudaSuccess) cudaGetLastError();
+    else if (at.type != cudaMemoryTypeUnregistered) return;
     const uint32_t threads = std::min(8u, std::max(1u, std::thread::hardware_concurrency()));
     auto work = [&](uint32_t t) {
         const size_t lo = bytes / threads * t, hi = t + 1 == threads ? bytes : bytes / threads * (t + 1);
