@@ -355,7 +355,9 @@ MK_API int mk_ctx_record(mk_ctx* ctx, int slot);
 MK_API int mk_ctx_elapsed(mk_ctx* ctx, int from_slot, int to_slot, float* ms);
 
 /* meikey_derive (src/service/gpu/kernel.cu:2062-2069, src/service/gpu.rs:783-804):
- * n full public keys (x sign included) of indices first..first+n-1 into host `out` (32·n bytes). */
+ * n full public keys (x sign included) of indices first..first+n-1 into host `out` (32·n bytes).
+ * The device memory for the keys, 32·n bytes and at most 128 MB, stays with the context for later
+ * calls and jobs until mk_ctx_destroy. */
 MK_API int mk_derive(mk_ctx* ctx, const uint8_t key[32], int seed_source, uint64_t first, uint64_t n, uint8_t* out);
 
 /* mk_derive that allocates nothing.  This entry point has no counterpart in the reference.

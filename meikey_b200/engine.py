@@ -163,7 +163,8 @@ class Context:
         return int(self._lib.mk_keys_per_iter(self._ptr))
 
     def derive(self, key: bytes, source: int, first: int, n: int) -> bytes:
-        """n full public keys (32 bytes each) of indices first..first+n-1."""
+        """n full public keys (32 bytes each) of indices first..first+n-1.  The device memory for
+        them (at most 128 MB) stays with the context for later calls."""
         out = _new_bytes(32 * n)
         _check(self._lib, self._ptr, self._lib.mk_derive(self._ptr, bytes(key), source, first, n, out))
         return out
