@@ -188,27 +188,6 @@ void set_incremental(const mk_ctx* c, const uint8_t s0[32], uint64_t base, mkb::
     L.incr = c->incr;
 }
 
-int self_check(mk_ctx* c) {
-    // every seed source, an odd first index (seed from the second half of a block)
-    const uint64_t n = 257;
-    std::vector<uint8_t> got(32 * n);
-    for (int src = 0; src < 3; src++) {
-        uint8_t key[32];
-        for (int i = 0; i < 32; i++) key[i] = (uint8_t)(0x5a ^ (i * 37 + src * 101));
-        key[31] &= 0x7f;  // incremental scalars start below 2^255
-        uint64_t first = 0x123456789abull | 1;
-        int st = mk_derive(c, key, src, first, n, got.data());
-        if (st) return st;
-        for (uint64_t i = 0; i < n; i += (i < 8 ? 1 : 31)) {
-            uint8_t pk[32];
-            host_public_key(key, src, first + i, pk);
-            if (memcmp(pk, &got[32 * i], 32) != 0)
-                return fail(c, MK_ERR_SELF_CHECK, "GPU public keys differ from the host derivation");
-        }
-    }
-    return MK_OK;
-}
-
 }  // namespace
 
 namespace mkjobs {
@@ -249,6 +228,8 @@ int mk_last_error(const mk_ctx* ctx, char* buf, size_t size) {
     snprintf(buf, size, "%s", s);
     return MK_OK;
 }
+
+static int self_check(mk_ctx* c);
 
 int mk_ctx_create(int device, const mk_options* options, mk_ctx** out) try {
     if (!out) return MK_ERR_BAD_ARG;
@@ -455,7 +436,9 @@ static void touch_pages(uint8_t* out, size_t bytes) {
     for (auto& t : pool) t.join();
 }
 
-int mk_derive(mk_ctx* c, const uint8_t key[32], int seed_source, uint64_t first, uint64_t n, uint8_t* out) try {
+// mk_derive with a number of keys per thread (0: launch_derive's own choice).
+static int derive(mk_ctx* c, const uint8_t key[32], int seed_source, uint64_t first, uint64_t n, uint32_t keys,
+                  uint8_t* out) {
     if (!c || !key || (!out && n)) return fail(c, MK_ERR_BAD_ARG, "bad argument");
     if (int st = check_source(c, key, seed_source)) return st;
     if (seed_source == MK_SEED_INCREMENTAL && n != 0 && n - 1 > ~0ull - first)  // last index first + n - 1
@@ -481,7 +464,7 @@ int mk_derive(mk_ctx* c, const uint8_t key[32], int seed_source, uint64_t first,
         L.out = d_out;
         L.count = cnt;
         if (seed_source == MK_SEED_INCREMENTAL) set_incremental(c, key, L.base, L);
-        cudaError_t e = mkb::launch_derive(L, c->info.sms, c->stream);
+        cudaError_t e = mkb::launch_derive(L, c->info.sms, keys, c->stream);
         if (e == cudaSuccess) touch_pages(out + 32 * done, cnt * 32);
         if (e == cudaSuccess) e = cudaMemcpyAsync(out + 32 * done, d_out, cnt * 32, cudaMemcpyDeviceToHost, c->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
@@ -492,7 +475,37 @@ int mk_derive(mk_ctx* c, const uint8_t key[32], int seed_source, uint64_t first,
     }
     pool_free(c, d_out);
     return MK_OK;
+}
+
+int mk_derive(mk_ctx* c, const uint8_t key[32], int seed_source, uint64_t first, uint64_t n, uint8_t* out) try {
+    return derive(c, key, seed_source, first, n, 0, out);
 } MK_ABI_CATCH(c ? &c->err : nullptr)
+
+// Derived keys of every seed source with every number of keys per thread: each is a kernel of its own,
+// and more than one key chains the denominators, takes both halves of a ChaCha20 block and all entries
+// of the step table.  One key per thread is compared with the host derivation (55 us a key, so some of
+// them), the others with it.
+static int self_check(mk_ctx* c) {
+    const uint64_t n = 257, first = 0x123456789abull | 1;  // an odd first index: the second half of a block
+    std::vector<uint8_t> one(32 * n), got(32 * n);
+    for (int src = 0; src < 3; src++) {
+        uint8_t key[32];
+        for (int i = 0; i < 32; i++) key[i] = (uint8_t)(0x5a ^ (i * 37 + src * 101));
+        key[31] &= 0x7f;  // incremental scalars start below 2^255
+        if (int st = derive(c, key, src, first, n, 1, one.data())) return st;
+        for (uint64_t i = 0; i < n; i += (i < 8 ? 1 : 31)) {
+            uint8_t pk[32];
+            host_public_key(key, src, first + i, pk);
+            if (memcmp(pk, &one[32 * i], 32) != 0)
+                return fail(c, MK_ERR_SELF_CHECK, "GPU public keys differ from the host derivation");
+        }
+        for (uint32_t keys = 2; keys <= mkb::DERIVE_MAX_KEYS; keys *= 2) {
+            if (int st = derive(c, key, src, first, n, keys, got.data())) return st;
+            if (got != one) return fail(c, MK_ERR_SELF_CHECK, "GPU public keys depend on the keys per thread");
+        }
+    }
+    return MK_OK;
+}
 
 // Same keys as mk_derive, with the device output staged in the library's fixed device
 // array instead of a cudaMalloc'd buffer: this call allocates nothing.  Every slot of the
@@ -515,7 +528,7 @@ int mk_derive_noalloc(mk_ctx* c, const uint8_t key[32], int seed_source, uint64_
     L.base = first;
     L.out = staging;
     L.count = n;
-    MK_CUDA(c, mkb::launch_derive(L, c->info.sms, c->stream));
+    MK_CUDA(c, mkb::launch_derive(L, c->info.sms, 0, c->stream));
     MK_CUDA(c, cudaMemcpyAsync(out, staging, n * 32, cudaMemcpyDeviceToHost, c->stream));
     MK_CUDA(c, cudaStreamSynchronize(c->stream));
     return MK_OK;

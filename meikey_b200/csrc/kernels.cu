@@ -856,7 +856,6 @@ __global__ void __launch_bounds__(BLOCK, 512 / BLOCK) k_search(const KeyLaunch L
 }
 
 constexpr int DERIVE_BLOCK = 128;
-constexpr uint32_t DERIVE_MAX_KEYS = 16;
 
 // Derive kernel: full public keys (x sign included) of indices base .. base+count-1, KPT
 // consecutive ones per thread, with one inversion of its 2·KPT denominators per thread.  INCR: the
@@ -1007,16 +1006,17 @@ cudaError_t search_occupancy(uint32_t kpt, uint32_t block, uint32_t table_smem, 
 // most DERIVE_MAX_KEYS.  On B200 a call of 257 keys takes 72 us (61 us in the kernel) where 16 keys
 // behind each other in a thread took 1286; 4099 keys 100 us against 726 at 8; 2^20 keys are 1.4 ms in
 // the kernel, at 16 keys per thread.
-cudaError_t launch_derive(const KeyLaunch& L, uint32_t sms, cudaStream_t st) {
+cudaError_t launch_derive(const KeyLaunch& L, uint32_t sms, uint32_t keys, cudaStream_t st) {
     const bool incr = L.seed_src == SEED_INCREMENTAL;
     if (incr && !L.incr) return cudaErrorInvalidValue;
-    uint32_t k = 1;
-    while (k < DERIVE_MAX_KEYS && (L.count + k - 1) / k > (uint64_t)sms * 512) k *= 2;
+    uint32_t k = keys ? keys : 1;
+    while (!keys && k < DERIVE_MAX_KEYS && (L.count + k - 1) / k > (uint64_t)sms * 512) k *= 2;
     const void* f = nullptr;
 #define MK_FN(K) \
     if (k == K) f = incr ? (const void*)k_derive<K, true> : (const void*)k_derive<K, false>;
     MK_FN(1) MK_FN(2) MK_FN(4) MK_FN(8) MK_FN(16)
 #undef MK_FN
+    if (!f) return cudaErrorInvalidValue;
     const size_t dyn = incr ? 0 : DERIVE_BLOCK * sizeof(EntrySlot);
     cudaError_t e = prepare(f, dyn);
     if (e != cudaSuccess) return e;

@@ -80,8 +80,10 @@ constexpr int INCR_STEPS = 16;    // j·B for j = 0 .. keys per thread - 1
 constexpr int INCR_ENTRIES = INCR_WINDOWS * 16 + INCR_STEPS;
 
 cudaError_t launch_search(const KeyLaunch& L, uint32_t kpt, uint32_t block, uint32_t grid, cudaStream_t st);
-// Public keys of L.base .. L.base + L.count - 1 (count > 0) into L.out.
-cudaError_t launch_derive(const KeyLaunch& L, uint32_t sms, cudaStream_t st);
+constexpr uint32_t DERIVE_MAX_KEYS = 16;
+// Public keys of L.base .. L.base + L.count - 1 (count > 0) into L.out.  `keys` per thread: 1, 2, 4, 8 or
+// DERIVE_MAX_KEYS; 0 takes the fewest that one wave holds.
+cudaError_t launch_derive(const KeyLaunch& L, uint32_t sms, uint32_t keys, cudaStream_t st);
 // Field multiplications per second in radix 2^32 (the search kernel's), radix 2^25.5 and
 // radix 2^51 in FP64; *radix51_exact tells whether radix-2^51 chains matched radix 2^32.
 cudaError_t measure_field_mul_rates(int sms, cudaStream_t st, double* radix32_per_s, double* radix26_per_s,
