@@ -91,7 +91,7 @@ typedef struct mk_options {
                                  keys_per_thread x counted threads / pools, for pools a divisor of the
                                  counted threads (480; 512 with inverter_rotates; 352 with hash_warps) of
                                  at most 32, e.g. 256 = 8 x 480 / 15; searches take the pool count that
-                                 comes nearest to it (256 = 8 x 512 / 16).  0: 32 pools (keys_per_thread x 15,
+                                 comes nearest to it (256 = 8 x 512 / 16), 4 at least.  0: 32 pools (keys_per_thread x 15,
                                  x 16 with inverter_rotates, x 11 with hash_warps); else
                                  MK_ERR_OUT_OF_RANGE when no pool count gives it */
     uint32_t table_in_smem;   /* 1: every search CTA copies the comb table into shared memory and reads its

@@ -939,12 +939,15 @@ static uint32_t dfa_smem_bytes(const mk_job* j) {
 }
 
 // Field inversions per CTA and iteration of the kernel that serves a context's searches of a
-// source: the pools whose batches come nearest to the keys per inversion asked for.
+// source: the pools whose batches come nearest to the keys per inversion asked for, at least 4.  Fewer
+// make the inverting warp's chain (3 products per thread of a pool) longer than the other warps' work:
+// 33 M hashed candidates on B200 at 1, 2, 4 and 8 pools take 57, 42, 39 and 36 ms, where 16 keys per thread
+// and one pool, while searches still ran as many keys per thread as the context says, took 47.
 static uint32_t search_pools(const mk_ctx* c, bool incr) {
     if (!c->inv_batch) return 32;
     const uint32_t keys = mkb::search_kernel_threads(incr, c->block, c->table_smem) *
                           mkb::search_kernel_keys(incr, c->kpt, c->table_smem);
-    return std::min(32u, std::max(1u, (keys + c->inv_batch / 2) / c->inv_batch));
+    return std::min(32u, std::max(4u, (keys + c->inv_batch / 2) / c->inv_batch));
 }
 
 // Kernel parameters of one search launch of a job.
