@@ -556,38 +556,43 @@ static DfaFilter dfa_filter(const uint8_t* table, uint32_t states) {
     DfaFilter f{};
     f.chance = 1.0;
     auto at = [&](uint32_t s, uint32_t v) {
-        const size_t i = ((size_t)s * 65 + v) * 2;
-        return (uint32_t)table[i] | (uint32_t)table[i + 1] << 8;
+        uint16_t t;  // little-endian, as the host is
+        memcpy(&t, table + ((size_t)s * 65 + v) * 2, 2);
+        return (uint32_t)t;
     };
     auto accepts = [&](uint32_t s) { return s == 0 || at(s, 64) != 0; };  // at the end of the key
     if (states < 2 || accepts(1)) return f;
-    // states from which the key can still match
+    // states from which the key can still match; from the last state down, the order in which the
+    // library's tables settle in one pass
     std::vector<char> live(states);
     for (uint32_t s = 0; s < states; s++) live[s] = accepts(s);
     for (bool more = true; more;) {
         more = false;
-        for (uint32_t s = 0; s < states; s++)
-            for (uint32_t v = 0; v < 64 && !live[s]; v++)
-                if (live[at(s, v)]) live[s] = more = true;
+        for (uint32_t s = states; s-- > 0;)
+            if (!live[s]) {
+                for (uint32_t v = 0; v < 64; v++) live[s] |= live[at(s, v)];
+                more = more || live[s];
+            }
     }
-    std::vector<char> now(states, 0), next(states);
-    now[1] = 1;
+    live[1] = 0;  // the last way from the start state does not come back to it
+    std::vector<uint32_t> now(1, 1u), next;
+    std::vector<uint32_t> seen(states, 0u);  // the last character a state was listed for
     double chance = 43.0;
     for (uint32_t k = 0; k < mkb::BUCKET_CHARS; k++) {
-        std::fill(next.begin(), next.end(), 0);
-        int n = 0;
-        for (uint32_t v = 0; v < 64; v++) {
-            bool any = false;
-            for (uint32_t s = 0; s < states; s++)
-                if (now[s] && at(s, v) != 1 && live[at(s, v)]) next[at(s, v)] = any = true;
-            if (any) {
-                f.values[k] |= 1ull << v;
-                n++;
+        next.clear();
+        for (uint32_t s : now) {
+            uint64_t on = 0;  // the values that lead on from s
+            for (uint32_t v = 0; v < 64; v++) on |= (uint64_t)live[at(s, v)] << v;
+            f.values[k] |= on;
+            for (; on; on &= on - 1) {
+                const uint32_t t = at(s, (uint32_t)__builtin_ctzll(on));
+                if (seen[t] != k + 1) next.push_back(t);
+                seen[t] = k + 1;
             }
         }
         now.swap(next);
-        chance *= n / 64.0;
-        for (uint32_t s = 0; s < states; s++) f.end[k + 1] = f.end[k + 1] || (now[s] && accepts(s));
+        chance *= __builtin_popcountll(f.values[k]) / 64.0;
+        for (uint32_t s : now) f.end[k + 1] = f.end[k + 1] || accepts(s);
     }
     if (!f.end[1] && !f.end[2]) f.chance = chance;
     return f;
