@@ -44,6 +44,7 @@ struct mk_ctx {
     uint32_t layout = mkb::LAYOUT_INVERTER_WARP;  // which threads an iteration's span counts
     uint32_t inv_batch = 0;   // keys per field inversion asked for (0: 32 inversions per CTA and iteration)
     uint32_t table_smem = 0;  // bytes of the comb table each search CTA keeps in shared memory (0: HBM)
+    uint32_t dfa_room[2] = {};  // shared memory for DFA tables: hashed seeds, incremental source
     uint32_t hit_capacity = 1u << 16;
     uint8_t* noalloc = nullptr;  // device address of mk_derive_noalloc's fixed staging array
     std::string err;
@@ -58,6 +59,7 @@ struct mk_job {
     mkb::MatchSet* d_match = nullptr;
     std::vector<uint8_t*> d_dfa;
     bool light = true;            // neither regex needles nor the 4-gram prefilter
+    bool prefilter = false;       // the 4-gram prefilter is on
     uint32_t* d_gram4 = nullptr;  // 4-gram prefilter bitmap (2 MB), allocated on first use
     mkb::HitRecord* d_hits = nullptr;
     uint32_t cap = 1u << 16;
@@ -323,6 +325,8 @@ int mk_ctx_create(int device, const mk_options* options, mk_ctx** out) try {
     if (occ < 1) return fail(c, MK_ERR_NOT_BUILT, "kernel does not fit on this device");
     uint32_t per_sm = o.blocks_per_sm ? std::min<uint32_t>(o.blocks_per_sm, (uint32_t)occ) : (uint32_t)occ;
     c->grid = (uint32_t)prop.multiProcessorCount * per_sm;
+    for (int incr = 0; incr < 2; incr++)
+        MK_CUDA(c, mkb::search_dfa_room(incr, c->block, per_sm, &c->dfa_room[incr]));
     // table
     size_t bytes = (size_t)c->geom.entries * mkb::COMB_STRIDE_WORDS * 4;
     e = cudaMalloc(&c->table, bytes);
@@ -843,7 +847,8 @@ static int upload_needles(mk_job* j, mkb::MatchSet& ms, std::vector<mkh25519::Ne
     MK_CUDA(c, cudaMemcpyAsync(j->d_match, &ms, sizeof ms, cudaMemcpyHostToDevice, c->stream));
     MK_CUDA(c, cudaStreamSynchronize(c->stream));
     j->h2d += sizeof ms;
-    j->light = ms.n_regex == 0 && !ms.gram4;
+    j->prefilter = ms.gram4 != nullptr;
+    j->light = ms.n_regex == 0 && !j->prefilter;
     j->needles = std::move(hosts);
     return MK_OK;
 }
@@ -934,13 +939,18 @@ void mk_job_destroy(mk_job* j) try {
     delete j;
 } MK_ABI_CATCH_VOID
 
-// Shared memory for the job's DFA tables when they fit (the kernel then reads them there).
+// Shared memory for the job's DFA tables when they are small: as much as leaves an SM the CTAs that the
+// grid is sized for (block = 256 has two, and the second one's place would go to 20 KB of tables: 33 M
+// candidates on B200, 8 keys per thread, eight regexes 45.1 -> 42.3 ms, four others 44.3 -> 40.8), or, with
+// the 4-gram prefilter, all of them (64 text needles beside the eight regexes: 52.6 ms with one CTA and
+// all tables, 54.2 with two and two tables in global memory).
 static uint32_t dfa_smem_bytes(const mk_job* j) {
-    if (j->ctx->table_smem) return 0;  // a comb table kept in shared memory takes that room
     uint64_t total = 0;
     for (const auto& h : j->needles)
         if (h.mode == MK_MODE_REGEX) total += ((uint64_t)h.len * 130 + 15) & ~15ull;
-    return total <= mkb::DFA_SMEM_MAX ? (uint32_t)total : 0;
+    if (total > mkb::DFA_SMEM_MAX || j->ctx->table_smem) return 0;  // a comb table takes that room
+    if (j->prefilter) return (uint32_t)total;
+    return std::min((uint32_t)total, j->ctx->dfa_room[j->source == MK_SEED_INCREMENTAL]);
 }
 
 // Field inversions per CTA and iteration of the kernel that serves a context's searches of a

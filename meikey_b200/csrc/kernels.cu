@@ -291,9 +291,10 @@ __device__ __forceinline__ bool quick_match(const MatchSet& ms, const u32 pk[8])
 
 // Tests one key (y only; the character at position 42 is tried with both x signs, as
 // kernel.cu:1804-1875 does) and sets bit `id` of hit_words for every needle that may match.
-// `lane_masks` and `lane_buckets` are tables with every value's entry once per lane (value v of lane
-// l at v * 32 + l), so that every lane reads its own banks: the low half of mask word 0 for jobs whose
-// text needles fit in 32 bits of state, and the bucket filter.  Called by all 32 lanes of a warp.
+// `lane_masks` and `lane_buckets` are tables with every value's entry once per lane, so that every lane
+// reads its own banks: the low half of mask word 0 for jobs whose text needles fit in 32 bits of state
+// (value v of lane l at v * 32 + l), and the bucket filter, whose 64-bit entries are read half a warp at a
+// time (value v of lanes l and l + 16 at v * 16 + l).  Called by all 32 lanes of a warp.
 // LIGHT: the job has neither the prefilter nor regex needles; their code costs the kernel
 // registers (spills) that a job of a few needles runs faster without (one needle on B200: 0.929 ->
 // 0.936 G keys/s, incremental 12.6 -> 12.9).
@@ -315,13 +316,13 @@ __device__ __forceinline__ void match_key(const MatchSet& ms, const u32* lane_ma
     // through to them (58 needles; half of them at 128).
     u32 flags = ~0u;  // the buckets the key may hold something of
     if (!LIGHT && ms.buckets) {
-        const u64* lm = lane_buckets + (threadIdx.x & 31u);
+        const u64* lm = lane_buckets + (threadIdx.x & 15u);
         u64 D = 0;
         u32 acc = 0;
 #pragma unroll
         for (int pos = 1; pos < 44; pos++) {
-            u64 mk = lm[value(pos) * 32u];
-            if (pos == MK_SIGN_POS) mk |= lm[(value(pos) | 2u) * 32u];
+            u64 mk = lm[value(pos) * 16u];
+            if (pos == MK_SIGN_POS) mk |= lm[(value(pos) | 2u) * 16u];
             D = (D << BUCKETS | ((1ull << BUCKETS) - 1)) & mk;
             acc |= (u32)(D >> 32);
         }
@@ -723,7 +724,7 @@ __global__ void __launch_bounds__(BLOCK, 512 / BLOCK) k_search(const KeyLaunch L
     __shared__ CombGeom g;
     __shared__ MatchSet ms;
     __shared__ u32 lane_masks[64 * 32];  // see match_key
-    __shared__ u64 lane_buckets[LIGHT ? 1 : 64 * 32];
+    __shared__ u64 lane_buckets[LIGHT ? 1 : 64 * 16];
     __shared__ u32 key[8];
     __shared__ mkh::CounterMid mid;
     __shared__ volatile u64 stop_iter;
@@ -747,34 +748,33 @@ __global__ void __launch_bounds__(BLOCK, 512 / BLOCK) k_search(const KeyLaunch L
         for (u32 e = tid; e < (u32)g.entries; e += BLOCK)
 #pragma unroll
             for (int q = 0; q < 6; q++) stab[e * 6 + q] = L.table[(u64)e * (COMB_STRIDE_WORDS / 4) + q];
-    u32 dfa_need = 0;
-    for (u32 r = 0; !LIGHT && r < ms.n_regex; r++) dfa_need += (ms.dfa_states[r] * 130u + 15u) & ~15u;
-    if (!LIGHT && L.dfa_smem && dfa_need <= L.dfa_smem) {
-        // stage the job's DFA tables behind the other dynamic buffers (only when the launch
-        // reserved room for all of them) and point the matcher at the copies (16-byte
-        // aligned tables, copied in u16 units)
+    if (!LIGHT && L.dfa_smem) {
+        // stage the job's DFA tables behind the other dynamic buffers, those that every key walks first,
+        // as many as the launch reserved room for, and point the matcher at the copies (16-byte aligned
+        // tables, copied in u16 units)
         uint8_t* area = reinterpret_cast<uint8_t*>(INCR ? (void*)slots : (void*)(slots + CT));
-        u32 off = 0;
-        for (u32 r = 0; r < ms.n_regex; r++) {
+        auto each_staged = [&](auto f) {
+            u32 off = 0;
+            for (u32 rest = 0; rest < 2; rest++)
+                for (u32 r = 0; r < ms.n_regex; r++) {
+                    const u32 bytes = (ms.dfa_states[r] * 130u + 15u) & ~15u;
+                    if (((ms.regex_always >> r) & 1u) == rest || bytes > L.dfa_smem - off) continue;
+                    f(r, area + off);
+                    off += bytes;
+                }
+        };
+        each_staged([&](u32 r, uint8_t* to) {
             const uint16_t* src = reinterpret_cast<const uint16_t*>(ms.dfa[r]);
-            uint16_t* dst = reinterpret_cast<uint16_t*>(area + off);
-            const u32 halves = ms.dfa_states[r] * 65u;
-            for (u32 i = tid; i < halves; i += BLOCK) dst[i] = src[i];
-            off += (halves * 2u + 15u) & ~15u;
-        }
+            uint16_t* dst = reinterpret_cast<uint16_t*>(to);
+            for (u32 i = tid; i < ms.dfa_states[r] * 65u; i += BLOCK) dst[i] = src[i];
+        });
         __syncthreads();
-        if (tid == 0) {
-            off = 0;
-            for (u32 r = 0; r < ms.n_regex; r++) {
-                ms.dfa[r] = area + off;
-                off += (ms.dfa_states[r] * 130u + 15u) & ~15u;
-            }
-        }
+        if (tid == 0) each_staged([&](u32 r, uint8_t* to) { ms.dfa[r] = to; });
     }
     if (ms.narrow)
         for (u32 i = tid; i < 64u * 32u; i += BLOCK) lane_masks[i] = (u32)ms.mask[0][i >> 5];
     if (!LIGHT && ms.buckets)
-        for (u32 i = tid; i < 64u * 32u; i += BLOCK) lane_buckets[i] = ms.bucket[i >> 5];
+        for (u32 i = tid; i < 64u * 16u; i += BLOCK) lane_buckets[i] = ms.bucket[i >> 4];
     if (INCR && tid < (u32)INCR_STEPS) step_to_yx(steps, tid);
     if (tid == 0 && L.seed_src == 1) mid = mkh::counter_mid(key);
     __syncthreads();
@@ -1000,6 +1000,26 @@ cudaError_t search_occupancy(uint32_t kpt, uint32_t block, uint32_t table_smem, 
     cudaError_t e = search_kernel(false, kpt, block, false, 0, table_smem, &f, &dyn);
     if (e != cudaSuccess) return e;
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, f, (int)block, dyn);
+}
+
+cudaError_t search_dfa_room(bool incr, uint32_t block, uint32_t ctas, uint32_t* room) {
+    const void* f = nullptr;
+    size_t dyn = 0;
+    *room = 0;
+    cudaError_t e = search_kernel(incr, 0, block, false, 0, 0, &f, &dyn);
+    cudaFuncAttributes fa{};
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, f);
+    int device = 0, sm = 0, reserved = 0, cta_max = 0;
+    if (e == cudaSuccess) e = cudaGetDevice(&device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&cta_max, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+    if (e != cudaSuccess) return e;
+    // a CTA's share in whole kilobytes, a multiple of the granularity shared memory is given out in
+    const size_t share = std::min((size_t)cta_max, ((size_t)sm / ctas - reserved) & ~(size_t)1023);
+    const size_t used = fa.sharedSizeBytes + dyn;
+    if (share > used) *room = std::min(DFA_SMEM_MAX, (uint32_t)(share - used) & ~15u);
+    return cudaSuccess;
 }
 
 // Keys per thread of a derive: the fewest that let one wave (512 threads per SM) hold them all, at

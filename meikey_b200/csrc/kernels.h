@@ -36,8 +36,8 @@ struct KeyLaunch {
     uint32_t delta[24];    // CTAs·search_kernel_threads·keys·B: a search thread's jump between iterations
     // the job has neither regex needles nor the 4-gram prefilter (picks the kernel)
     bool light;
-    // bytes of shared memory for the job's DFA tables (each 16-byte aligned; 0: read them
-    // from global memory)
+    // bytes of shared memory for the job's DFA tables (each 16-byte aligned; those that do not
+    // fit are read from global memory)
     uint32_t dfa_smem;
     // field inversions per CTA and iteration of a search, 1..32 (one per lane of the inverting
     // warp): each pools the products of every inv_pools-th compute thread
@@ -112,6 +112,9 @@ constexpr double MADS_INVERT = 18 * (30 * 6 + 2 * 72);
 // kernel's shared-memory limit like launch_search does.
 cudaError_t search_kernel(bool incr, uint32_t kpt, uint32_t block, bool light, uint32_t dfa_smem, uint32_t table_smem,
                           const void** func, size_t* dyn);
+// Shared memory that DFA tables may take without keeping `ctas` search CTAs from sharing an SM, at most
+// DFA_SMEM_MAX.
+cudaError_t search_dfa_room(bool incr, uint32_t block, uint32_t ctas, uint32_t* room);
 cudaError_t search_occupancy(uint32_t kpt, uint32_t block, uint32_t table_smem, int* blocks_per_sm);
 // multiply-adds per second of the carry-chain row microbenchmark and of plain mad.lo.u32
 cudaError_t measure_mad_peaks(int sms, cudaStream_t st, double* chain_per_s, double* lo_per_s);
