@@ -417,7 +417,7 @@ def workload_config(workload, ctx, step_candidates=None, steps=None):
             "keys_per_thread": info["keys_per_thread"],
             "block": info["block"],
             "grid": info["grid"],
-            # keys sharing one field inversion (mk_options.inversion_batch)
+            # as asked for (mk_options.inversion_batch); searches take the nearest number of inversions
             "inversion_batch": info["inversion_batch"],
             "l2": ("no memory-resident inputs: each thread steps its own point, the 14 KB step tables "
                    "stay on chip" if workload == "incremental" else

@@ -135,7 +135,11 @@ typedef struct mk_info {
     uint64_t table_bytes;
     uint64_t keys_per_iter;   /* grid · (block - 32; block with inverter_rotates; 352 with hash_warps) · keys_per_thread */
     char name[96];
-    uint32_t inversion_batch; /* keys sharing one field inversion */
+    uint32_t inversion_batch; /* mk_options.inversion_batch, or for 0 what 32 pools make of the counted threads:
+                                 keys_per_iter / (grid · pools).  Searches share an inversion among
+                                 block · 8 / pools keys (hashed seeds) or (block - 32) · 16 / pools (incremental
+                                 source), with 32 pools for 0 and else as many as come nearest to it, 4 at
+                                 least: a default context says 240 and its hashed searches share among 128 */
     uint32_t table_in_smem;   /* 1: search CTAs read the comb table from shared memory */
 } mk_info;
 

@@ -448,14 +448,15 @@ BUILT_VARIANTS = [(4, 256), (8, 256), (16, 256), (4, 512), (8, 512), (16, 512)]
 
 
 def compute_threads(block: int, hash_warps: int = 0, inverter_rotates: int = 0) -> int:
-    """Threads of a search CTA that derive keys."""
+    """Threads of a search CTA that the span of an iteration counts."""
     return 352 if hash_warps else block if inverter_rotates else block - 32
 
 
 def inversion_batches(keys_per_thread: int, block: int, hash_warps: int = 0, inverter_rotates: int = 0,
                       lo: int = 64, hi: int = 512):
-    """The inversion batches in [lo, hi] a layout can run: keys per thread x compute threads /
-    pools, for pool counts that divide the compute threads and are at most 32."""
+    """The inversion batches in [lo, hi] a layout accepts: keys per thread x counted threads /
+    pools, for pool counts that divide the counted threads and are at most 32 (searches take the
+    pool count of their own kernel that comes nearest, at least 4)."""
     ct = compute_threads(block, hash_warps, inverter_rotates)
     return sorted({keys_per_thread * ct // p for p in range(1, 33)
                    if ct % p == 0 and lo <= keys_per_thread * ct // p <= hi})
@@ -464,10 +465,12 @@ def inversion_batches(keys_per_thread: int, block: int, hash_warps: int = 0, inv
 def tune_space(rows=(11, 12, 13, 14, 16), variants=BUILT_VARIANTS, blocks_per_sm=(0,), hash_warps=(0, 4),
                inverter_rotates=(0,), inversion_batch=(0,), table_in_smem=(0,)):
     """Candidate options: comb rows (table size against multiplications per key) x keys per
-    thread and block x CTAs per SM x the hashing-warp layout (built for block 512, keys per
-    thread 8 and 16) x the counted threads (block - 32, or all with inverter_rotates; not with
-    hashing warps) x the inversion batch (keys per field inversion; 0 = 32 pools,
-    "all" = every batch of 64..512 the layout can run)."""
+    thread and block x CTAs per SM x the counted threads (352 with hash_warps, which takes block
+    512 and keys per thread 8 and 16; block - 32, or all with inverter_rotates) x the inversion
+    batch (keys per field inversion; 0 = 32 pools, "all" = every batch of 64..512 the layout
+    accepts).  Rows, block and batch choose how a key is computed (with table_in_smem keys per
+    thread too); the others only the span of an iteration, so candidates that differ in nothing
+    else differ by its rounding and by noise."""
     out = []
     for r in rows:
         for (k, b) in variants:

@@ -24,6 +24,7 @@ def pools_of(ctx, source):
 def test_pools(oracle, kpt, block, hw, rot, batch, hashed, incremental):
     with mk.Context(device=0, table_rows=16, keys_per_thread=kpt, block=block, hash_warps=hw, hit_capacity=1 << 18,
                     inverter_rotates=bool(rot), inversion_batch=batch) as ctx:
+        assert ctx.info["inversion_batch"] == batch  # as asked, whatever pools come of it
         for source, want in ((mk.SEED_COUNTER, hashed), (mk.SEED_INCREMENTAL, incremental)):
             if want is None:
                 continue
@@ -32,5 +33,16 @@ def test_pools(oracle, kpt, block, hw, rot, batch, hashed, incremental):
             with ctx.job(key, source, [mk.Needle.suffix("Zq")]) as job:
                 job.launch(2**30 + 7, 3)
                 hits, _ = job.hits(cap=1 << 18)
-            n = 3 * ctx.keys_per_iter
-            assert [i for i, _ in hits] == oracle.search(key, source, 2**30 + 7, n, b"Zq", 2, False, 1)
+            # the start of the second iteration and the end of the last one
+            for first in (2**30 + 7 + ctx.keys_per_iter, 2**30 + 7 + 3 * ctx.keys_per_iter - 100000):
+                want = oracle.search(key, source, first, 100000, b"Zq", 2, False, 1)
+                assert [i for i, _ in hits if first <= i < first + 100000] == want
+
+
+@pytest.mark.parametrize("kpt,block,hw,rot,says", [(16, 512, 0, 0, 240), (8, 256, 0, 1, 64), (16, 512, 4, 0, 176)])
+def test_info_and_pools_without_a_batch(kpt, block, hw, rot, says):
+    with mk.Context(device=0, table_rows=16, keys_per_thread=kpt, block=block, hash_warps=hw,
+                    inverter_rotates=bool(rot)) as ctx:
+        assert ctx.info["inversion_batch"] == says
+        assert pools_of(ctx, mk.SEED_COUNTER) == pytest.approx(32, rel=1e-9)
+        assert pools_of(ctx, mk.SEED_INCREMENTAL) == pytest.approx(32, rel=1e-9)
