@@ -31,6 +31,7 @@ import hashlib
 import json
 import math
 import os
+import re
 import statistics
 import subprocess
 import sys
@@ -427,15 +428,25 @@ def workload_config(workload, ctx, step_candidates=None, steps=None):
     return cfg
 
 
-def traffic_per_key(workload):
-    """DRAM bytes per key of the search kernel from the committed ncu summary of this workload."""
-    path = os.path.join(ROOT, "profiles", "k_search_dram.json" if workload == "secure" else
-                        f"k_search_{workload}_dram.json")
+def device_code_digest():
+    """SHA-256 of the search kernels' sources without comments and spaces."""
+    h = hashlib.sha256()
+    for name in ("kernels.cu", "kernels.h", "types.h", "fe32.cuh", "ge.cuh", "modinv.cuh", "hash.cuh"):
+        with open(os.path.join(ROOT, "meikey_b200", "csrc", name)) as f:
+            h.update(re.sub(r"//[^\n]*|\s+", "", f.read()).encode())
+    return h.hexdigest()
+
+
+def traffic_per_key(workload, folder=os.path.join(ROOT, "profiles")):
+    """DRAM bytes per key of the search kernel from the committed ncu summary of this workload; None
+    when there is none or it was captured from other device code than this tree's."""
+    path = os.path.join(folder, "k_search_dram.json" if workload == "secure" else f"k_search_{workload}_dram.json")
     try:
         with open(path) as f:
-            return json.load(f).get("dram_bytes_per_key")
+            profile = json.load(f)
     except (OSError, ValueError):
         return None
+    return profile.get("dram_bytes_per_key") if profile.get("device_code") == device_code_digest() else None
 
 
 def _pct(xs, q):
