@@ -1,5 +1,10 @@
 // Inversion modulo p = 2^255 - 19 by division steps (Bernstein and Yang, "Fast constant-time gcd
-// computation and modular inversion", CHES 2019, with the half-integer start of delta).
+// computation and modular inversion", CHES 2019).  The half-integer start of delta with its bound of
+// 590 steps, the nine signed limbs of 30 bits, the limb-by-limb application of a matrix with two
+// running sums, and the names zeta, cf, cg, cd, ce are those of libsecp256k1 (src/modinv32 and
+// doc/safegcd_implementation.md, by Pieter Wuille and Peter Dettman; MIT licence).  The step on
+// wrapping words, the correction by a centred multiple of p = -19 + 2^255 and the final sign and fold
+// are this file's own.
 //
 // A division step on (delta, f, g), f odd, needs only the lowest bits of f and g, so 30 of them
 // run on 32-bit words and are collected in a 2x2 matrix of integers below 2^30 in magnitude, which
