@@ -10,6 +10,10 @@
 //
 // Reference behaviour: src/service/gpu/kernel.cu:1898-2069 (meikey_search / meikey_derive).
 // A launch covers the same consecutive indices from its base.
+//
+// Rates in comments are both sides of the change they explain, measured when it was made; later changes
+// moved both.  As they stand the kernels run one needle at 0.95-0.98 G keys/s on hashed seeds and at
+// 15.6 G on the incremental source (B200, long launches).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -110,8 +114,8 @@ struct EntrySlot {
 // digit swaps the first two on their way into the slot and takes -2dxy, which the entry holds as
 // its last 32 bytes, so the addition needs no selects (48 an addition).  With the tight sums of
 // ge_add_niels and the rows of fe_mul that open a pair first, one addition takes 2320 instead of
-// 2451 cycles of an SM sub-partition (16 warps per SM, the multiply pipe 93 % busy), and the search
-// of hashed seeds runs at 0.926 instead of 0.889 G keys/s.
+// 2451 cycles of an SM sub-partition (16 warps per SM, the multiply pipe 93 % busy): hashed seeds
+// 0.889 -> 0.926 G keys/s.
 __device__ __forceinline__ void fetch_entry(EntrySlot& slot, int which, const uint4* table, u64 idx, bool neg) {
     const uint4* src = table + idx * (COMB_STRIDE_WORDS / 4);
     const u32 dst = (u32)__cvta_generic_to_shared(&slot.q[which][0]);
@@ -683,7 +687,7 @@ __device__ __forceinline__ void incr_fracs(const ge& Q, const uint4* steps, Batc
 //     warp it mod the CTA's warps, so that consecutive inversions run on different SM
 //     sub-partitions and every warp carries the same share.  A dedicated inverter leaves its
 //     sub-partition with three compute warps against four (warp w runs on sub-partition w % 4):
-//     on B200, 8 keys per thread, 0.82 G keys/s against 0.89 with the rotating duty.  The inverting
+//     on B200, 8 keys per thread, 0.82 -> 0.89 G keys/s with the rotating duty.  The inverting
 //     warp does its backward pass of it-1 first: by then the others have arrived, so it does not
 //     wait for the slowest of them, and they still have a whole forward pass to run before they need
 //     the inverses (0.936 -> 0.974 G keys/s; 0.916 -> 0.966 at 16 pools, whose chain is longer);

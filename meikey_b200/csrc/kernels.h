@@ -52,7 +52,7 @@ struct KeyLaunch {
 // hashed seeds rotate the inversion over every warp, the incremental source and comb tables in
 // shared memory leave it to the last one.  (Warps that only hash beside comb warps, 0.877 G keys/s
 // on B200 and 0.908 with all 16 other warps at the comb, and SHA-512 rounds inside the comb rows,
-// 0.69, lose to hashing in every warp, 0.926: operations of the ALU and of the multiply pipe from
+// 0.69, lost to hashing in every warp, 0.926 in the same build: operations of the ALU and of the multiply pipe from
 // different warps compete for register reads instead of overlapping.)
 constexpr uint32_t LAYOUT_INVERTER_WARP = 0, LAYOUT_ROTATING = 1, LAYOUT_HASH_WARPS = 4;
 
