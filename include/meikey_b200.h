@@ -418,8 +418,9 @@ MK_API int mk_autotune(int device, mk_tune_entry* entries, uint32_t n, uint32_t 
                        uint32_t* best);
 
 /* mk_autotune timed on the caller's own job instead of the fixed secure-path one: the key,
- * seed source and needles of mk_job_prepare (the best options depend on the matching work;
- * inverter_rotates pays with many needles).  A candidate whose job cannot be prepared (e.g.
+ * seed source and needles of mk_job_prepare (the best options depend on the seed
+ * source and the matching work; candidates that differ only in what an iteration spans run the
+ * same kernel).  A candidate whose job cannot be prepared (e.g.
  * hash_warps with the incremental source) is dropped with that status. */
 MK_API int mk_autotune_job(int device, mk_tune_entry* entries, uint32_t n, uint32_t finalists, uint64_t trial_keys,
                            const uint8_t key[32], int seed_source, const mk_needle* needles, uint32_t n_needles,

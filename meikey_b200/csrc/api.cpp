@@ -38,7 +38,7 @@ struct mk_ctx {
     CombGeom geom{};
     uint4* table = nullptr;
     uint4* incr = nullptr;           // incremental source: window table then step table
-    uint32_t delta[24] = {};         // keys_per_iter·B (table form)
+    uint32_t delta[24] = {};         // jump of an incremental search thread between iterations (table form)
     uint32_t kpt = 8, block = 256, grid = 0;
     uint32_t hash_warps = 0;  // 4: hashed seed sources only
     uint32_t layout = mkb::LAYOUT_INVERTER_WARP;  // which threads an iteration's span counts

@@ -713,7 +713,7 @@ __device__ __forceinline__ void incr_fracs(const ge& Q, const uint4* steps, Batc
 // (tests/test_search_buffers.py model-checks both forms with their accesses to the buffers).
 // INCR: the incremental source.  A compute thread keeps the point Q of its middle index (key
 // KPT/2) in the current iteration; its keys are Q ± d·B from the step table, and Q advances by
-// keys_per_iter·B (one mixed addition) per iteration.  No comb table is read.
+// CTAs·CT·KPT·B (one mixed addition) per iteration.  No comb table is read.
 // STAB: the comb table lives in shared memory (copied by every CTA at the start, in place of
 // the staging slots; tables of a few hundred to a few thousand entries, 40+ rows).
 template <int KPT, int BLOCK, bool INCR, bool ROT, bool LIGHT, bool STAB = false>

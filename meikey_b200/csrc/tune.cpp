@@ -5,7 +5,7 @@
 // keys differ from the host derivation is dropped (MK_ERR_SELF_CHECK), and times one launch
 // of about `trial_keys` candidates after a warm-up launch: of a fixed secure-path job
 // (mk_autotune) or of the caller's own job (mk_autotune_job: seed source, key and needles,
-// since the best options depend on the matching work, e.g. inverter_rotates for many needles).  Stage 2 keeps the
+// since the best options depend on its seed source and matching work).  Stage 2 keeps the
 // `finalists` fastest, holds their contexts together and times them in rounds of
 // alternating order (forward, backward, forward), keeping each one's best rate, so that a
 // drift of the clock over the sweep does not favour whichever ran first.
